@@ -93,6 +93,14 @@ EFL_DEV float det4(const float* m) {
 
 // utils/area_fraction.wgsl:10-12
 EFL_DEV float area_fraction(float l0, float l1) { return fclamp01(fmaxf(l0, l1) / fabsf(l0 - l1)); }
+// area_fraction(l0, l1) > 0.  The division decides only where its quotient may round to 0 or an operand is not
+// finite; otherwise the sign of the larger value does.
+EFL_DEV bool area_fraction_positive(float l0, float l1) {
+    const float m = fmaxf(l0, l1);
+    if (!(m > 0.0f)) return false;  // a NaN operand leaves the other one or NaN: the fraction is 0 or below
+    if (m >= 1e-30f && fabsf(l0 - l1) <= 1e8f) return true;
+    return area_fraction(l0, l1) > 0.0f;
+}
 // utils/area_fraction.wgsl:14-56 -> (i-1/2, i+1/2, j-1/2, j+1/2)
 EFL_DEV float4 area_fractions(const PF& ls, int x, int y) {
     float c0 = ls.ld(x - 1, y - 1), c1 = ls.ld(x, y - 1), c2 = ls.ld(x + 1, y - 1);
@@ -821,103 +829,108 @@ __global__ void k_solve_velocity_uv(PF u0, PF u1, PF us, PF v0, PF v1, PF vs, PF
         solve_velocity_at<1>(v0, v1, vs, p0, ls0, fv, U, d);
 }
 
-// extrapolate/initialize_u_valid.wgsl:6-30 / initialize_v_valid.wgsl:6-30
-template <int COMP>
-__global__ void k_init_valid(PI valid, PF ls0, Dom d) {
-    int x = gx(), y = gy();
-    if (COMP == 0 ? (x > d.nx || y >= d.xrows()) : (x >= d.ycols() || y > d.ny)) return;
-    float c0, c1, c2, c3, c4, c5;
-    if (COMP == 0) {
-        c0 = ls0.ld(x - 1, y - 1); c1 = ls0.ld(x, y - 1); c2 = ls0.ld(x - 1, y);
-        c3 = ls0.ld(x, y); c4 = ls0.ld(x - 1, y + 1); c5 = ls0.ld(x, y + 1);
-    } else {
-        c0 = ls0.ld(x - 1, y - 1); c1 = ls0.ld(x - 1, y); c2 = ls0.ld(x, y - 1);
-        c3 = ls0.ld(x, y); c4 = ls0.ld(x + 1, y - 1); c5 = ls0.ld(x + 1, y);
-    }
-    float vm = 0.25f * (c0 + c1 + c2 + c3);
-    float vp = 0.25f * (c2 + c3 + c4 + c5);
-    valid.st(x, y, area_fraction(vm, vp) > 0.0f ? 0 : 1);
-}
-// extrapolate/extrapolate_{u,v}.wgsl:5-63 over [0,x1) x [0,y1)
-__global__ void k_extrapolate(PF f, PI vin, PI vout, int x1, int y1) {
-    int x = gx(), y = gy();
-    if (x >= x1 || y >= y1) return;
-    const int W = vin.w, H = vin.h;
-    if (vin.ld(x, y) == 1) {
-        vout.st(x, y, 1);
-        return;
-    }
-    int count = 0;
-    float nu = 0.0f;
-    if (x + 1 < W && y < H && vin.ld(x + 1, y) == 1) { nu += f.ld(x + 1, y); count += 1; }
-    if (x - 1 > 0 && y > 0 && vin.ld(x - 1, y) == 1) { nu += f.ld(x - 1, y); count += 1; }
-    if (x < W && y + 1 < H && vin.ld(x, y + 1) == 1) { nu += f.ld(x, y + 1); count += 1; }
-    if (x > 0 && y - 1 > 0 && vin.ld(x, y - 1) == 1) { nu += f.ld(x, y - 1); count += 1; }
-    if (count > 0) {
-        nu /= (float)count;
-        f.st(x, y, nu);
-        vout.st(x, y, 1);
-    } else {
-        vout.st(x, y, 0);
-    }
-}
-
 // initialize_{u,v}_valid + the 10 extrapolation sweeps of render_node.rs:540-608
-// in ONE launch, for grids whose dispatches cover every face (nx and ny
-// multiples of 64): blockIdx.z = component; each CTA owns a 32 x 32 tile of
-// faces, holds it with a 10-face halo in shared memory and runs the sweeps
-// there (each sweep reads the valid flags of the previous one and only
-// valid neighbours' velocities, so the result equals 10 global sweeps).
-// Writes the velocity, the final flags (the "in" plane) and the flags after
-// the ninth sweep (the "out" plane), as the per-sweep kernels leave them.
-constexpr int EX_T = 32, EX_H = 10, EX_E = EX_T + 2 * EX_H;
+// in ONE launch: blockIdx.z = component; each CTA owns a 32 x 32 tile of
+// faces and holds it with a 10-face halo in shared memory (each sweep reads
+// the valid flags of the previous one and only valid neighbours' velocities,
+// so the result equals 10 global sweeps).  Writes the velocity, the flags
+// after the tenth sweep (the "in" plane) and after the ninth (the "out"
+// plane), as the per-sweep kernels leave them.
+//
+// Latency and issue bound it (a few CTAs on small grids, each a chain of 10
+// sweeps).  A face turns valid once and its value is computed once, in that
+// sweep: one warp runs the ten sweeps on the flags alone (a 64-bit word per
+// image row, two rows per lane, neighbour rows by shuffles) and leaves the
+// sweep in which each face turns valid, and the faces of each sweep as a list;
+// then a sweep is one face per thread, its neighbours being valid if their
+// sweep is an earlier one.  The form before it (byte flags, every face visited
+// in every sweep by 256 threads with run-time row divisions) took 39 us at
+// 64^2 and 48 us at 768 x 512.
+//
+// Faces outside the reference's dispatch (floor(n / 64) * 64 rows or columns,
+// pipeline.rs:175-186) keep their velocity and both their flag planes; each
+// sweep reads their flag from the plane that it reads.
+constexpr int EX_T = 32, EX_H = 10, EX_E = EX_T + 2 * EX_H, EX_THREADS = 512;
 struct ExtrapArgs {
     PF f[2];
     PI vin[2], vout[2];
     PF ls;
     const float2* range;  // per 32 x 32 cell tile of ls: (min, max)
     int rtx, rty;         // cell tiles per row / column
+    int cw[2], ch[2];     // faces covered by the dispatch, per component
 };
 // (min, max) of the level set over each 32 x 32 tile of cells (one CTA per tile).
 __global__ void __launch_bounds__(256) k_ls_tile_range(PF ls, float2* range, int rtx) {
     const int x0 = blockIdx.x * EX_T, y0 = blockIdx.y * EX_T;
     float lo = INFINITY, hi = -INFINITY;
+    int nan = 0;  // a NaN makes the tile non-uniform below
     for (int i = threadIdx.x; i < EX_T * EX_T; i += 256) {
         const int x = x0 + (i & (EX_T - 1)), y = y0 + i / EX_T;
         if (x < ls.w && y < ls.h) {
             const float v = ls.at(x, y);
             lo = fminf(lo, v);
             hi = fmaxf(hi, v);
-            if (v != v) lo = hi = NAN;  // a NaN makes the tile non-uniform below
+            nan |= v != v;
         }
     }
-    __shared__ float slo[256], shi[256];
-    slo[threadIdx.x] = lo;
-    shi[threadIdx.x] = hi;
-    __syncthreads();
-    for (int k = 128; k > 0; k >>= 1) {
-        if (threadIdx.x < k) {
-            const float a = slo[threadIdx.x + k], b = shi[threadIdx.x + k];
-            slo[threadIdx.x] = (a != a || slo[threadIdx.x] != slo[threadIdx.x]) ? NAN : fminf(slo[threadIdx.x], a);
-            shi[threadIdx.x] = (b != b || shi[threadIdx.x] != shi[threadIdx.x]) ? NAN : fmaxf(shi[threadIdx.x], b);
-        }
-        __syncthreads();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
-    if (threadIdx.x == 0) range[blockIdx.y * rtx + blockIdx.x] = make_float2(slo[0], shi[0]);
+    __shared__ float slo[8], shi[8];
+    if ((threadIdx.x & 31) == 0) {
+        slo[threadIdx.x >> 5] = lo;
+        shi[threadIdx.x >> 5] = hi;
+    }
+    const int any_nan = __syncthreads_or(nan);
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) {
+            lo = fminf(lo, slo[k]);
+            hi = fmaxf(hi, shi[k]);
+        }
+        range[blockIdx.y * rtx + blockIdx.x] = any_nan ? make_float2(NAN, NAN) : make_float2(lo, hi);
+    }
 }
-__global__ void __launch_bounds__(256) k_extrapolate_fused(ExtrapArgs a) {
-    __shared__ float sf[EX_E][EX_E];
-    __shared__ unsigned char sv[2][EX_E][EX_E];
+__global__ void __launch_bounds__(EX_THREADS) k_extrapolate_fused(ExtrapArgs a) {
+    typedef unsigned long long row_t;
+    static_assert(EX_E <= 64 && EX_THREADS % 64 == 0 && EX_THREADS >= 320, "an image row is one word; two warps cover a row");
+    constexpr int LW = EX_E + 2, NLS = LW * LW, NFC = EX_E * EX_E, PERF = (NFC + EX_THREADS - 1) / EX_THREADS;
+    constexpr unsigned char NEVER = 15, OUTSIDE = 16;
+    __shared__ float sf[NFC];
+    __shared__ float sl[NLS];          // level set of the cells (x0 - 1 .., y0 - 1 ..)
+    __shared__ row_t sv[64];           // valid flags at the start, bit lx
+    __shared__ row_t stat[2][64];      // flags of the faces outside the dispatch, "in" and "out" plane
+    __shared__ row_t fresh_s[10][64];  // faces that turn valid in a sweep
+    __shared__ unsigned char st[NFC];  // 1 + the sweep in which a face turns valid (0: at the start, NEVER: not in
+                                       // ten sweeps); OUTSIDE + both flags of a face outside the dispatch
+    __shared__ unsigned short list[NFC];
+    __shared__ int total, first_of[10], count_of[10];
     const int comp = blockIdx.z;
     const PF f = a.f[comp];
-    const int W = f.w, H = f.h;
+    const PI vin = a.vin[comp], vout = a.vout[comp];
+    const int W = f.w, H = f.h, CW = a.cw[comp], CH = a.ch[comp];
     const int x0 = blockIdx.x * EX_T - EX_H, y0 = blockIdx.y * EX_T - EX_H;
     const int tid = threadIdx.x;
+    // The same flag for every owned face.
+    auto write_flags = [&](int v) {
+        for (int i = tid; i < EX_T * EX_T / 4; i += EX_THREADS) {
+            const int x = x0 + EX_H + (i & 7) * 4, y = y0 + EX_H + (i >> 3);
+            if (y >= CH) continue;
+            if (x + 3 < CW) {  // x is a multiple of 4 and the pitch one of 32: 16-byte aligned
+                *reinterpret_cast<int4*>(&vin.at(x, y)) = make_int4(v, v, v, v);
+                *reinterpret_cast<int4*>(&vout.at(x, y)) = make_int4(v, v, v, v);
+            } else {
+                for (int k = x; k < CW; ++k) vin.at(k, y) = vout.at(k, y) = v;
+            }
+        }
+    };
+    const bool covered = min(x0 + EX_E, W) <= CW && min(y0 + EX_E, H) <= CH;
     // Every face the tile's image and flags read lies over the 3 x 3 cell tiles around it (the 10-face halo
     // and the one-cell level-set stencil stay within one tile).  All of their level set < 0: every face is
     // valid (area_fraction <= 0); all of it > 1e-30: none is (area_fraction > 0; the bound keeps the corner
     // averages normal).  Either way the ten sweeps change nothing: write the flags only.
-    {
+    if (covered) {
         int neg = 1, pos = 1;
         if (tid < 9) {
             const int tx = min(max((int)blockIdx.x - 1 + tid % 3, 0), a.rtx - 1);
@@ -928,89 +941,164 @@ __global__ void __launch_bounds__(256) k_extrapolate_fused(ExtrapArgs a) {
         }
         const int all_neg = __syncthreads_and(neg), all_pos = __syncthreads_and(pos);
         if (all_neg || all_pos) {
-            const int v = all_neg ? 1 : 0;
-            for (int i = tid; i < EX_T * EX_T; i += 256) {
-                const int x = x0 + EX_H + (i & (EX_T - 1)), y = y0 + EX_H + i / EX_T;
-                if ((unsigned)x >= (unsigned)W || (unsigned)y >= (unsigned)H) continue;
-                a.vin[comp].at(x, y) = v;
-                a.vout[comp].at(x, y) = v;
-            }
+            write_flags(all_neg ? 1 : 0);
             return;
         }
     }
-    for (int i = tid; i < EX_E * EX_E; i += 256) {
-        const int ly = i / EX_E, lx = i - ly * EX_E, x = x0 + lx, y = y0 + ly;
-        float fv = 0.0f;
-        unsigned char v = 0;
-        if ((unsigned)x < (unsigned)W && (unsigned)y < (unsigned)H) {
-            fv = f.at(x, y);
-            float c0, c1, c2, c3, c4, c5;  // extrapolate/initialize_{u,v}_valid.wgsl
-            if (comp == 0) {
-                c0 = a.ls.ld(x - 1, y - 1); c1 = a.ls.ld(x, y - 1); c2 = a.ls.ld(x - 1, y);
-                c3 = a.ls.ld(x, y); c4 = a.ls.ld(x - 1, y + 1); c5 = a.ls.ld(x, y + 1);
-            } else {
-                c0 = a.ls.ld(x - 1, y - 1); c1 = a.ls.ld(x - 1, y); c2 = a.ls.ld(x, y - 1);
-                c3 = a.ls.ld(x, y); c4 = a.ls.ld(x + 1, y - 1); c5 = a.ls.ld(x + 1, y);
-            }
-            const float vm = 0.25f * (c0 + c1 + c2 + c3);
-            const float vp = 0.25f * (c2 + c3 + c4 + c5);
-            v = area_fraction(vm, vp) > 0.0f ? 0 : 1;
-        }
-        sf[ly][lx] = fv;
-        sv[0][ly][lx] = v;
+#pragma unroll
+    for (int k = 0; k < (NLS + EX_THREADS - 1) / EX_THREADS; ++k) {
+        const int i = tid + k * EX_THREADS;
+        if (i < NLS) sl[i] = a.ls.ld(x0 - 1 + i % LW, y0 - 1 + i / LW);
     }
-    // A tile whose image is all valid or all invalid (away from the fluid's boundary: most of a large grid)
-    // comes out of the ten sweeps unchanged, with both flag planes equal to the start flag: write the flags
-    // and skip the sweeps and the face values (only faces inside the domain count).
+#pragma unroll
+    for (int k = 0; k < PERF; ++k) {
+        const int i = tid + k * EX_THREADS;
+        if (i < NFC) sf[i] = f.ld(x0 + i % EX_E, y0 + i / EX_E);
+    }
+    if (tid < 64) sv[tid] = stat[0][tid] = stat[1][tid] = 0;
+    if (tid == 0) total = 0;
+    __syncthreads();
+    // Two warps per image row: lane = column, the second warp 32 columns on.
+    const int lane = tid & 31, half = (tid >> 5) & 1, row0 = tid >> 6;
+    constexpr int ROWS = EX_THREADS / 64, PER = (EX_E + ROWS - 1) / ROWS;
+    const int lx = half * 32 + lane, x = x0 + lx;
     int any_valid = 0, any_invalid = 0;
-    for (int i = tid; i < EX_E * EX_E; i += 256) {
-        const int ly = i / EX_E, lx = i - ly * EX_E, x = x0 + lx, y = y0 + ly;
-        if ((unsigned)x < (unsigned)W && (unsigned)y < (unsigned)H) {
-            if (sv[0][ly][lx]) any_valid = 1;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int ly = row0 + k * ROWS, y = y0 + ly;
+        if (ly >= EX_E) break;
+        bool v = false, s0 = false, s1 = false;
+        if (lx < EX_E && (unsigned)x < (unsigned)W && (unsigned)y < (unsigned)H) {
+            if (x < CW && y < CH) {
+                // extrapolate/initialize_{u,v}_valid.wgsl; c[LW + 1] is the cell (x, y)
+                const float* c = sl + ly * LW + lx;
+                const float c0 = c[0], c3 = c[LW + 1];
+                const float c1 = comp == 0 ? c[1] : c[LW], c2 = comp == 0 ? c[LW] : c[1];
+                const float c4 = comp == 0 ? c[2 * LW] : c[2], c5 = comp == 0 ? c[2 * LW + 1] : c[LW + 2];
+                const float vm = 0.25f * (c0 + c1 + c2 + c3);
+                const float vp = 0.25f * (c2 + c3 + c4 + c5);
+                v = !area_fraction_positive(vm, vp);
+            } else {
+                s0 = vin.at(x, y) == 1;
+                s1 = vout.at(x, y) == 1;
+                v = s0;
+            }
+            if (v) any_valid = 1;
             else any_invalid = 1;
+            if (s0 != s1) any_valid = any_invalid = 1;
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, v);
+        if (lane == 0) reinterpret_cast<unsigned*>(&sv[ly])[half] = b;
+        if (!covered) {
+            const unsigned b0 = __ballot_sync(0xffffffffu, s0), b1 = __ballot_sync(0xffffffffu, s1);
+            if (lane == 0) {
+                reinterpret_cast<unsigned*>(&stat[0][ly])[half] = b0;
+                reinterpret_cast<unsigned*>(&stat[1][ly])[half] = b1;
+            }
         }
     }
-    const bool mixed = __syncthreads_or(any_valid) && __syncthreads_or(any_invalid);
-    if (!mixed) {
-        for (int i = tid; i < EX_T * EX_T; i += 256) {
-            const int ly = EX_H + i / EX_T, lx = EX_H + i % EX_T, x = x0 + lx, y = y0 + ly;
-            if ((unsigned)x >= (unsigned)W || (unsigned)y >= (unsigned)H) continue;
-            const int v = sv[0][ly][lx];
-            a.vin[comp].at(x, y) = v;
-            a.vout[comp].at(x, y) = v;
-        }
+    // A tile whose image is all valid or all invalid comes out of the ten sweeps unchanged, with both flag
+    // planes equal to the start flag (only faces inside the domain count).
+    const int has_valid = __syncthreads_or(any_valid), has_invalid = __syncthreads_or(any_invalid);
+    if (!(has_valid && has_invalid)) {
+        write_flags(has_valid ? 1 : 0);
         return;
     }
+    // The sweeps on the flags (extrapolate_{u,v}.wgsl:5-63): lane l holds the image rows 2 l and 2 l + 1.
+    if (tid < 32) {
+        auto cols = [&](int lo, int hi) -> row_t {  // the columns whose x lies in [lo, hi)
+            const int l = max(lo - x0, 0), h = min(hi - x0, EX_E);
+            return l >= h ? 0ull : ((1ull << (h - l)) - 1ull) << l;
+        };
+        const row_t mcov = cols(0, CW), mright = cols(0, W - 1), mleft = cols(2, W), mup = cols(1, W);
+        row_t v[2], s0[2], s1[2], mc[2], ml[2], mu[2], md[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int ly = 2 * tid + q, y = y0 + ly;
+            v[q] = sv[ly];
+            s0[q] = covered ? 0 : stat[0][ly];
+            s1[q] = covered ? 0 : stat[1][ly];
+            mc[q] = y >= 0 && y < CH && ly < EX_E ? mcov : 0;
+            ml[q] = y > 0 ? mleft : 0;
+            md[q] = y + 1 < H ? ~0ull : 0;
+            mu[q] = y - 1 > 0 ? mup : 0;
+        }
+        for (int s = 0; s < 10; ++s) {
+            row_t up = __shfl_up_sync(0xffffffffu, v[1], 1), dn = __shfl_down_sync(0xffffffffu, v[0], 1);
+            if (tid == 0) up = 0;
+            if (tid == 31) dn = 0;
+            const row_t n0 = ((v[0] >> 1) & mright) | ((v[0] << 1) & ml[0]) | (v[1] & md[0]) | (up & mu[0]);
+            const row_t n1 = ((v[1] >> 1) & mright) | ((v[1] << 1) & ml[1]) | (dn & md[1]) | (v[0] & mu[1]);
+            const row_t f0 = ~v[0] & n0 & mc[0], f1 = ~v[1] & n1 & mc[1];
+            fresh_s[s][2 * tid] = f0;
+            fresh_s[s][2 * tid + 1] = f1;
+            v[0] = (v[0] & mc[0]) | f0 | (s & 1 ? s0[0] : s1[0]);  // as the next sweep reads them
+            v[1] = (v[1] & mc[1]) | f1 | (s & 1 ? s0[1] : s1[1]);
+        }
+    }
+    if (tid >= 32) {  // meanwhile: the faces that never turn valid so far, the valid ones, the ones outside
+        for (int i = tid - 32; i < NFC; i += EX_THREADS - 32) {
+            const int ly = i / EX_E, c = i - ly * EX_E;
+            int n = (sv[ly] >> c) & 1ull ? 0 : NEVER;
+            if (!covered && (x0 + c >= CW || y0 + ly >= CH))
+                n = OUTSIDE + (int)((stat[0][ly] >> c) & 1ull) + 2 * (int)((stat[1][ly] >> c) & 1ull);
+            st[i] = (unsigned char)n;
+        }
+    }
+    __syncthreads();
+    // The faces of each sweep as a list (a warp per sweep, two rows per lane).
+    if (tid < 320) {
+        const int s = tid >> 5;
+        row_t f[2] = {fresh_s[s][2 * lane], fresh_s[s][2 * lane + 1]};
+        const int n = __popcll(f[0]) + __popcll(f[1]);
+        int pre = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int q = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre += q;
+        }
+        int base = 0;
+        if (lane == 31) {
+            base = pre ? atomicAdd(&total, pre) : 0;
+            first_of[s] = base;
+            count_of[s] = pre;
+        }
+        int to = __shfl_sync(0xffffffffu, base, 31) + pre - n;
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            for (row_t m = f[q]; m; m &= m - 1) {
+                const int i = (2 * lane + q) * EX_E + __ffsll(m) - 1;
+                list[to++] = (unsigned short)i;
+                st[i] = (unsigned char)(s + 1);
+            }
+    }
+    __syncthreads();
     for (int s = 0; s < 10; ++s) {
-        const int in = s & 1, out = in ^ 1, lo = 1 + s, n = EX_E - 2 * lo;
-        for (int i = tid; i < n * n; i += 256) {
-            const int ly = lo + i / n, lx = lo + i % n, x = x0 + lx, y = y0 + ly;
-            if ((unsigned)x >= (unsigned)W || (unsigned)y >= (unsigned)H) continue;
-            if (sv[in][ly][lx] == 1) {
-                sv[out][ly][lx] = 1;
-                continue;
-            }
-            int count = 0;
-            float nu = 0.0f;  // extrapolate_{u,v}.wgsl:5-63, neighbour order and bounds as the reference
-            if (x + 1 < W && sv[in][ly][lx + 1] == 1) { nu += sf[ly][lx + 1]; count += 1; }
-            if (x - 1 > 0 && y > 0 && sv[in][ly][lx - 1] == 1) { nu += sf[ly][lx - 1]; count += 1; }
-            if (y + 1 < H && sv[in][ly + 1][lx] == 1) { nu += sf[ly + 1][lx]; count += 1; }
-            if (x > 0 && y - 1 > 0 && sv[in][ly - 1][lx] == 1) { nu += sf[ly - 1][lx]; count += 1; }
-            if (count > 0) {
-                sf[ly][lx] = nu / (float)count;
-                sv[out][ly][lx] = 1;
-            } else {
-                sv[out][ly][lx] = 0;
-            }
+        for (int j = tid; j < count_of[s]; j += EX_THREADS) {
+            const int i = list[first_of[s] + j], ly = i / EX_E, c = i - ly * EX_E, gx = x0 + c, gy = y0 + ly;
+            // Every load first; a face on the image's rim misses a neighbour, and its value is not read by the
+            // faces the tile owns.
+            const int r = min(i + 1, NFC - 1), l = max(i - 1, 0), dn = min(i + EX_E, NFC - 1), up = max(i - EX_E, 0);
+            auto valid = [&](int n) -> bool { return n < OUTSIDE ? n <= s : (n >> (s & 1)) & 1; };
+            const bool vr = gx + 1 < W && c + 1 < EX_E && valid(st[r]), vl = gx - 1 > 0 && gy > 0 && c > 0 && valid(st[l]);
+            const bool vd = gy + 1 < H && ly + 1 < EX_E && valid(st[dn]);
+            const bool vu = gx > 0 && gy - 1 > 0 && ly > 0 && valid(st[up]);
+            const float fr = sf[r], fl = sf[l], fd = sf[dn], fu = sf[up];
+            float nu = 0.0f;  // neighbour order and bounds as the reference
+            nu = vr ? nu + fr : nu;
+            nu = vl ? nu + fl : nu;
+            nu = vd ? nu + fd : nu;
+            nu = vu ? nu + fu : nu;
+            sf[i] = nu / (float)((int)vr + (int)vl + (int)vd + (int)vu);
         }
         __syncthreads();
     }
-    for (int i = tid; i < EX_T * EX_T; i += 256) {
-        const int ly = EX_H + i / EX_T, lx = EX_H + i % EX_T, x = x0 + lx, y = y0 + ly;
-        if ((unsigned)x >= (unsigned)W || (unsigned)y >= (unsigned)H) continue;
-        f.at(x, y) = sf[ly][lx];
-        a.vin[comp].at(x, y) = sv[0][ly][lx];   // after the tenth sweep
-        a.vout[comp].at(x, y) = sv[1][ly][lx];  // after the ninth
+    for (int i = tid; i < EX_T * EX_T; i += EX_THREADS) {
+        const int oy = EX_H + i / EX_T, ox = EX_H + i % EX_T, gx = x0 + ox, gy = y0 + oy;
+        if (gx >= CW || gy >= CH) continue;
+        f.at(gx, gy) = sf[oy * EX_E + ox];
+        vin.at(gx, gy) = st[oy * EX_E + ox] <= 10;  // after the tenth sweep
+        vout.at(gx, gy) = st[oy * EX_E + ox] <= 9;  // after the ninth
     }
 }
 

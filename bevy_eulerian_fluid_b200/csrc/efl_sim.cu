@@ -1158,25 +1158,12 @@ efl_status st_solve_velocity(efl_sim* s) {
 }
 efl_status st_extrapolate(efl_sim* s) {  // render_node.rs:540-608
     Dom d = s->dom();
-    if (d.nx % 64 == 0 && d.ny % 64 == 0) {  // every face covered: one fused launch
-        const int rtx = (d.nx + EX_T - 1) / EX_T, rty = (d.ny + EX_T - 1) / EX_T;
-        k_ls_tile_range<<<dim3(rtx, rty), 256, count_launch(), s->stream>>>(s->ls0, s->d_lsrange, rtx);
-        ExtrapArgs a{{s->u0, s->v0}, {s->uvi, s->vvi}, {s->uvo, s->vvo}, s->ls0, s->d_lsrange, rtx, rty};
-        const dim3 g((d.nx + 1 + EX_T - 1) / EX_T, (d.ny + 1 + EX_T - 1) / EX_T, 2);
-        k_extrapolate_fused<<<g, 256, count_launch(), s->stream>>>(a);
-        LAUNCH_CHECK();
-        return EFL_OK;
-    }
-    dim3 gu = grid2d(d.nx + 1, d.ny, kBlock), gv = grid2d(d.nx, d.ny + 1, kBlock);
-    int xrows = (d.ny / 64) * 64, ycols = (d.nx / 64) * 64;
-    k_init_valid<0><<<gu, kBlock, count_launch(), s->stream>>>(s->uvi, s->ls0, d);
-    k_init_valid<1><<<gv, kBlock, count_launch(), s->stream>>>(s->vvi, s->ls0, d);
-    for (int k = 0; k < 10 / 2; ++k) {
-        k_extrapolate<<<gu, kBlock, count_launch(), s->stream>>>(s->u0, s->uvi, s->uvo, d.nx + 1, xrows);
-        k_extrapolate<<<gu, kBlock, count_launch(), s->stream>>>(s->u0, s->uvo, s->uvi, d.nx + 1, xrows);
-        k_extrapolate<<<gv, kBlock, count_launch(), s->stream>>>(s->v0, s->vvi, s->vvo, ycols, d.ny + 1);
-        k_extrapolate<<<gv, kBlock, count_launch(), s->stream>>>(s->v0, s->vvo, s->vvi, ycols, d.ny + 1);
-    }
+    const int rtx = (d.nx + EX_T - 1) / EX_T, rty = (d.ny + EX_T - 1) / EX_T;
+    k_ls_tile_range<<<dim3(rtx, rty), 256, count_launch(), s->stream>>>(s->ls0, s->d_lsrange, rtx);
+    ExtrapArgs a{{s->u0, s->v0}, {s->uvi, s->vvi}, {s->uvo, s->vvo}, s->ls0, s->d_lsrange, rtx, rty,
+                 {d.nx + 1, (d.nx / 64) * 64}, {(d.ny / 64) * 64, d.ny + 1}};
+    const dim3 g((d.nx + 1 + EX_T - 1) / EX_T, (d.ny + 1 + EX_T - 1) / EX_T, 2);
+    k_extrapolate_fused<<<g, EX_THREADS, count_launch(), s->stream>>>(a);
     LAUNCH_CHECK();
     return EFL_OK;
 }

@@ -1,0 +1,52 @@
+"""The tiled stage kernels at the sizes where a tile, its halo or its masks end, against the CPU oracle, bit for bit:
+the fast iterative method (56 x 32 cells with a 20-cell halo, 10 iterations per launch) and the velocity
+extrapolation (32 x 32 faces with a 10-face halo)."""
+import numpy as np
+import pytest
+
+from bevy_eulerian_fluid_b200 import _capi as capi
+from bevy_eulerian_fluid_b200 import scenes
+
+from .helpers import compare_fields, make_pair
+
+pytestmark = pytest.mark.gpu
+
+
+def _splash(nx, ny, iterations=10):
+    """Water on the left, two droplets (one across a tile corner) and a jet: interfaces in every part of the grid."""
+    cfg = scenes.base_config(nx, ny)
+    cfg.reinit.fim_iterations = iterations
+    r = 0.11 * min(nx, ny)
+    once = [scenes.aabb_source((-0.25 * nx, -0.2 * ny), (0.25 * nx, 0.3 * ny)),
+            scenes.circle_source((56 - 0.5 * nx, 0.5 * ny - 32), r), scenes.circle_source((0.3 * nx, 0.2 * ny), r)]
+    jet = [scenes.circle_source((0.1 * nx, 0.3 * ny), 0.06 * min(nx, ny), velocity=(25.0, -40.0))]
+    return scenes.Scene(f"splash_{nx}x{ny}", cfg, oneshot=once, continuous=jet)
+
+
+@pytest.mark.parametrize("nx,ny,iterations", [(64, 64, 10), (56, 32, 10), (112, 64, 1), (120, 72, 9), (168, 40, 11),
+                                              (64, 200, 20), (200, 136, 25), (128, 96, 0), (16, 16, 10), (24, 440, 10),
+                                              (704, 448, 10)])
+def test_tiled_stages_bit_exact(oracle_api, gpu_api, nx, ny, iterations):
+    o, g = make_pair(_splash(nx, ny, iterations), oracle_api, gpu_api)
+    for _ in range(7):
+        o.step(scenes.DT)
+        g.step(scenes.DT)
+    assert not compare_fields(g, o)
+
+
+@pytest.mark.parametrize("nx,ny", [(200, 136), (128, 64)])
+def test_extrapolation_reads_flags_outside_the_dispatch(oracle_api, gpu_api, nx, ny):
+    """Faces beyond floor(n / 64) * 64 keep whatever flags they hold, and the sweeps read them."""
+    o, g = make_pair(_splash(nx, ny), oracle_api, gpu_api)
+    rng = np.random.default_rng(5)
+    for s in (o, g):
+        s.step(scenes.DT)
+        s.step(scenes.DT)
+    for f in (capi.FIELD_U_VALID, capi.FIELD_V_VALID):
+        flags = (rng.random(o.get(f).shape) < 0.3).astype(np.int32)
+        o.set(f, flags)
+        g.set(f, flags)
+    for _ in range(3):
+        for s in (o, g):
+            s.step(scenes.DT)
+    assert not compare_fields(g, o)
