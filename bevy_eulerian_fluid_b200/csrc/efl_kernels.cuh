@@ -1248,262 +1248,238 @@ __global__ void k_jfa_sdf(P2 seeds, PF ls1, PF ls0, Dom d) {
     ls0.st(x, y, sdf * (level < 0.0f ? -1.0f : 1.0f));
 }
 
-// fast_iterative_method/initialize.wgsl:10-40
-__global__ void k_fim_init(PF ls1, PF ls0, PU lab0, Dom d) {
-    int x = gx(), y = gy();
-    if (x >= d.cx() || y >= d.cy()) return;
-    float level = ls1.ld(x, y);
-    const int ox[4] = {-1, 1, 0, 0}, oy[4] = {0, 0, -1, 1};
-    bool src = false;
-    for (int i = 0; i < 4 && !src; ++i) {
-        int ax = x + ox[i], ay = y + oy[i];
-        if (ax >= 0 && ay >= 0 && ax < d.nx && ay < d.ny && level * ls1.ld(ax, ay) <= 0.0f) src = true;
-    }
-    if (src) {
-        ls0.st(x, y, level);
-        lab0.st(x, y, LABEL_SOURCE);
-    } else {
-        ls0.st(x, y, wsign(level) * FIM_LARGE);
-        lab0.st(x, y, LABEL_NONE);
-    }
+// fast_iterative_method/update.wgsl:13-54 in its deterministic two-phase form (the reference writes neighbours
+// from inside one dispatch, a data race), together with initialize.wgsl:10-40 and
+// initialize_active_label.wgsl:8-40, in ONE launch per FIM_HALO / 2 iterations.  Phase A: active cells update
+// from the iteration-start phi and flag convergence.  Phase B: an inactive cell next to a cell that converged
+// in A is re-solved from the post-A phi and activated, with the sign of the raster-last converged neighbour
+// (down, right, left, up).
+//
+// A CTA owns FIM_TW x FIM_TH cells and holds them with a halo of FIM_HALO cells in shared memory.  One
+// iteration's result at a cell depends on cells at most 2 away (phase A reads radius 1, phase B reads phase A's
+// result at radius 1), so values go wrong only near the image's edge, 2 cells deeper per iteration: after
+// FIM_HALO / 2 iterations the owned cells are exact.  INIT: the start state comes from the advected level set
+// (source cells, sign * large elsewhere, active neighbours of the sources); otherwise from the planes (S, L) of
+// the launch before, which must be another pair than (SD, LD): a CTA that starts late must still see its
+// neighbours' values of the launch's start.
+//
+// The cells that change form a thin band around the interface, and on small grids the work is latency- and
+// issue-bound (a few CTAs and a chain of 10 iterations).  So the CTA keeps the active cells as a list in shared
+// memory, one cell per thread, and the labels as bit masks, one word per 32 columns of an image row, one word per
+// thread: phase A solves the listed cells and marks those that converged, the words beside converged cells give
+// the candidates of phase B (each once, whatever the number of its converged neighbours), and phase B solves the
+// listed candidates.  The images s and t differ at active cells alone: A writes t there, B copies those back and
+// writes s where it activates, and A rewrites t at every active cell before B reads it.  The order of a list does
+// not matter: a phase reads one image and writes the other.
+// The start state costs no launch of its own.  Before: two launches for the start state, then 20 per-phase
+// launches (2.0 + 3.0 us each at 256^2) or, on large grids, a 72 x 72 image with every cell visited in every
+// phase (181 us at 2048^2, 379 us at 4096^2).
+constexpr int FIM_HALO = 20, FIM_TW = 56, FIM_TH = 32, FIM_THREADS = 768;
+constexpr int FIM_IW = FIM_TW + 2 * FIM_HALO, FIM_IH = FIM_TH + 2 * FIM_HALO, FIM_NW = FIM_IW / 32;
+constexpr int FIM_PW = FIM_IW + 2;                        // row pitch of s and t: a ring of large values
+constexpr int FIM_LW = FIM_IW + 4, FIM_LH = FIM_IH + 4;   // staged level set: the image and two cells around it
+constexpr int FIM_CELLS = ((FIM_IH + 2) * FIM_PW + 3) / 4 * 4;
+constexpr int FIM_TBUF = FIM_CELLS > FIM_LW * FIM_LH ? FIM_CELLS : FIM_LW * FIM_LH;
+constexpr int FIM_WORDS = FIM_IH * FIM_NW, FIM_LIST = FIM_IW * FIM_IH;
+typedef unsigned FimMask[FIM_IH + 2][FIM_NW + 2];  // [row + 1][word + 1]: a rim of zeros
+struct FimTile {
+    float s[FIM_CELLS], t[FIM_TBUF];  // t: the staged level set first
+    FimMask src, act, conv[2];        // source, active (converged ones included), converged in even / odd iterations
+    int count[2], ncand;
+    unsigned short list[2][FIM_LIST], cand[FIM_LIST];
+};
+constexpr size_t FIM_SMEM = sizeof(FimTile);
+// update.wgsl:56-83 on an image with a ring of large values (abs_get_phi gives that outside the domain)
+EFL_DEV float fim_solve(const float* a, int i) {
+    const float xm = fminf(fabsf(a[i - 1]), fabsf(a[i + 1]));
+    const float ym = fminf(fabsf(a[i - FIM_PW]), fabsf(a[i + FIM_PW]));
+    const float d = xm - ym;
+    const bool one = d > SQRT2_F || d < -SQRT2_F;  // from one side only (selects: no divergent chains)
+    const float both = 0.5f * (xm + ym + sqrtf(one ? 1.0f : 2.0f - d * d));
+    return one ? (d > SQRT2_F ? ym : xm) + 1.0f : both;
 }
-// fast_iterative_method/initialize_active_label.wgsl:8-40.  tile_active (optional): set to 1 for every
-// 32 x 32 tile (FIM_TILE) that holds an active cell.
-__global__ void k_fim_active(PU lab0, PU lab, Dom d, unsigned* tile_active, int tiles_x) {
-    int x = gx(), y = gy();
-    if (x >= d.cx() || y >= d.cy()) return;
-    if (lab0.ld(x, y) == LABEL_SOURCE) {
-        lab.st(x, y, LABEL_SOURCE);
-        return;
-    }
-    const int ox[4] = {-1, 1, 0, 0}, oy[4] = {0, 0, -1, 1};
-    uint32_t out = LABEL_NONE;
-    for (int i = 0; i < 4; ++i) {
-        int ax = x + ox[i], ay = y + oy[i];
-        if (ax >= 0 && ay >= 0 && ax < d.nx && ay < d.ny && lab0.ld(ax, ay) == LABEL_SOURCE) {
-            out = LABEL_ACTIVE;
-            break;
-        }
-    }
-    lab.st(x, y, out);
-    if (tile_active && out == LABEL_ACTIVE) {
-        unsigned* f = &tile_active[(y / 32) * tiles_x + x / 32];
-        if (*f == 0u) atomicOr(f, 1u);
-    }
+// Appends i to list for the lanes with `take` (a whole warp calls it).
+EFL_DEV void fim_append(unsigned short* list, int* count, bool take, int i) {
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (!m) return;
+    const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
+    int at = 0;
+    if (lane == lead) at = atomicAdd(count, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, lead);
+    if (take) list[at + __popc(m & ((1u << lane) - 1u))] = (unsigned short)i;
 }
-// fast_iterative_method/update.wgsl:56-83
-EFL_DEV float abs_get_phi(const PF& p, int x, int y) {
-    if (x < 0 || y < 0 || x >= p.w || y >= p.h) return FIM_LARGE;
-    return fabsf(p.at(x, y));
-}
-EFL_DEV float solve_quadratic_2d(const PF& p, int x, int y) {
-    float xm = fminf(abs_get_phi(p, x - 1, y), abs_get_phi(p, x + 1, y));
-    float ym = fminf(abs_get_phi(p, x, y - 1), abs_get_phi(p, x, y + 1));
-    float d = xm - ym;
-    if (d > SQRT2_F) return ym + 1.0f;
-    if (d < -SQRT2_F) return xm + 1.0f;
-    return 0.5f * (xm + ym + sqrtf(2.0f - d * d));
-}
-// Deterministic two-phase form of fast_iterative_method/update.wgsl:13-54
-// (the reference writes neighbours from inside one dispatch, a data race).
-// Phase A: active cells update from the iteration-start phi and flag
-// convergence.  Phase B: an inactive cell next to a cell that converged in
-// A is re-solved from the post-A phi and activated, with the sign of the
-// raster-last converged neighbour (down, right, left, up).
-__global__ void k_fim_phase_a(PF S, PU L, PF T, PU LT, Dom d) {
-    int x = gx(), y = gy();
-    if (x >= d.cx() || y >= d.cy()) return;
-    uint32_t l = L.at(x, y);
-    float p = S.at(x, y);
-    if (l != LABEL_ACTIVE) {
-        T.at(x, y) = p;
-        LT.at(x, y) = l;
-        return;
-    }
-    float q = solve_quadratic_2d(S, x, y) * wsign(p);
-    T.at(x, y) = q;
-    LT.at(x, y) = (fabsf(p - q) > FIM_EPS) ? LABEL_ACTIVE : LABEL_CONVERGED;
-}
-__global__ void k_fim_phase_b(PF T, PU LT, PF S, PU L, Dom d) {
-    int x = gx(), y = gy();
-    const int W = d.cx(), H = d.cy();
-    if (x >= W || y >= H) return;
-    uint32_t l = LT.at(x, y);
-    float t = T.at(x, y);
-    if (l == LABEL_NONE) {
-        const int wo[4][2] = {{0, 1}, {1, 0}, {-1, 0}, {0, -1}};
-        int wx = -1, wy = -1;
-        for (int k = 0; k < 4; ++k) {
-            int ax = x + wo[k][0], ay = y + wo[k][1];
-            if (ax >= 0 && ay >= 0 && ax < W && ay < H && LT.at(ax, ay) == LABEL_CONVERGED) {
-                wx = ax;
-                wy = ay;
-                break;
-            }
-        }
-        if (wx >= 0) {
-            float pn = fabsf(t);
-            float qn = solve_quadratic_2d(T, x, y);
-            if (pn > qn) {
-                S.at(x, y) = qn * wsign(T.at(wx, wy));
-                L.at(x, y) = LABEL_ACTIVE;
-                return;
-            }
-        }
-        S.at(x, y) = t;
-        L.at(x, y) = LABEL_NONE;
-    } else {
-        S.at(x, y) = t;
-        L.at(x, y) = l == LABEL_CONVERGED ? LABEL_NONE : l;
-    }
-}
-
-// Iterations of the two-phase FIM update (k_fim_phase_a then k_fim_phase_b,
-// `iters` times) in one launch, temporally blocked: a CTA holds its 32 x 32
-// tile plus a halo of HALO cells in shared memory and runs the iterations
-// there.  One iteration's result at a cell depends on cells at most 2 away
-// (phase A reads radius 1, phase B reads phase A's result at radius 1), so
-// values go wrong only near the image edge, 2 cells deeper per iteration:
-// with iters <= HALO / 2 the owned tile is exact.  A cell changes only while
-// it is active, and activity spreads one cell per iteration, so a tile whose
-// image holds no active cell is left untouched (most of a large grid, away
-// from the interface): such CTAs read the labels and leave.  Two halos: 20
-// (the 10 iterations in one launch; large grids, where most tiles leave at
-// once) and 4 (2 iterations per launch, 1.56x the owned cells in the image;
-// small grids, where a 72 x 72 image per 32 x 32 tile would be 5x the work).
-constexpr int FIM_TILE = 32, FIM_HALO = 20, FIM_THREADS = 512, FIM_HALO_NARROW = 4, FIM_THREADS_NARROW = 256;
-__host__ __device__ constexpr size_t fim_smem(int halo) {
-    return (size_t)4 * (FIM_TILE + 2 * halo) * (FIM_TILE + 2 * halo) * 4;
-}
-constexpr size_t FIM_SMEM = fim_smem(FIM_HALO);
-// Each launch reads (S, L) and writes its tiles into (SD, LD), another pair of planes: a CTA that started late
-// must still see its neighbours' values of the launch's start in its halo.  A tile that leaves early copies its
-// cells across.  tile_active: the flags k_fim_active left (a tile whose 3 x 3 neighbourhood holds no active
-// cell has none in its image, HALO < FIM_TILE, and leaves at once); valid for the first launch only.
-template <int HALO, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_fim_tiled(PF S, PU L, PF SD, PU LD, Dom d, int iters, int tiles_x,
-                                                       const unsigned* tile_active) {
+template <bool INIT>
+__global__ void __launch_bounds__(FIM_THREADS, 2) k_fim(PF S, PU L, PF SD, PU LD, Dom d, int iters, int tiles_x) {
+    static_assert(FIM_IW % 32 == 0 && 2 * FIM_WORDS <= FIM_THREADS && 2 * (FIM_IH + 2) <= FIM_THREADS,
+                  "image rows of whole words, two threads per word, one per rim cell");
     extern __shared__ __align__(16) unsigned char fim_raw[];
-    constexpr int FIM_IMG = FIM_TILE + 2 * HALO, N = FIM_IMG * FIM_IMG;
-    static_assert(HALO < FIM_TILE, "the image lies within the 3 x 3 tiles around the owned one");
-    auto copy_across = [&]() {  // the owned tile unchanged
-        const int tx0 = (int)(blockIdx.x % tiles_x) * FIM_TILE, ty0 = (int)(blockIdx.x / tiles_x) * FIM_TILE;
-        for (int i = threadIdx.x; i < FIM_TILE * FIM_TILE; i += THREADS) {
-            const int gx = tx0 + i % FIM_TILE, gy = ty0 + i / FIM_TILE;
-            if (gx < d.nx && gy < d.ny) {
-                SD.at(gx, gy) = S.at(gx, gy);
-                LD.at(gx, gy) = L.at(gx, gy);
+    FimTile& T = *reinterpret_cast<FimTile*>(fim_raw);
+    float *s = T.s, *t = T.t;
+    constexpr int WARPS = FIM_THREADS / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int x0 = (int)(blockIdx.x % tiles_x) * FIM_TW - FIM_HALO, y0 = (int)(blockIdx.x / tiles_x) * FIM_TH - FIM_HALO;
+    const int W = d.nx, H = d.ny;  // the dispatch domain (sizes are multiples of 8) and the planes' extent
+    for (int i = tid; i < 4 * (int)(sizeof(FimMask) / 4); i += FIM_THREADS) (&T.src[0][0])[i] = 0u;
+    if (tid < 2) T.count[tid] = 0;
+    // The ring of s.
+    for (int i = tid; i < 2 * FIM_PW + 2 * FIM_IH; i += FIM_THREADS) {
+        const int at = i < FIM_PW       ? i
+                       : i < 2 * FIM_PW ? (FIM_IH + 1) * FIM_PW + i - FIM_PW
+                                        : ((i - 2 * FIM_PW) / 2 + 1) * FIM_PW + (i & 1) * (FIM_PW - 1);
+        s[at] = FIM_LARGE;
+    }
+    if constexpr (INIT) {
+        // The level set, NaN outside the domain: no product with it is <= 0.
+#pragma unroll
+        for (int k = 0; k < (FIM_LW * FIM_LH + FIM_THREADS - 1) / FIM_THREADS; ++k) {
+            const int i = tid + k * FIM_THREADS, gx = x0 - 2 + i % FIM_LW, gy = y0 - 2 + i / FIM_LW;
+            if (i < FIM_LW * FIM_LH)
+                t[i] = (unsigned)gx < (unsigned)W && (unsigned)gy < (unsigned)H ? S.at(gx, gy) : NAN;
+        }
+        __syncthreads();
+        // initialize.wgsl: a source cell has an in-domain neighbour of another sign (or is 0)
+        auto source = [&](const float* q) -> bool {
+            const float l = *q;
+            return (l * q[-1] <= 0.0f) | (l * q[1] <= 0.0f) | (l * q[-FIM_LW] <= 0.0f) | (l * q[FIM_LW] <= 0.0f);
+        };
+#pragma unroll 5
+        for (int it = warp; it < (FIM_IH + 2) * FIM_NW; it += WARPS) {
+            const int r = it / FIM_NW, w = it % FIM_NW, ix = 32 * w + lane;  // image row r - 1
+            const float* q = t + (r + 1) * FIM_LW + ix + 2;
+            const bool sc = source(q);
+            const unsigned b = __ballot_sync(0xffffffffu, sc);
+            if (lane == 0) T.src[r][w + 1] = b;
+            if (r >= 1 && r <= FIM_IH) {
+                const bool in = (unsigned)(x0 + ix) < (unsigned)W && (unsigned)(y0 + r - 1) < (unsigned)H;
+                s[r * FIM_PW + ix + 1] = in ? (sc ? *q : wsign(*q) * FIM_LARGE) : FIM_LARGE;
             }
         }
-    };
-    if (tile_active) {
-        const int tiles_y = (d.ny + FIM_TILE - 1) / FIM_TILE;
-        int any = 0;
-        if (threadIdx.x < 9) {
-            const int tx = (int)(blockIdx.x % tiles_x) - 1 + (int)threadIdx.x % 3;
-            const int ty = (int)(blockIdx.x / tiles_x) - 1 + (int)threadIdx.x / 3;
-            if (tx >= 0 && ty >= 0 && tx < tiles_x && ty < tiles_y) any = tile_active[ty * tiles_x + tx] != 0u;
+        if (tid < 2 * (FIM_IH + 2)) {  // the cells beside the image's first and last column
+            const int r = tid >> 1;
+            if (tid & 1) T.src[r][FIM_NW + 1] = source(t + (r + 1) * FIM_LW + FIM_IW + 2) ? 1u : 0u;
+            else T.src[r][0] = source(t + (r + 1) * FIM_LW + 1) ? 0x80000000u : 0u;
         }
-        if (!__syncthreads_or(any)) {
-            copy_across();
-            return;
+    } else {
+        for (int it = warp; it < FIM_WORDS; it += WARPS) {
+            const int r = it / FIM_NW + 1, w = it % FIM_NW, gx = x0 + 32 * w + lane, gy = y0 + r - 1;
+            uint32_t l = LABEL_NONE;
+            float v = FIM_LARGE;
+            if ((unsigned)gx < (unsigned)W && (unsigned)gy < (unsigned)H) {
+                l = L.at(gx, gy);
+                v = S.at(gx, gy);
+            }
+            s[r * FIM_PW + 32 * w + lane + 1] = v;
+            const unsigned b = __ballot_sync(0xffffffffu, l == LABEL_SOURCE);
+            const unsigned a = __ballot_sync(0xffffffffu, l == LABEL_ACTIVE);
+            if (lane == 0) {
+                T.src[r][w + 1] = b;
+                T.act[r][w + 1] = a;
+            }
         }
-    }
-    float* s = reinterpret_cast<float*>(fim_raw);
-    float* t = s + N;
-    uint32_t* l = reinterpret_cast<uint32_t*>(t + N);
-    uint32_t* lt = l + N;
-    const int x0 = (int)(blockIdx.x % tiles_x) * FIM_TILE - HALO, y0 = (int)(blockIdx.x / tiles_x) * FIM_TILE - HALO;
-    const int W = d.nx, H = d.ny;  // the dispatch domain (sizes are multiples of 8) and the planes' extent
-    int act = 0;
-    for (int i = threadIdx.x; i < N; i += THREADS) {
-        const int gx = x0 + i % FIM_IMG, gy = y0 + i / FIM_IMG;
-        const bool in = gx >= 0 && gy >= 0 && gx < W && gy < H;
-        const uint32_t lv = in ? L.at(gx, gy) : LABEL_NONE;
-        l[i] = lv;
-        act |= lv == LABEL_ACTIVE;
-    }
-    if (!__syncthreads_or(act)) {
-        copy_across();
-        return;
-    }
-    for (int i = threadIdx.x; i < N; i += THREADS) {
-        const int gx = x0 + i % FIM_IMG, gy = y0 + i / FIM_IMG;
-        s[i] = (gx >= 0 && gy >= 0 && gx < W && gy < H) ? S.at(gx, gy) : 0.0f;
     }
     __syncthreads();
-    // |phi| of a neighbour: FIM_LARGE outside the domain (update.wgsl:56-60) and, where the image ends,
-    // a stand-in whose error stays in the halo.
-    auto absphi = [&](const float* a, int ix, int iy) -> float {
-        const int gx = x0 + ix, gy = y0 + iy;
-        if (gx < 0 || gy < 0 || gx >= W || gy >= H) return FIM_LARGE;
-        if (ix < 0 || iy < 0 || ix >= FIM_IMG || iy >= FIM_IMG) return FIM_LARGE;
-        return fabsf(a[iy * FIM_IMG + ix]);
+    // This thread's half of a word (the cells of a word are listed by two threads): the cells in the domain, and
+    // (row, word) of the masks.
+    const int wi = tid >> 1, mr = min(wi / FIM_NW, FIM_IH - 1) + 1, mw = wi % FIM_NW + 1;
+    const unsigned mine = tid & 1 ? 0xffff0000u : 0xffffu;
+    const int wx = x0 + 32 * (mw - 1), cell0 = mr * FIM_PW + 32 * (mw - 1) + 1;
+    const bool word = wi < FIM_WORDS && y0 + mr - 1 >= 0 && y0 + mr - 1 < H;
+    const unsigned dom = !word || wx >= W || wx <= -32
+                             ? 0u
+                             : (W - wx >= 32 ? ~0u : (1u << (W - wx)) - 1u) & (wx >= 0 ? ~0u : ~0u << -wx);
+    // Lists the cells of bits m, the word's; cells of one word stay together.
+    auto list_bits = [&](unsigned short* list, int* count, unsigned m) {
+        if (!m) return;
+        int at = atomicAdd(count, __popc(m));
+        for (; m; m &= m - 1) list[at++] = (unsigned short)(cell0 + __ffs(m) - 1);
     };
-    auto quad = [&](const float* a, int ix, int iy) -> float {  // solve_quadratic_2d (update.wgsl:62-83)
-        const float xm = fminf(absphi(a, ix - 1, iy), absphi(a, ix + 1, iy));
-        const float ym = fminf(absphi(a, ix, iy - 1), absphi(a, ix, iy + 1));
-        const float dd = xm - ym;
-        if (dd > SQRT2_F) return ym + 1.0f;
-        if (dd < -SQRT2_F) return xm + 1.0f;
-        return 0.5f * (xm + ym + sqrtf(2.0f - dd * dd));
+    auto beside = [&](const FimMask& M) -> unsigned {  // the word's cells with a marked neighbour
+        const unsigned c = M[mr][mw];
+        return M[mr + 1][mw] | M[mr - 1][mw] | (c >> 1) | (M[mr][mw + 1] << 31) | (c << 1) | (M[mr][mw - 1] >> 31);
     };
-    for (int it = 0; it < iters; ++it) {
-        for (int i = threadIdx.x; i < N; i += THREADS) {  // phase A
-            const int ix = i % FIM_IMG, iy = i / FIM_IMG;
-            const uint32_t lv = l[i];
-            const float p = s[i];
-            if (lv != LABEL_ACTIVE) {
-                t[i] = p;
-                lt[i] = lv;
-            } else {
-                const float q = quad(s, ix, iy) * wsign(p);
-                t[i] = q;
-                lt[i] = (fabsf(p - q) > FIM_EPS) ? LABEL_ACTIVE : LABEL_CONVERGED;
-            }
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < N; i += THREADS) {  // phase B
-            const int ix = i % FIM_IMG, iy = i / FIM_IMG;
-            const int gx = x0 + ix, gy = y0 + iy;
-            const uint32_t lv = lt[i];
-            const float tv = t[i];
-            if (lv == LABEL_NONE) {
-                const int wo[4][2] = {{0, 1}, {1, 0}, {-1, 0}, {0, -1}};
-                int wi = -1;
-                for (int k = 0; k < 4; ++k) {
-                    const int ax = ix + wo[k][0], ay = iy + wo[k][1];
-                    const int bx = gx + wo[k][0], by = gy + wo[k][1];
-                    if (bx >= 0 && by >= 0 && bx < W && by < H && ax >= 0 && ay >= 0 && ax < FIM_IMG &&
-                        ay < FIM_IMG && lt[ay * FIM_IMG + ax] == LABEL_CONVERGED) {
-                        wi = ay * FIM_IMG + ax;
-                        break;
-                    }
-                }
-                if (wi >= 0) {
-                    const float pn = fabsf(tv);
-                    const float qn = quad(t, ix, iy);
-                    if (pn > qn) {
-                        s[i] = qn * wsign(t[wi]);
-                        l[i] = LABEL_ACTIVE;
-                        continue;
-                    }
-                }
-                s[i] = tv;
-                l[i] = LABEL_NONE;
-            } else {
-                s[i] = tv;
-                l[i] = lv == LABEL_CONVERGED ? LABEL_NONE : lv;
-            }
-        }
-        __syncthreads();
+    if (word) {
+        // initialize_active_label.wgsl: every other in-domain cell beside a source cell
+        const unsigned a = INIT ? beside(T.src) & ~T.src[mr][mw] & dom : T.act[mr][mw];
+        if (INIT && (tid & 1)) T.act[mr][mw] = a;
+        list_bits(T.list[0], &T.count[0], a & mine);
     }
-    for (int i = threadIdx.x; i < FIM_TILE * FIM_TILE; i += THREADS) {
-        const int ix = HALO + i % FIM_TILE, iy = HALO + i / FIM_TILE;
+    __syncthreads();
+    // A cell changes only while it is active, so an image without an active cell (most of a large grid) stays.
+    int n = T.count[0];
+    if (n) {
+        for (int i = tid; i < FIM_CELLS / 4; i += FIM_THREADS)
+            reinterpret_cast<float4*>(t)[i] = reinterpret_cast<const float4*>(s)[i];
+        __syncthreads();
+        for (int k = 0; k < iters; ++k) {
+            const int cur = k & 1, nxt = cur ^ 1;
+            FimMask& conv = T.conv[cur];
+            // phase A
+            for (int j = tid; j < (n + 31) / 32 * 32; j += FIM_THREADS) {
+                bool still = false;
+                int i = 0;
+                if (j < n) {
+                    i = T.list[cur][j];
+                    const float p = s[i];
+                    const float q = fim_solve(s, i) * wsign(p);
+                    t[i] = q;
+                    still = fabsf(p - q) > FIM_EPS;
+                    if (!still) {
+                        const int r = i / FIM_PW, x = i - r * FIM_PW - 1;
+                        atomicOr(&conv[r][(x >> 5) + 1], 1u << (x & 31));
+                    }
+                }
+                fim_append(T.list[nxt], &T.count[nxt], still, i);
+            }
+            if (tid == 0) T.ncand = 0;
+            __syncthreads();
+            // phase B: inactive cells beside a converged one
+            if (word) {
+                const unsigned a = T.act[mr][mw];
+                list_bits(T.cand, &T.ncand, beside(conv) & ~(a | T.src[mr][mw]) & dom & mine);
+            }
+            for (int j = tid; j < n; j += FIM_THREADS) {
+                const int i = T.list[cur][j];
+                s[i] = t[i];
+            }
+            __syncthreads();
+            const int nc = T.ncand;
+            if (word && (tid & 1)) atomicAnd(&T.act[mr][mw], ~conv[mr][mw]);  // free again
+            for (int j = tid; j < (nc + 31) / 32 * 32; j += FIM_THREADS) {
+                bool fresh = false;
+                int c = 0;
+                if (j < nc) {
+                    c = T.cand[j];
+                    const float qn = fim_solve(t, c);
+                    if (fabsf(t[c]) > qn) {
+                        const int r = c / FIM_PW, x = c - r * FIM_PW - 1, w = (x >> 5) + 1, b = x & 31;
+                        const unsigned right = (conv[r][w] >> 1) | (conv[r][w + 1] << 31);
+                        const unsigned left = (conv[r][w] << 1) | (conv[r][w - 1] >> 31);
+                        const int from = (conv[r + 1][w] >> b) & 1u ? c + FIM_PW
+                                         : (right >> b) & 1u        ? c + 1
+                                         : (left >> b) & 1u         ? c - 1
+                                                                    : c - FIM_PW;
+                        s[c] = qn * wsign(t[from]);
+                        atomicOr(&T.act[r][w], 1u << b);
+                        fresh = true;
+                    }
+                }
+                fim_append(T.list[nxt], &T.count[nxt], fresh, c);
+            }
+            if (tid < FIM_WORDS) T.conv[nxt][tid / FIM_NW + 1][tid % FIM_NW + 1] = 0u;
+            if (tid == 0) T.count[cur] = 0;
+            __syncthreads();
+            n = T.count[nxt];
+        }
+    }
+    for (int i = tid; i < FIM_TW * FIM_TH; i += FIM_THREADS) {
+        const int ix = FIM_HALO + i % FIM_TW, iy = FIM_HALO + i / FIM_TW;
         const int gx = x0 + ix, gy = y0 + iy;
         if (gx < W && gy < H) {
-            SD.at(gx, gy) = s[iy * FIM_IMG + ix];
-            LD.at(gx, gy) = l[iy * FIM_IMG + ix];
+            const int w = (ix >> 5) + 1, b = ix & 31;
+            SD.at(gx, gy) = s[(iy + 1) * FIM_PW + ix + 1];
+            LD.at(gx, gy) = (T.src[iy + 1][w] >> b) & 1u   ? LABEL_SOURCE
+                            : (T.act[iy + 1][w] >> b) & 1u ? LABEL_ACTIVE
+                                                           : LABEL_NONE;
         }
     }
 }

@@ -108,7 +108,7 @@ struct efl_sim {
     // fields (see efl_kernels.cuh for the layout)
     PF u0, u1, v0, v1, us, vs, ls_s, div, p0, p1, ls0, ls1, fu, fv, phiT, r0;
     PI sid, uvi, uvo, vvi, vvo;
-    PU lab0, lab, labT, upd;
+    PU lab, labT, upd;
     P2 grad, seeds[2], srcvel;
     int seeds_final = 0;
     std::vector<Level> mg;      // reference fixed-count solve (f32 iterate)
@@ -124,7 +124,6 @@ struct efl_sim {
     double2* d_partials = nullptr;
     int n_partials = 0;
     float2* d_lsrange = nullptr;     // level-set (min, max) per 32 x 32 cell tile (fused extrapolation)
-    unsigned* d_fimtiles = nullptr;  // per 32 x 32 tile: holds an active cell at the start of the FIM iterations
     double* d_norms = nullptr;
     double* h_norms = nullptr;  // pinned
     unsigned long long* d_count = nullptr;
@@ -144,7 +143,6 @@ struct efl_sim {
     PF mix_d2{};       // second correction buffer (batched solve)
     PF xbuf{};         // second halo-exchange plane of the persistent solves, allocated on first use
     bool owns_stream = true;
-    bool batch_member = false;  // its stages run beside the other simulations' (a batch's fan-out)
     float* d_vel = nullptr;  // velocity-magnitude partials (efl_velocity_magnitude)
     int cap_vel = 0;
     efl_rigid_body* d_rigid = nullptr;  // device-integrated bodies (efl_set_rigid_bodies)
@@ -325,32 +323,21 @@ std::vector<int> jfa_steps(int nx, int ny) {  // jump_flooding.rs:201-209
     return st;
 }
 
-// The tiled FIM kernel's dynamic shared memory (above the 48 KB default), set once per device.
-bool fim_tiled_ready() {
+// The FIM kernels' dynamic shared memory (above the 48 KB default), set once per device.
+bool fim_ready() {
     int dev = 0;
     cudaGetDevice(&dev);
     static int state[64] = {};  // 0 unknown, 1 ready, 2 refused
     if (dev < 0 || dev >= 64) return false;
     if (!state[dev]) {
-        state[dev] = cudaFuncSetAttribute(k_fim_tiled<FIM_HALO, FIM_THREADS>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIM_SMEM) ==
-                             cudaSuccess
-                         ? 1
-                         : 2;
+        const bool ok = cudaFuncSetAttribute(k_fim<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIM_SMEM) ==
+                            cudaSuccess &&
+                        cudaFuncSetAttribute(k_fim<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIM_SMEM) ==
+                            cudaSuccess;
+        state[dev] = ok ? 1 : 2;
         cudaGetLastError();
     }
     return state[dev] == 1;
-}
-
-// Which FIM form runs: EFL_FIM_TILED=0 the per-phase launches, =1 the temporally blocked kernel with the
-// 20-cell halo (10 iterations per launch), =2 the one with the 4-cell halo (2 per launch), at every size; unset
-// (or anything else) the size rule in st_reinit.  All forms give bit-identical level sets.
-int fim_form_override() {
-    static const int v = [] {
-        const char* e = std::getenv("EFL_FIM_TILED");
-        return e && e[0] >= '0' && e[0] <= '2' && !e[1] ? e[0] - '0' : -1;
-    }();
-    return v;
 }
 
 efl_status st_reinit(efl_sim* s) {  // reinitialize_levelset.rs:162-243
@@ -366,45 +353,23 @@ efl_status st_reinit(efl_sim* s) {  // reinitialize_levelset.rs:162-243
         s->seeds_final = src;
         k_jfa_sdf<<<g, kBlock, count_launch(), s->stream>>>(s->seeds[src], s->ls1, s->ls0, d);
     } else {
-        const int tx = (d.nx + FIM_TILE - 1) / FIM_TILE, ty = (d.ny + FIM_TILE - 1) / FIM_TILE;
-        // The wide halo pays where the grid is large and the interface a small part of it (C3: 4096^2: one
-        // launch, most tiles leave at once).  On small grids a simulation stepped alone is latency-bound and
-        // takes the per-phase launches (each shorter than a tiled launch); a batch member, whose launches run
-        // beside the other simulations', takes the narrow halo (a quarter of the launches, a fifth of the
-        // traffic).
-        const int force = fim_form_override();
-        int form = force >= 0 ? force : tx * ty >= 4 * s->solver.num_sms ? 1 : s->batch_member ? 2 : 0;
-        if (form == 1 && !fim_tiled_ready()) form = 2;
+        if (!fim_ready()) return set_err(s, EFL_ERR_CUDA, "fast iterative method: shared-memory attribute refused");
+        const int tx = (d.nx + FIM_TW - 1) / FIM_TW, ty = (d.ny + FIM_TH - 1) / FIM_TH;
         const uint32_t iters = s->cfg.reinit.fim_iterations;
-        const int per = form == 1 ? FIM_HALO / 2 : FIM_HALO_NARROW / 2;
-        const int launches = form ? (int)((iters + per - 1) / per) : 0;
-        // The tiled launches alternate between (ls0, lab) and (phiT, labT) and must end in (ls0, lab): the
-        // start state goes into the pair that makes the last launch land there.
+        constexpr uint32_t per = FIM_HALO / 2;
+        const uint32_t launches = std::max<uint32_t>(1, (iters + per - 1) / per);
+        // The launches alternate between (ls0, lab) and (phiT, labT) so that the last one lands in (ls0, lab).
         PF S[2] = {s->ls0, s->phiT};
         PU L[2] = {s->lab, s->labT};
-        const int first = launches & 1;
-        k_fim_init<<<g, kBlock, count_launch(), s->stream>>>(s->ls1, S[first], s->lab0, d);
-        if (form) CU(cudaMemsetAsync(s->d_fimtiles, 0, (size_t)tx * ty * sizeof(unsigned), s->stream));
-        k_fim_active<<<g, kBlock, count_launch(), s->stream>>>(s->lab0, L[first], d, form ? s->d_fimtiles : nullptr,
-                                                                tx);
-        if (form) {  // the iterations, halo / 2 per launch
-            int cur = first;
-            for (uint32_t k = 0; k < iters; k += per, cur ^= 1) {
-                const int n = (int)std::min<uint32_t>(per, iters - k);
-                const unsigned* act = k == 0 ? s->d_fimtiles : nullptr;
-                if (form == 1)
-                    k_fim_tiled<FIM_HALO, FIM_THREADS><<<tx * ty, FIM_THREADS, FIM_SMEM + count_launch(), s->stream>>>(
-                        S[cur], L[cur], S[cur ^ 1], L[cur ^ 1], d, n, tx, act);
-                else
-                    k_fim_tiled<FIM_HALO_NARROW, FIM_THREADS_NARROW>
-                        <<<tx * ty, FIM_THREADS_NARROW, fim_smem(FIM_HALO_NARROW) + count_launch(), s->stream>>>(
-                            S[cur], L[cur], S[cur ^ 1], L[cur ^ 1], d, n, tx, act);
-            }
-        } else {
-            for (uint32_t k = 0; k < s->cfg.reinit.fim_iterations; ++k) {
-                k_fim_phase_a<<<g, kBlock, count_launch(), s->stream>>>(s->ls0, s->lab, s->phiT, s->labT, d);
-                k_fim_phase_b<<<g, kBlock, count_launch(), s->stream>>>(s->phiT, s->labT, s->ls0, s->lab, d);
-            }
+        for (uint32_t k = 0; k < launches; ++k) {
+            const int to = (int)((launches - 1 - k) & 1);
+            const int n = (int)std::min<uint32_t>(per, iters - k * per);
+            if (k == 0)
+                k_fim<true><<<tx * ty, FIM_THREADS, FIM_SMEM + count_launch(), s->stream>>>(s->ls1, L[to], S[to], L[to],
+                                                                                            d, n, tx);
+            else
+                k_fim<false><<<tx * ty, FIM_THREADS, FIM_SMEM + count_launch(), s->stream>>>(S[to ^ 1], L[to ^ 1], S[to],
+                                                                                             L[to], d, n, tx);
         }
     }
     LAUNCH_CHECK();
@@ -1445,7 +1410,6 @@ efl_status efl_create(const efl_config* cfg, efl_sim** out) {
     CTRY(alloc_plane(s, s->uvo, nx + 1, ny, P, R));
     CTRY(alloc_plane(s, s->vvi, nx, ny + 1, P, R));
     CTRY(alloc_plane(s, s->vvo, nx, ny + 1, P, R));
-    CTRY(alloc_plane(s, s->lab0, nx, ny, P, R));
     CTRY(alloc_plane(s, s->lab, nx, ny, P, R));
     CTRY(alloc_plane(s, s->labT, nx, ny, P, R));
     CTRY(alloc_plane(s, s->upd, nx, ny, P, R));
@@ -1459,7 +1423,6 @@ efl_status efl_create(const efl_config* cfg, efl_sim** out) {
     s->n_partials = std::min(1024, std::max(1, (nx * ny + NORM_THREADS - 1) / NORM_THREADS));
     CTRY(alloc_raw(s, s->d_partials, s->n_partials));
     CTRY(alloc_raw(s, s->d_lsrange, (size_t)((nx + EX_T - 1) / EX_T) * ((ny + EX_T - 1) / EX_T)));
-    CTRY(alloc_raw(s, s->d_fimtiles, (size_t)((nx + FIM_TILE - 1) / FIM_TILE) * ((ny + FIM_TILE - 1) / FIM_TILE)));
     CTRY(alloc_raw(s, s->d_norms, 2));
     CTRY(alloc_raw(s, s->d_count, 1));
     if (cudaMallocHost(&s->h_norms, 4 * sizeof(double)) != cudaSuccess)
@@ -2412,7 +2375,6 @@ efl_status efl_batch_create(const efl_config* cfgs, uint32_t n, efl_batch** out)
         cudaStreamDestroy(s->stream);
         s->stream = b->stream;
         s->owns_stream = false;
-        s->batch_member = true;
         b->sims.push_back(s);
         if (ensure_mix_planes(s) != EFL_OK) {
             std::string m = s->err;
