@@ -28,6 +28,7 @@
 #include "efl_unet.cuh"
 #include "efl_pls.cuh"
 #include "efl_slab.cuh"
+#include "efl_vcycle.cuh"
 
 using namespace efl;
 
@@ -138,6 +139,7 @@ struct efl_sim {
     SweepTma tma_pre1;   // TMA maps of the preconditioner's level 1 (error flag shared with tma)
     const float* tma_pre1_x = nullptr;  // level 1's iterate plane the maps were built over
     SweepTma tma_pre;    // TMA maps of the preconditioner's level 0 (error flag shared with tma)
+    DevBuf vc_image[2];           // the coarse levels' geometry in a solve's V-cycles (f32, f64 levels); owned by bufs
     GraphCache gc;                // captured step segments
     uint64_t graph_epoch = 1;     // counts the setters that change kernel arguments
     PF mix_d2{};       // second correction buffer (batched solve)
@@ -602,11 +604,53 @@ efl_status gs_iterations(efl_sim* s, const LevelT<T>& L, float weight, float res
 }
 
 // multi_grid.rs:390-475 (smoother weight 1.0, resolution_scale 2^i: multi_grid.rs:268-270).
-// symmetric (the MGPCG preconditioner): post-smoothing black then red.
+// symmetric (the MGPCG preconditioner): post-smoothing black then red.  geom: VC_GEOM_STORE in the first V-cycle of
+// a solve, VC_GEOM_LOAD in the later ones (the coarse levels' geometry is the same), VC_GEOM_ONCE for a single one.
 template <class T>
-efl_status v_cycle(efl_sim* s, std::vector<LevelT<T>>& mg, size_t i, bool symmetric = false) {
+efl_status v_cycle(efl_sim* s, std::vector<LevelT<T>>& mg, size_t i, bool symmetric = false, int geom = VC_GEOM_ONCE) {
     const efl_projection& P = s->cfg.projection;
     const LevelT<T>& L = mg[i];
+    // The rest in one launch of one cluster, from the first level of at most 256^2 cells whose slabs fit (above, a
+    // level's launches have enough cells to fill the device); long flat levels (more than 1024 columns) that do not
+    // fit take the one-CTA form.
+    if ((int64_t)L.nx * L.ny <= VC_MAX_CELLS) {
+        VcArgs<T> a{};
+        size_t limit = 0, smem = 0;
+        const int nc = vc_cluster_size<T>(&limit);
+        if (nc && vc_plan(mg, i, nc, limit, &a, &smem)) {
+            a.x_zero = i > 0;  // the restriction onto a coarse level starts its iterate at zero
+            a.mode = geom;
+            if (geom != VC_GEOM_ONCE) {
+                DevBuf& im = s->vc_image[sizeof(T) == 8];
+                const size_t bytes = (size_t)nc * a.nimg;
+                if (im.bytes < bytes) {  // the first V-cycle of a solve only: never inside a stream capture
+                    unsigned char* q = nullptr;
+                    TRY(alloc_raw(s, q, bytes));
+                    im.p = q;
+                    im.bytes = bytes;
+                }
+                a.image = (unsigned char*)im.p;
+            }
+            vc_factors(&a, s->U.dx, s->U.rho, s->U.dt);
+            a.pre = (int)P.mg_pre;
+            a.post = (int)P.mg_post;
+            a.coarsest = (int)P.mg_coarsest;
+            a.symmetric = symmetric ? 1 : 0;
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = nc;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3(nc);
+            cfg.blockDim = dim3(VC_THREADS);
+            cfg.dynamicSmemBytes = smem + count_launch();
+            cfg.stream = s->stream;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            CU(cudaLaunchKernelEx(&cfg, k_vcycle_cluster<T>, a));
+            return EFL_OK;
+        }
+    }
     if ((int64_t)L.nx * L.ny <= VT_MAX_CELLS && mg.size() <= VT_MAX_LEVELS) {  // the rest in one launch
         VTailArgs<T> a{};
         for (size_t k = 0; k < mg.size(); ++k) a.lv[k] = mg[k];
@@ -630,7 +674,7 @@ efl_status v_cycle(efl_sim* s, std::vector<LevelT<T>>& mg, size_t i, bool symmet
     k_residual_restrict<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(L, C, s->U.dt, s->U.rho,
                                                                                           scale * s->U.dx);
     LAUNCH_CHECK();
-    TRY(v_cycle(s, mg, i + 1, symmetric));
+    TRY(v_cycle(s, mg, i + 1, symmetric, geom));
     k_prolongation<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(L, C);
     LAUNCH_CHECK();
     return gs_iterations(s, L, 1.0f, scale, P.mg_post, symmetric);
@@ -819,9 +863,9 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
         }
         s->cg_ready = true;
     }
-    // Level 1 of the preconditioner streams through TMA too where it is too large for the single-CTA tail
+    // Level 1 of the preconditioner streams through TMA too where it is too large for the cluster's levels
     // (C3: 2048^2); its maps follow the level's planes, which efl_set_projection may reallocate.
-    if (s->tma.ok && s->mg.size() > 2 && s->alt32_1.p && (int64_t)s->mg[1].nx * s->mg[1].ny > VT_MAX_CELLS &&
+    if (s->tma.ok && s->mg.size() > 2 && s->alt32_1.p && (int64_t)s->mg[1].nx * s->mg[1].ny > VC_MAX_CELLS &&
         s->tma_pre1_x != s->mg[1].x.p) {
         s->tma_pre1.d_err = s->tma.d_err;
         sweep_tma_init(s->tma_pre1, s->mg[1], s->alt32_1);
@@ -851,7 +895,7 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
     // four k_gs_color launches each.
     const bool tma0 = s->tma_pre.ok && P.mg_pre == 2 && P.mg_post == 2 && pre.size() > 1;
     const bool tma1 = tma0 && s->tma_pre1.ok && s->tma_pre1_x == pre[1].x.p && pre.size() > 2;
-    auto precondition = [&]() -> efl_status {  // z = M r, then r . z into totals[2]
+    auto precondition = [&](int geom) -> efl_status {  // z = M r, then r . z into totals[2]
         CU(cudaMemset2DAsync(C.z32.p, (size_t)C.z32.P * sizeof(float), 0, (size_t)nx * sizeof(float), ny, s->stream));
         if (tma0) {
             const float dxs = s->U.dx;  // resolution scale 1 at level 0
@@ -873,20 +917,20 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
                 k_residual_restrict<float><<<grid2d(C2.nx, C2.ny, kBlock), kBlock, count_launch(), s->stream>>>(
                     L1, C2, s->U.dt, s->U.rho, dxs1);
                 LAUNCH_CHECK();
-                TRY(v_cycle(s, pre, 2, true));
+                TRY(v_cycle(s, pre, 2, true, geom));
                 k_prolongation<float><<<grid2d(C2.nx, C2.ny, kBlock), kBlock, count_launch(), s->stream>>>(L1, C2);
                 LAUNCH_CHECK();
                 TRY(tma_sweep_pass(s->tma_pre1, C1.nx, C1.ny, C1.x, 1, s->solver.num_sms, dxs1, s->U.rho, s->U.dt,
                                    1.0f, 2, 0, s->tma.d_err, s->stream));
             } else {
-                TRY(v_cycle(s, pre, 1, true));
+                TRY(v_cycle(s, pre, 1, true, geom));
             }
             k_prolongation<float><<<grid2d(C1.nx, C1.ny, kBlock), kBlock, count_launch(), s->stream>>>(L0, C1);
             LAUNCH_CHECK();
             TRY(tma_sweep_pass(s->tma_pre, nx, ny, C.z32, 1, s->solver.num_sms, dxs, s->U.rho, s->U.dt, 1.0f, 2,
                                0, s->tma.d_err, s->stream));
         } else {
-            TRY(v_cycle(s, pre, 0, true));
+            TRY(v_cycle(s, pre, 0, true, geom));
         }
         cg_sum_enqueue(s, TermDotRZ{C.r, C.z32, M}, 2);
         return EFL_OK;
@@ -901,7 +945,7 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
     if (!(rel <= (double)P.tolerance) && P.max_iterations > 0) {
         k_cg_mask<<<g, kBlock, count_launch(), s->stream>>>(L.x, M, nx, ny);
         k_cg_residual<<<g, kBlock, count_launch(), s->stream>>>(L.x, L.b, C.r, C.r32, M, factor, nx, ny);
-        TRY(precondition());
+        TRY(precondition(VC_GEOM_STORE));
         k_cg_scalar<<<1, 1, count_launch(), s->stream>>>(CG_RZ, C.totals, C.sc);
         k_cg_direction<<<g, kBlock, count_launch(), s->stream>>>(C.p, C.z32, M, C.sc, 1, nx, ny);
         LAUNCH_CHECK();
@@ -914,7 +958,7 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
             k_cg_scalar<<<1, 1, count_launch(), s->stream>>>(CG_ALPHA, C.totals, C.sc);
             k_cg_axpy<<<g, kBlock, count_launch(), s->stream>>>(L.x, C.r, C.r32, C.p, C.ap, M, C.sc, nx, ny);
             cg_sum_enqueue(s, TermNorm{L.x, L.b, M, factor, nx, ny}, 1);
-            TRY(precondition());
+            TRY(precondition(VC_GEOM_LOAD));
             k_cg_scalar<<<1, 1, count_launch(), s->stream>>>(CG_BETA, C.totals, C.sc);
             k_cg_direction<<<g, kBlock, count_launch(), s->stream>>>(C.p, C.z32, M, C.sc, 0, nx, ny);
             LAUNCH_CHECK();
@@ -1092,7 +1136,7 @@ efl_status st_projection(efl_sim* s, efl_step_stats* st) {
             TRY(relative_residual(s, L, &r));
             r0 = r;
             while (!(r <= (double)P.tolerance) && iters < P.max_iterations) {
-                TRY(v_cycle(s, s->mg64, 0));
+                TRY(v_cycle(s, s->mg64, 0, false, iters == 0 ? VC_GEOM_STORE : VC_GEOM_LOAD));
                 ++iters;
                 TRY(relative_residual(s, L, &r));
             }

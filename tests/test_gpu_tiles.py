@@ -50,3 +50,21 @@ def test_extrapolation_reads_flags_outside_the_dispatch(oracle_api, gpu_api, nx,
         for s in (o, g):
             s.step(scenes.DT)
     assert not compare_fields(g, o)
+
+
+@pytest.mark.parametrize("method,tolerance", [(capi.PROJECTION_MULTIGRID, 0.0), (capi.PROJECTION_MULTIGRID, 1e-3),
+                                              (capi.PROJECTION_MGPCG, 1e-5)])
+@pytest.mark.parametrize("nx,ny", [(64, 64), (16, 16), (136, 88), (24, 200), (256, 256), (1024, 32), (328, 264),
+                                   (512, 640)])
+def test_v_cycle_levels_bit_exact(oracle_api, gpu_api, nx, ny, method, tolerance):
+    """The lower levels of a V-cycle in one cluster: slabs of every height, odd coarse sizes, levels gathered in one
+    CTA, f32 (one cycle, the preconditioner) and f64 (iterated cycles)."""
+    sc = _splash(nx, ny)
+    sc.cfg.projection.method = method
+    sc.cfg.projection.tolerance = tolerance
+    sc.cfg.projection.max_iterations = 12
+    o, g = make_pair(sc, oracle_api, gpu_api)
+    for _ in range(4):
+        so, sg = o.step(scenes.DT), g.step(scenes.DT)
+        assert so.pressure_iterations == sg.pressure_iterations
+    assert not compare_fields(g, o)
