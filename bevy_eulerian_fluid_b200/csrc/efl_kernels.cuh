@@ -65,6 +65,13 @@ EFL_DEV float fclamp01(float v) { return fminf(fmaxf(v, 0.0f), 1.0f); }
 EFL_DEV float fclampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 EFL_DEV float wsign(float v) { return v > 0.0f ? 1.0f : (v < 0.0f ? -1.0f : 0.0f); }
 EFL_DEV float wlength(float x, float y) { return sqrtf(x * x + y * y); }
+// a / b with a selected by the caller: a zero a takes the division's slow path, for the whole warp, so lanes whose
+// quotient is not used get another numerator, and the compiler must not see through that selection (20 fixed-count
+// iterations at 256^2: 45 -> 33 us).
+EFL_DEV float div_any(float a, float b) {
+    asm volatile("" : "+f"(a));
+    return a / b;
+}
 EFL_DEV float wmix(float a, float b, float t) { return a * (1.0f - t) + b * t; }
 EFL_DEV int f2i(float v) { return __float2int_rz(v); }  // truncate, saturate, NaN -> 0
 EFL_DEV float2 mat_xy(const float* m, float x, float y) {

@@ -1297,7 +1297,7 @@ EFL_DEV float gs32_update(float cb, float4 w, float den, float p, float pl, floa
     nume = nume + w.y * pr;
     nume = nume + w.z * pu;
     nume = nume + w.w * pd;
-    const float pn = nume / den;
+    const float pn = div_any(upd ? nume : 1.0f, den);
     const float v = wgt * pn + omw * p;
     return upd ? v : (zero ? 0.0f : p);
 }
