@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(VC_THREADS, 1) k_vcycle_cluster(const __grid_c
                             nume = nume + (T)w[p0 + i][q][2] * xu[i];
                             nume = nume + (T)w[p0 + i][q][3] * xd[i];
                             if constexpr (sizeof(T) == 8) pn[i] = nume * dn[p0 + i][q];
-                            else pn[i] = nume / dn[p0 + i][q];
+                            else pn[i] = (upd & (1u << (2 * (p0 + i) + q)) ? nume : T(1)) / dn[p0 + i][q];  // (0 / 1 is slow)
                         }
                     } else {
 #pragma unroll
