@@ -767,38 +767,106 @@ __global__ void k_narrow(Plane<double> x, PF p0) {
     p0.at(i, y) = (float)x.at(i, y);
 }
 
-// shaders/jacobi_iteration.wgsl:39-91 (levelset_solid fractions = face planes)
-__global__ void k_jacobi(PF p_in, PF p_out, PF ls0, PF fu, PF fv, PF div, Uniform U, Dom d) {
-    int x = gx(), y = gy();
-    if (x >= d.cx() || y >= d.cy()) return;
-    float lij = ls0.ld(x, y);
-    float out;
-    if (lij >= 0.0f) {
-        out = 0.0f;
-    } else {
-        float f0 = fu.ld(x, y), f1 = fu.ld(x + 1, y), f2 = fv.ld(x, y), f3 = fv.ld(x, y + 1);
-        if (f0 == 0.0f && f1 == 0.0f && f2 == 0.0f && f3 == 0.0f) {
-            out = p_in.ld(x, y);
-        } else {
-            float p_m = p_in.ld(x - 1, y), p_p = p_in.ld(x + 1, y), p_jm = p_in.ld(x, y - 1), p_jp = p_in.ld(x, y + 1);
-            float l_m = ls0.ld(x - 1, y), l_p = ls0.ld(x + 1, y), l_jm = ls0.ld(x, y - 1), l_jp = ls0.ld(x, y + 1);
-            float ff_m = fminf(0.0f, l_m / lij), ff_p = fminf(0.0f, l_p / lij);
-            float ff_jm = fminf(0.0f, l_jm / lij), ff_jp = fminf(0.0f, l_jp / lij);
-            float coef = f0 * (1.0f - ff_m) + f1 * (1.0f - ff_p) + f2 * (1.0f - ff_jm) + f3 * (1.0f - ff_jp);
-            if (fabsf(coef) < 1.0e-6f) {
-                out = 0.0f;
-            } else {
-                float div_ij = div.ld(x, y);
-                float factor = U.dx * U.rho / U.dt;
-                float d00 = f0 * (ff_m >= 0.0f ? 1.0f : 0.0f) * p_m;
-                float d10 = f1 * (ff_p >= 0.0f ? 1.0f : 0.0f) * p_p;
-                float d01 = f2 * (ff_jm >= 0.0f ? 1.0f : 0.0f) * p_jm;
-                float d11 = f3 * (ff_jp >= 0.0f ? 1.0f : 0.0f) * p_jp;
-                out = (d00 + d10 + d01 + d11 - factor * div_ij) / coef;
-            }
+// shaders/jacobi_iteration.wgsl:39-91 (levelset_solid fractions = face planes), JC_K iterations per launch: a CTA
+// holds its 32 x 32 cells with a halo of JC_K cells in shared memory (an iteration reads radius 1, so after JC_K of
+// them the owned cells are exact), each thread the coefficients of its cells in registers.  The reference's 100
+// iterations as a launch each were bound by their launches on small grids (2.6 us of kernel and about 1 us of gap at
+// 200 x 136: 360 us) and by passes over memory on large ones; ten per launch take 16.5 us, most of it the cells' chains
+// of sums and a division, and read the grid once.
+constexpr int JC_T = 32, JC_K = 10, JC_E = JC_T + 2 * JC_K, JC_P = JC_E + 2, JC_THREADS = 1024;
+__global__ void __launch_bounds__(JC_THREADS) k_jacobi(PF p_in, PF p_out, PF ls0, PF fu, PF fv, PF div, Uniform U, Dom d) {
+    constexpr int N = JC_E * JC_E, PER = (N + JC_THREADS - 1) / JC_THREADS;
+    __shared__ float sp[2][JC_P * JC_P];  // with a ring of zeros
+    const int x0 = blockIdx.x * JC_T - JC_K, y0 = blockIdx.y * JC_T - JC_K;
+    // Every load of the tile in flight at once: the level set with a ring (into the second image first), then the
+    // cells' pressure, fractions and divergence; 0 outside the domain.
+    float ring[(JC_P * JC_P + JC_THREADS - 1) / JC_THREADS];
+#pragma unroll
+    for (int k = 0; k < (JC_P * JC_P + JC_THREADS - 1) / JC_THREADS; ++k) {
+        const int i = threadIdx.x + k * JC_THREADS;
+        ring[k] = i < JC_P * JC_P ? ls0.ld(x0 - 1 + i % JC_P, y0 - 1 + i / JC_P) : 0.0f;
+    }
+    float w[PER][4], coef[PER], rhs[PER], pv[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * JC_THREADS, ly = i / JC_E, lx = i - ly * JC_E, x = x0 + lx, y = y0 + ly;
+        const bool in = i < N && x >= 0 && y >= 0 && x < d.cx() && y < d.cy();
+        pv[k] = in ? p_in.at(x, y) : 0.0f;
+        rhs[k] = in ? div.at(x, y) : 0.0f;
+        w[k][0] = in ? fu.at(x, y) : 0.0f;
+        w[k][1] = in ? fu.at(x + 1, y) : 0.0f;
+        w[k][2] = in ? fv.at(x, y) : 0.0f;
+        w[k][3] = in ? fv.at(x, y + 1) : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < (JC_P * JC_P + JC_THREADS - 1) / JC_THREADS; ++k) {
+        const int i = threadIdx.x + k * JC_THREADS;
+        if (i < JC_P * JC_P) {
+            sp[0][i] = 0.0f;
+            sp[1][i] = ring[k];
         }
     }
-    p_out.st(x, y, out);
+    __syncthreads();
+    unsigned upd = 0, keep = 0;  // update cells; fully solid cells, which keep their value (every other one is 0)
+    const float factor = U.dx * U.rho / U.dt;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * JC_THREADS, ly = i / JC_E, lx = i - ly * JC_E, x = x0 + lx, y = y0 + ly;
+        const bool in = i < N && x >= 0 && y >= 0 && x < d.cx() && y < d.cy();
+        const int at = in ? (ly + 1) * JC_P + lx + 1 : JC_P + 1;
+        const float* l = sp[1] + at;
+        const float lij = *l;
+        const bool wet = in && !(lij >= 0.0f), open = !(w[k][0] == 0.0f && w[k][1] == 0.0f && w[k][2] == 0.0f && w[k][3] == 0.0f);
+        const float nb[4] = {l[-1], l[1], l[-JC_P], l[JC_P]};
+        float c = 0.0f, ww[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // fminf(0, nb / lij) is 0 unless nb > 0
+            const float ff = wet && nb[q] > 0.0f ? fminf(0.0f, nb[q] / lij) : 0.0f;
+            const float t = w[k][q] * (1.0f - ff);
+            c = q ? c + t : t;
+            ww[q] = w[k][q] * (ff >= 0.0f ? 1.0f : 0.0f);
+        }
+        if (wet && !open) keep |= 1u << k;
+        const bool u = wet && open && !(fabsf(c) < 1.0e-6f);
+        if (u) upd |= 1u << k;
+        coef[k] = u ? c : 1.0f;
+        rhs[k] = factor * rhs[k];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[k][q] = u ? ww[q] : 0.0f;
+        if (in) sp[0][at] = pv[k];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 4 * JC_P; i += JC_THREADS) {  // the second image's ring
+        const int e = i / JC_P, q = i % JC_P;
+        sp[1][e == 0 ? q : e == 1 ? (JC_P - 1) * JC_P + q : e == 2 ? q * JC_P : q * JC_P + JC_P - 1] = 0.0f;
+    }
+    __syncthreads();
+    int at[PER], need[PER];  // a cell's place, and the iterations after which the owned cells still depend on it
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * JC_THREADS, ly = i / JC_E, lx = i - ly * JC_E;
+        at[k] = (ly + 1) * JC_P + lx + 1;
+        need[k] = i < N ? min(min(lx, JC_E - 1 - lx), min(ly, JC_E - 1 - ly)) : -1;
+    }
+#pragma unroll 1
+    for (int it = 0; it < JC_K; ++it) {
+        const float* a = sp[it & 1];
+        float* b = sp[(it & 1) ^ 1];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            if (need[k] <= it) continue;  // a value of the rim: too far out to reach an owned cell
+            const float* c = a + at[k];
+            float n = w[k][0] * c[-1] + w[k][1] * c[1] + w[k][2] * c[-JC_P] + w[k][3] * c[JC_P] - rhs[k];
+            if (!((upd >> k) & 1u)) n = 1.0f;
+            const float v = div_any(n, coef[k]);
+            b[at[k]] = (upd >> k) & 1u ? v : (keep >> k) & 1u ? c[0] : 0.0f;
+        }
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < JC_T * JC_T; i += JC_THREADS) {
+        const int lx = JC_K + i % JC_T, ly = JC_K + i / JC_T, x = x0 + lx, y = y0 + ly;
+        if (x < d.cx() && y < d.cy()) p_out.at(x, y) = sp[JC_K & 1][(ly + 1) * JC_P + lx + 1];
+    }
 }
 
 // solve_velocity_u.wgsl:15-47 / solve_velocity_v.wgsl:15-45

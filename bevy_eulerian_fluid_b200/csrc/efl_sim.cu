@@ -1092,10 +1092,11 @@ efl_status st_projection(efl_sim* s, efl_step_stats* st) {
     int conv = 1;
     double r0 = -1.0, r1 = -1.0;
     if (P.method == EFL_PROJECTION_JACOBI) {
-        dim3 g = grid2d(d.nx, d.ny, kBlock);
-        for (int it = 0; it < 50; ++it) {  // projection.rs:135-143
-            k_jacobi<<<g, kBlock, count_launch(), s->stream>>>(s->p0, s->p1, s->ls0, s->fu, s->fv, s->div, s->U, d);
-            k_jacobi<<<g, kBlock, count_launch(), s->stream>>>(s->p1, s->p0, s->ls0, s->fu, s->fv, s->div, s->U, d);
+        static_assert(100 % (2 * JC_K) == 0, "the last launch lands in p0");
+        for (int it = 0; it < 100; it += 2 * JC_K) {  // projection.rs:135-143: 50 pairs of iterations
+            const dim3 g((d.nx + JC_T - 1) / JC_T, (d.ny + JC_T - 1) / JC_T);
+            k_jacobi<<<g, JC_THREADS, count_launch(), s->stream>>>(s->p0, s->p1, s->ls0, s->fu, s->fv, s->div, s->U, d);
+            k_jacobi<<<g, JC_THREADS, count_launch(), s->stream>>>(s->p1, s->p0, s->ls0, s->fu, s->fv, s->div, s->U, d);
         }
         LAUNCH_CHECK();
         iters = 50;

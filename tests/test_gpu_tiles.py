@@ -68,3 +68,15 @@ def test_v_cycle_levels_bit_exact(oracle_api, gpu_api, nx, ny, method, tolerance
         so, sg = o.step(scenes.DT), g.step(scenes.DT)
         assert so.pressure_iterations == sg.pressure_iterations
     assert not compare_fields(g, o)
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 16), (32, 64), (40, 24), (200, 136), (96, 320)])
+def test_jacobi_tiles_bit_exact(oracle_api, gpu_api, nx, ny):
+    """Ten Jacobi iterations per launch on 32 x 32 tiles with a 10-cell halo."""
+    sc = _splash(nx, ny)
+    sc.cfg.projection.method = capi.PROJECTION_JACOBI
+    o, g = make_pair(sc, oracle_api, gpu_api)
+    for _ in range(5):
+        o.step(scenes.DT)
+        g.step(scenes.DT)
+    assert not compare_fields(g, o)
