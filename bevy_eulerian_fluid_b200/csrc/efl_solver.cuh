@@ -5,16 +5,14 @@
 //  * solve_gs_fixed: n red-black iterations as one launch per colour
 //    (k_gs_color), f32 (the reference's fixed-count mode) or f64.
 //  * solve_gsmix_persistent: the tolerance-driven solve (mixed-precision
-//    iterative refinement, below) as ONE cooperative launch.  Each CTA owns a
-//    tile of the grid and keeps the tile plus a halo of 2k cells in shared
-//    memory -- FP64 iterate, right-hand side and diagonal, f32 correction,
-//    coefficients and residual, the cell modes -- so that k red-black
-//    iterations run from shared memory between two halo exchanges (temporal
-//    blocking; the result is identical to k global sweeps because a
-//    half-sweep only reads the other colour).  Halos are exchanged through
-//    L2 behind a grid barrier whose spin is bounded; the relative residual is
-//    reduced and tested on the device every check_interval iterations, so the
-//    whole solve needs no host round trip.
+//    iterative refinement, below) as ONE cooperative launch over the tiles that
+//    hold water.  Each CTA keeps its tile plus a halo of 2k cells on chip, so
+//    that k red-black iterations run between two halo exchanges (temporal
+//    blocking; the result is identical to k global sweeps because a half-sweep
+//    only reads the other colour).  Halos are exchanged through L2 behind a
+//    grid barrier whose spin is bounded; the relative residual is reduced and
+//    tested on the device every check_interval iterations, so the whole solve
+//    needs no host round trip.
 //  * solve_gsmix_global: the same solve with global-memory kernels and a host
 //    loop, for grids the persistent scheme does not cover.
 //  * solve_gs32_tiled: fixed-count f32 sweeps through shared-memory tiles
@@ -56,10 +54,9 @@ struct SolverWorkspace {
     double2* partials = nullptr;
     int max_blocks = 0;
     long long spin_limit = 0;  // grid-barrier polls before giving up (0: kBarrierSpinLimit)
-    bool use_reg = true;       // register-resident form of the persistent solve (else the shared-memory form)
+    unsigned char* wet = nullptr;  // per 32 x 8 block: holds a cell with level set < 0 (k_wet_blocks)
 };
 
-constexpr int PS_THREADS = 1024;
 
 constexpr long long kBarrierSpinLimit = 1ll << 25;  // acquire polls (~ 1 s)
 
@@ -105,7 +102,6 @@ EFL_DEV bool grid_barrier(GridBarrier* gb, unsigned nblocks, long long limit) {
 
 struct PersistentParams {
     Level64 L;  // level 0: x = FP64 iterate (global), b = widened divergence
-    int tx, ty, halo, kmax;
     int tiles_x;
     double cdiv;    // ((dx*dx)*rho)/dt (gauss_seidel.wgsl:58)
     double factor;  // dt/rho/dx/dx (residual.wgsl:34)
@@ -118,6 +114,9 @@ struct PersistentParams {
     long long spin_limit;  // grid-barrier polls before giving up
     PF dbuf2;              // the exchanges alternate between the correction planes dbuf and dbuf2
     float one;             // 1.0f, passed at run time (see x2_add1)
+    const unsigned char* wet;  // per 32 x 8 block of cells (row pitch wet_w): holds a cell with level set < 0
+    int wet_w, ntiles;
+    int retry;             // run only if the launch before this one found too many tiles (result->error == 2)
 };
 
 constexpr unsigned char MODE_SKIP = 0;     // outside the domain or on the tile's outer ring
@@ -180,6 +179,7 @@ inline efl_status solver_init(SolverWorkspace& ws, int nx, int ny, int device, s
     if (cudaMalloc(&ws.barrier, sizeof(GridBarrier)) != cudaSuccess ||
         cudaMalloc(&ws.result, sizeof(SolveResult)) != cudaSuccess ||
         cudaMalloc(&ws.partials, ws.max_blocks * sizeof(double2)) != cudaSuccess ||
+        cudaMalloc(&ws.wet, (size_t)((nx + 31) / 32) * ((ny + 7) / 8)) != cudaSuccess ||
         cudaMallocHost(&ws.h_result, sizeof(SolveResult)) != cudaSuccess) {
         *err = "solver workspace allocation failed";
         return EFL_ERR_OUT_OF_MEMORY;
@@ -190,6 +190,7 @@ inline void solver_free(SolverWorkspace& ws) {
     if (ws.barrier) cudaFree(ws.barrier);
     if (ws.result) cudaFree(ws.result);
     if (ws.partials) cudaFree(ws.partials);
+    if (ws.wet) cudaFree(ws.wet);
     if (ws.h_result) cudaFreeHost(ws.h_result);
     ws = SolverWorkspace{};
 }
@@ -220,645 +221,10 @@ inline efl_status solve_gs_fixed(SolverWorkspace&, const LevelT<T>& L, const Uni
 // in exact arithmetic these are the RBGS iterates themselves: the
 // iteration counts are those of red-black Gauss-Seidel, while the sweeps move
 // f32 data.
-// Shared-memory image of one extended tile (EX x EY cells, EX even), stored
-// per colour in checkerboard-compressed form: cell (lx, ly) of colour
-// c = (gx + gy) & 1 lives at [c][ly][lx >> 1].  A cell's left / right
-// neighbours are the other colour's entries (lx >> 1) - 1 + (lx & 1) and
-// (lx >> 1) + (lx & 1) of the same row, up / down are entry lx >> 1 of the
-// rows above and below, so a warp reads consecutive words.
-template <int EX, int EY>
-struct MixTile {
-    static constexpr int W2 = EX / 2;
-    static constexpr int N2 = W2 * EY;
-    double p[2][N2];  // FP64 iterate
-    double b[2][N2];
-    double den[2][N2];
-    float4 w[2][N2];
-    float d[2][N2];   // f32 correction
-    float rc[2][N2];  // f32 right-hand side of the correction
-    float inv[2][N2];
-    unsigned char mode[2][N2];
-};
-
-// Half-sweep h (0-based within a block of red-black iterations) of colour c
-// over the cells of rings >= 1 + h: rows and columns [1 + h, EX - 1 - h), the
-// region the remaining half-sweeps of the block still read.  Colour-c cells
-// of row ly sit at x = 2 j + odd, so a row has exactly (EX - 2 - 2 h) / 2 of
-// them and the work is a dense index range.
-template <int EX, int EY, int HH>
-EFL_DEV void mix_half_sweep_h(MixTile<EX, EY>& T, int base, int c, float w, float omw) {
-    constexpr int W2 = EX / 2, NJ = W2 - 1 - HH, ROWS = EY - 2 - 2 * HH, TOTAL = NJ * ROWS;
-    constexpr int X0 = 1 + HH, Y0 = 1 + HH;
-    const int o = 1 - c;
-    for (int i = threadIdx.x; i < TOTAL; i += PS_THREADS) {
-        const int r = i / NJ;
-        const int ly = Y0 + r;
-        const int odd = (base + ly + c) & 1;
-        const int k = ly * W2 + ((X0 - odd + 1) >> 1) + (i - r * NJ);
-        const unsigned char m = T.mode[c][k];
-        if (m & MODE_STD) {  // 1 * d is d exactly and inv is 0.25: the general update, without its loads
-            float nume = T.rc[c][k];
-            nume = nume + T.d[o][k - 1 + odd];
-            nume = nume + T.d[o][k + odd];
-            nume = nume + T.d[o][k - W2];
-            nume = nume + T.d[o][k + W2];
-            T.d[c][k] = w * (nume * 0.25f) + omw * T.d[c][k];
-        } else if (m & MODE_UPDATE) {
-            const float4 wk = T.w[c][k];
-            float nume = T.rc[c][k];
-            nume = nume + wk.x * T.d[o][k - 1 + odd];
-            nume = nume + wk.y * T.d[o][k + odd];
-            nume = nume + wk.z * T.d[o][k - W2];
-            nume = nume + wk.w * T.d[o][k + W2];
-            T.d[c][k] = w * (nume * T.inv[c][k]) + omw * T.d[c][k];
-        }
-    }
-}
-template <int EX, int EY>
-EFL_DEV void mix_half_sweep(MixTile<EX, EY>& T, int base, int c, int h, float w, float omw) {
-    switch (h) {  // h < 2 * KMAX <= 8
-        case 0: mix_half_sweep_h<EX, EY, 0>(T, base, c, w, omw); break;
-        case 1: mix_half_sweep_h<EX, EY, 1>(T, base, c, w, omw); break;
-        case 2: mix_half_sweep_h<EX, EY, 2>(T, base, c, w, omw); break;
-        case 3: mix_half_sweep_h<EX, EY, 3>(T, base, c, w, omw); break;
-        case 4: mix_half_sweep_h<EX, EY, 4>(T, base, c, w, omw); break;
-        case 5: mix_half_sweep_h<EX, EY, 5>(T, base, c, w, omw); break;
-        case 6: mix_half_sweep_h<EX, EY, 6>(T, base, c, w, omw); break;
-        default: mix_half_sweep_h<EX, EY, 7>(T, base, c, w, omw); break;
-    }
-}
-
-// FP64 residual at every cell of rings >= 1 (rc = f32(cdiv * r) for cells
-// that update, d = 0) and the norms over the owned cells.
-template <int EX, int EY>
-EFL_DEV double2 mix_check(MixTile<EX, EY>& T, int base, int H, int tx, int ty, double cdiv, double factor) {
-    constexpr int W2 = EX / 2;
-    double ar = 0.0, ab = 0.0;
-    for (int i = threadIdx.x; i < EX * EY; i += PS_THREADS) {
-        const int ly = i / EX, lx = i - ly * EX;
-        const int c = (base + lx + ly) & 1, o = 1 - c, odd = lx & 1;
-        const int k = ly * W2 + (lx >> 1);
-        const unsigned char m = T.mode[c][k];
-        float rcv = 0.0f;
-        const bool ring0 = lx == 0 || ly == 0 || lx == EX - 1 || ly == EY - 1;
-        if ((m & MODE_COUNTED) && !ring0) {
-            const float4 wk = T.w[c][k];
-            double sum = (double)wk.x * T.p[o][k - 1 + odd];
-            sum = sum + (double)wk.y * T.p[o][k + odd];
-            sum = sum + (double)wk.z * T.p[o][k - W2];
-            sum = sum + (double)wk.w * T.p[o][k + W2];
-            const double bb = T.b[c][k];
-            const double r = bb - factor * (T.den[c][k] * T.p[c][k] - sum);
-            if (m & MODE_UPDATE) rcv = (float)(cdiv * r);
-            if (lx >= H && lx < H + tx && ly >= H && ly < H + ty) {
-                ar += r * r;
-                ab += bb * bb;
-            }
-        }
-        T.rc[c][k] = rcv;
-        T.d[c][k] = 0.0f;
-    }
-    ar = warp_sum(ar);
-    ab = warp_sum(ab);
-    __shared__ double red_r[PS_THREADS / 32], red_b[PS_THREADS / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        red_r[wid] = ar;
-        red_b[wid] = ab;
-    }
-    __syncthreads();
-    double2 out = make_double2(0.0, 0.0);
-    if (threadIdx.x == 0) {
-        for (int q = 0; q < PS_THREADS / 32; ++q) {
-            out.x += red_r[q];
-            out.y += red_b[q];
-        }
-    }
-    __syncthreads();
-    return out;
-}
-
-// The halo ring of an EX x EY tile image with owned interior [H, EX - H) x [H, EY - H): 2 H rows of EX
-// cells (top, then bottom), then 2 H columns of each interior row.  Every thread loads its (at most
-// ceil(ring / threads)) cells from global memory before it stores any into the image, so a reload
-// costs one round of L2 latency.
-template <int EX, int EY, int H, class V>
-EFL_DEV void halo_reload(V (*img)[(EX / 2) * EY], const V* src, size_t pitch, int gx0, int gy0, int base, int nx,
-                         int ny) {
-    constexpr int TY = EY - 2 * H, RING = 2 * H * EX + 2 * H * TY;
-    constexpr int PER = (RING + PS_THREADS - 1) / PS_THREADS;
-    V v[PER];
-    int at[PER];
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int i = threadIdx.x + q * PS_THREADS;
-        at[q] = -1;
-        v[q] = V(0);
-        if (i < RING) {
-            int lx, ly;
-            if (i < 2 * H * EX) {
-                const int r = i / EX;
-                lx = i - r * EX;
-                ly = r < H ? r : TY + r;  // rows [0, H) then [EY - H, EY)
-            } else {
-                const int j = i - 2 * H * EX, r = j / (2 * H), c = j - r * (2 * H);
-                ly = H + r;
-                lx = c < H ? c : EX - 2 * H + c;  // columns [0, H) then [EX - H, EX)
-            }
-            const int gx = gx0 + lx, gy = gy0 + ly;
-            if ((unsigned)gx < (unsigned)nx && (unsigned)gy < (unsigned)ny) v[q] = __ldcg(&src[(size_t)gy * pitch + gx]);
-            at[q] = (((base + lx + ly) & 1) << 24) | (ly * (EX / 2) + (lx >> 1));
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < PER; ++q)
-        if (at[q] >= 0) img[at[q] >> 24][at[q] & 0xffffff] = v[q];
-}
-
-template <int EX, int EY, int KMAX>
-__global__ void __launch_bounds__(PS_THREADS, 1) k_gsmix_persistent(PersistentParams P, PF dbuf) {
-    static_assert(KMAX >= 1 && KMAX <= 4, "mix_half_sweep dispatches h < 8");
-    extern __shared__ __align__(16) unsigned char ps_raw[];
-    MixTile<EX, EY>& T = *reinterpret_cast<MixTile<EX, EY>*>(ps_raw);
-    constexpr int H = 2 * KMAX;
-    constexpr int W2 = EX / 2;
-    const int tx = EX - 2 * H, ty = EY - 2 * H;
-    const Level64& L = P.L;
-    const int tile = blockIdx.x;
-    const int gx0 = (tile % P.tiles_x) * tx - H, gy0 = (tile / P.tiles_x) * ty - H;
-    const int base = (gx0 + gy0) & 1;
-    const unsigned nblocks = gridDim.x;
-
-    for (int i = threadIdx.x; i < EX * EY; i += PS_THREADS) {
-        const int ly = i / EX, lx = i - ly * EX;
-        const int gx = gx0 + lx, gy = gy0 + ly;
-        const int c = (base + lx + ly) & 1, k = ly * W2 + (lx >> 1);
-        unsigned char m = MODE_SKIP;
-        double den = 0.0, bb = 0.0, pv = 0.0;
-        float inv = 0.0f;
-        float4 wk = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if ((unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny) {
-            const bool ring = lx == 0 || ly == 0 || lx == EX - 1 || ly == EY - 1;
-            const float phi = L.ls.at(gx, gy);
-            bb = L.b.at(gx, gy);
-            pv = __ldcg(&L.x.p[(size_t)gy * L.x.P + gx]);
-            bool update = false, counted = false;
-            if (phi < 0.0f) {
-                const float f[4] = {L.fu.at(gx, gy), L.fu.at(gx + 1, gy), L.fv.at(gx, gy), L.fv.at(gx, gy + 1)};
-                if (!(f[0] == 0.0f && f[1] == 0.0f && f[2] == 0.0f && f[3] == 0.0f)) {
-                    counted = true;
-                    const int ox[4] = {-1, 1, 0, 0}, oy[4] = {0, 0, -1, 1};
-                    float wv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int jx = gx + ox[q], jy = gy + oy[q];
-                        if ((unsigned)jx < (unsigned)L.nx && (unsigned)jy < (unsigned)L.ny) {
-                            const float level = L.ls.at(jx, jy);
-                            if (level < 0.0f) {
-                                den += (double)f[q];
-                                wv[q] = f[q];
-                            } else {
-                                den += (double)f[q] * (1.0 - (double)level / (double)phi);
-                            }
-                        }
-                    }
-                    wk = make_float4(wv[0], wv[1], wv[2], wv[3]);
-                    if (!(fabs(den) < (double)1.0e-6f)) {
-                        update = true;
-                        inv = (float)(1.0 / den);
-                    }
-                }
-            }
-            if (counted) m |= MODE_COUNTED;
-            if (!ring) m |= update ? MODE_UPDATE : MODE_ZERO;  // the outer ring never updates here
-            if (!ring && update && wk.x == 1.0f && wk.y == 1.0f && wk.z == 1.0f && wk.w == 1.0f) m |= MODE_STD;
-        }
-        T.mode[c][k] = m;
-        T.den[c][k] = den;
-        T.inv[c][k] = inv;
-        T.b[c][k] = bb;
-        T.w[c][k] = wk;
-        T.p[c][k] = pv;
-    }
-    __syncthreads();
-    const double cdiv = P.cdiv, factor = P.factor;
-    const float w = (float)P.weight, omw = 1.0f - (float)P.weight;
-    unsigned iters = 0;
-    double2 part = mix_check(T, base, H, tx, ty, cdiv, factor);
-    if (threadIdx.x == 0) P.partials[blockIdx.x] = part;
-    bool ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
-    double r = ok ? ps_total_relative(P.partials, nblocks) : 0.0;
-    const double r0 = r;
-    // pending: the partials of the current p are written but their total is not read yet.  A check
-    // whose next block has more than KMAX iterations skips its own grid barrier: the total is read
-    // at the next block's first halo exchange, and if the solve had converged, the iterations run
-    // meanwhile only changed the correction d, which is dropped -- p, the iteration count and r
-    // are those of the check.
-    bool pending = false;
-    while (ok && (pending || (!(r <= P.tol) && iters < P.max_iters))) {
-        unsigned todo = min(P.check_interval, P.max_iters - iters);
-        unsigned done = 0;
-        bool converged = false;
-        while (ok && todo > 0) {
-            const unsigned kk = min((unsigned)KMAX, todo);
-            for (unsigned it = 0; it < kk; ++it) {
-                mix_half_sweep(T, base, 1, 2 * it, w, omw);  // red: (x+y) odd
-                __syncthreads();
-                mix_half_sweep(T, base, 0, 2 * it + 1, w, omw);  // black
-                __syncthreads();
-            }
-            todo -= kk;
-            done += kk;
-            if (todo > 0) {  // exchange the correction's halo
-                for (int i = threadIdx.x; i < tx * ty; i += PS_THREADS) {
-                    const int ly = H + i / tx, lx = H + i % tx, gx = gx0 + lx, gy = gy0 + ly;
-                    if ((unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny)
-                        __stcg(&dbuf.p[(size_t)gy * dbuf.P + gx], T.d[(base + lx + ly) & 1][ly * W2 + (lx >> 1)]);
-                }
-                ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
-                if (!ok) break;
-                if (pending) {
-                    pending = false;
-                    r = ps_total_relative(P.partials, nblocks);
-                    if (r <= P.tol) {
-                        converged = true;
-                        break;
-                    }
-                }
-                halo_reload<EX, EY, H>(T.d, dbuf.p, (size_t)dbuf.P, gx0, gy0, base, L.nx, L.ny);
-                __syncthreads();
-            }
-        }
-        if (!ok || converged) break;
-        iters += done;
-        // p += d on the owned cells (0 where the reference zeroes p), then exchange p.
-        for (int i = threadIdx.x; i < tx * ty; i += PS_THREADS) {
-            const int ly = H + i / tx, lx = H + i % tx, gx = gx0 + lx, gy = gy0 + ly;
-            const int c = (base + lx + ly) & 1, k = ly * W2 + (lx >> 1);
-            if ((unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny) {
-                const double pv = (T.mode[c][k] & MODE_UPDATE) ? T.p[c][k] + (double)T.d[c][k] : 0.0;
-                T.p[c][k] = pv;
-                __stcg(&L.x.p[(size_t)gy * L.x.P + gx], pv);
-            }
-        }
-        ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
-        if (!ok) break;
-        halo_reload<EX, EY, H>(T.p, L.x.p, (size_t)L.x.P, gx0, gy0, base, L.nx, L.ny);
-        __syncthreads();
-        part = mix_check(T, base, H, tx, ty, cdiv, factor);
-        if (threadIdx.x == 0) P.partials[blockIdx.x] = part;
-        if (min(P.check_interval, P.max_iters - iters) > (unsigned)KMAX) {
-            pending = true;  // read at the next block's first halo exchange
-        } else {
-            ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
-            if (!ok) break;
-            r = ps_total_relative(P.partials, nblocks);
-        }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        P.result->iterations = iters;
-        P.result->converged = (ok && r <= P.tol) ? 1 : 0;
-        P.result->error = ok ? 0 : 1;
-        P.result->r0 = r0;
-        P.result->r1 = r;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Register-resident form of the persistent mixed solve.
-//
-// The same iterates as k_gsmix_persistent on every owned cell (the same f32
-// update in the same operation order, the same checks), with the sweep made
-// branch-free and short:
-//  * Thread (bx, by) owns the 2 x 2 block of cells (2bx + i, 2by + j) of the
-//    extended tile for the whole solve.  The tile origin is even, so the
-//    block's colours are fixed: cells 0 = (0, 0) and 3 = (1, 1) have the
-//    tile's base colour, cells 1 = (1, 0) and 2 = (0, 1) the other.  A
-//    half-sweep updates two of a thread's cells; of each cell's four
-//    neighbours, two are the thread's own cells (registers) and two belong to
-//    the blocks beside it (shared memory).
-//  * The correction d, right-hand side rc and 1/den live in registers; the
-//    face weights in shared memory in thread order (one 16-byte load per
-//    update, conflict-free); the shared image of d is stored per colour,
-//    compressed along x, so a warp's neighbour loads are consecutive words.
-//  * Every cell of rings >= 1 updates in every half-sweep (no shrinking
-//    ranges, no per-cell tests): a wrong value from the stale outer ring
-//    moves inwards one ring per half-sweep, so after the K iterations between
-//    two halo exchanges (2K half-sweeps, halo 2K) the owned cells are exact.
-//    Cells that are not update cells keep d = 0 (rc = 0, 1/den = 0); the
-//    outermost ring, which only the halo exchange writes, is skipped.
-// The FP64 iterate, right-hand side and diagonal stay in shared memory; only
-// the residual checks read them.
-template <int EX, int EY>
-struct QuadTile {
-    static constexpr int W2 = EX / 2, NB = (EX / 2) * (EY / 2);
-    static constexpr int WP = W2 % 16 == 4 ? W2 : W2 + ((4 - W2 % 16) + 16) % 16;  // row stride of d
-    double p[EY][EX];
-    double b[EY][EX];
-    double den[EY][EX];
-    float4 w[4][NB];     // face weights of cell q of block t at [q][t]
-    float d[2][EY][WP];  // [k][y][x / 2] with k = (x + y) & 1 in the image (k = 0: the tile's base colour)
-};
-
-// FP64 residual of the block's cells of rings >= 1 (rc = f32(cdiv r) on update
-// cells, d = 0) and the block's norms over its owned counted cells, summed in
-// a fixed order (returned by thread 0).
-template <int EX, int EY, int NT>
-EFL_DEV double2 quad_check(QuadTile<EX, EY>& T, int bx, int by, bool active, unsigned fl, float (&rc)[4],
-                           float (&dv)[4], double cdiv, double factor) {
-    constexpr int NB = QuadTile<EX, EY>::NB;
-    double ar = 0.0, ab = 0.0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int lx = 2 * bx + (q & 1), ly = 2 * by + (q >> 1);
-        float rcv = 0.0f;
-        if ((fl >> (8 + q)) & 1u) {  // counted and not on the outermost ring
-            const float4 wq = T.w[q][threadIdx.x < NB ? threadIdx.x : 0];
-            double sum = (double)wq.x * T.p[ly][lx - 1];
-            sum = sum + (double)wq.y * T.p[ly][lx + 1];
-            sum = sum + (double)wq.z * T.p[ly - 1][lx];
-            sum = sum + (double)wq.w * T.p[ly + 1][lx];
-            const double bb = T.b[ly][lx];
-            const double r = bb - factor * (T.den[ly][lx] * T.p[ly][lx] - sum);
-            if ((fl >> q) & 1u) rcv = (float)(cdiv * r);
-            if ((fl >> (16 + q)) & 1u) {
-                ar += r * r;
-                ab += bb * bb;
-            }
-        }
-        rc[q] = rcv;
-        dv[q] = 0.0f;
-    }
-    if (active) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) T.d[q == 0 || q == 3 ? 0 : 1][2 * by + (q >> 1)][bx] = 0.0f;
-    }
-    ar = warp_sum(ar);
-    ab = warp_sum(ab);
-    __shared__ double red_r[NT / 32], red_b[NT / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        red_r[wid] = ar;
-        red_b[wid] = ab;
-    }
-    __syncthreads();
-    double2 out = make_double2(0.0, 0.0);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < NT / 32; ++k) {
-            out.x += red_r[k];
-            out.y += red_b[k];
-        }
-    }
-    __syncthreads();
-    return out;
-}
-
-// One cell update (gauss_seidel.wgsl:45-88 on the correction, in the
-// reference's operation order: left, right, up, down).
-EFL_DEV float quad_update(float rc, float4 w, float inv, float d, float dl, float dr, float du, float dd, float wgt,
-                          float omw) {
-    float nume = rc;
-    nume = nume + w.x * dl;
-    nume = nume + w.y * dr;
-    nume = nume + w.z * du;
-    nume = nume + w.w * dd;
-    return wgt * (nume * inv) + omw * d;
-}
-
-template <int EX, int EY, int KMAX, int NT>
-__global__ void __launch_bounds__(NT, 1) k_gsmix_quad(PersistentParams P, PF dbuf) {
-    static_assert(KMAX >= 1 && EX % 2 == 0 && EY % 2 == 0, "even tile image");
-    static_assert((EX / 2) * (EY / 2) <= NT && NT % 32 == 0, "one thread per 2 x 2 block");
-    extern __shared__ __align__(16) unsigned char ps_raw[];
-    QuadTile<EX, EY>& T = *reinterpret_cast<QuadTile<EX, EY>*>(ps_raw);
-    constexpr int H = 2 * KMAX, W2 = EX / 2, NB = QuadTile<EX, EY>::NB;
-    constexpr int TXo = EX - 2 * H, TYo = EY - 2 * H;
-    static_assert(H % 2 == 0, "even halo: blocks are wholly owned or wholly halo");
-    const Level64& L = P.L;
-    const int tile = blockIdx.x;
-    const int gx0 = (tile % P.tiles_x) * TXo - H, gy0 = (tile / P.tiles_x) * TYo - H;
-    const unsigned nblocks = gridDim.x;
-    const bool active = threadIdx.x < NB;
-    const int bx = active ? (int)threadIdx.x % W2 : 0, by = active ? (int)threadIdx.x / W2 : 0;
-    const int base = (gx0 + gy0) & 1;  // colour of cells 0 and 3 (1 = red, (x + y) odd)
-    const bool owned = bx >= H / 2 && bx < (H + TXo) / 2 && by >= H / 2 && by < (H + TYo) / 2;
-    const bool ring0x = bx == 0 || bx == W2 - 1, ring0y = by == 0 || by == EY / 2 - 1;
-    float inv[4], rc[4], dv[4];
-    // bit q: update cell; bit 4 + q: live (not on the outermost ring); bit 8 + q: counted and live;
-    // bit 16 + q: owned and in the domain
-    unsigned fl = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int lx = 2 * bx + (q & 1), ly = 2 * by + (q >> 1);
-        const int gx = gx0 + lx, gy = gy0 + ly;
-        const bool edge = (ring0x && ((q & 1) == (bx == 0 ? 0 : 1))) || (ring0y && ((q >> 1) == (by == 0 ? 0 : 1)));
-        if (active && !edge) fl |= 1u << (4 + q);
-        float4 wq = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        inv[q] = 0.0f;
-        rc[q] = 0.0f;
-        dv[q] = 0.0f;
-        double den = 0.0, bb = 0.0, pv = 0.0;
-        if (active && (unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny) {
-            const float phi = L.ls.at(gx, gy);
-            bb = L.b.at(gx, gy);
-            pv = __ldcg(&L.x.p[(size_t)gy * L.x.P + gx]);
-            if (owned) fl |= 1u << (16 + q);
-            if (phi < 0.0f) {
-                const float f[4] = {L.fu.at(gx, gy), L.fu.at(gx + 1, gy), L.fv.at(gx, gy), L.fv.at(gx, gy + 1)};
-                if (!(f[0] == 0.0f && f[1] == 0.0f && f[2] == 0.0f && f[3] == 0.0f)) {
-                    if (!edge) fl |= 1u << (8 + q);
-                    const int ox[4] = {-1, 1, 0, 0}, oy[4] = {0, 0, -1, 1};
-                    float wv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int jx = gx + ox[k], jy = gy + oy[k];
-                        if ((unsigned)jx < (unsigned)L.nx && (unsigned)jy < (unsigned)L.ny) {
-                            const float level = L.ls.at(jx, jy);
-                            if (level < 0.0f) {
-                                den += (double)f[k];
-                                wv[k] = f[k];
-                            } else {
-                                den += (double)f[k] * (1.0 - (double)level / (double)phi);
-                            }
-                        }
-                    }
-                    wq = make_float4(wv[0], wv[1], wv[2], wv[3]);
-                    if (!(fabs(den) < (double)1.0e-6f) && !edge) {
-                        fl |= 1u << q;
-                        inv[q] = (float)(1.0 / den);
-                    }
-                }
-            }
-        }
-        if (active) {
-            T.p[ly][lx] = pv;
-            T.b[ly][lx] = bb;
-            T.den[ly][lx] = den;
-            T.w[q][threadIdx.x] = wq;
-        }
-    }
-    __syncthreads();
-    const double cdiv = P.cdiv, factor = P.factor;
-    const float wgt = (float)P.weight, omw = 1.0f - (float)P.weight;
-    const int t = active ? (int)threadIdx.x : 0;
-    const int r0 = 2 * by, r1 = 2 * by + 1;
-    // Shared-memory rows of the neighbours that belong to other blocks (clamped inside the image for the
-    // outermost blocks, whose loads are skipped).
-    const int bxl = bx > 0 ? bx - 1 : 0, bxr = bx < W2 - 1 ? bx + 1 : bx;
-    const int rup = r0 > 0 ? r0 - 1 : 0, rdn = r1 < EY - 1 ? r1 + 1 : r1;
-    // ring of the block (its outermost cell's distance to the image edge, + 1 for its inner cells)
-    const int bring = min(min(2 * bx + 1, EX - 2 * bx), min(2 * by + 1, EY - 2 * by)) - 1;
-    auto sweep_base = [&]() {  // cells 0 and 3 (the base colour c0 = base); neighbours of the other colour
-        float(*Do)[QuadTile<EX, EY>::WP] = T.d[1];
-        const float dl0 = (fl & 0x10u) ? Do[r0][bxl] : 0.0f, du0 = (fl & 0x10u) ? Do[rup][bx] : 0.0f;
-        const float dr3 = (fl & 0x80u) ? Do[r1][bxr] : 0.0f, dd3 = (fl & 0x80u) ? Do[rdn][bx] : 0.0f;
-        if (fl & 0x10u) {
-            dv[0] = quad_update(rc[0], T.w[0][t], inv[0], dv[0], dl0, dv[1], du0, dv[2], wgt, omw);
-            T.d[0][r0][bx] = dv[0];
-        }
-        if (fl & 0x80u) {
-            dv[3] = quad_update(rc[3], T.w[3][t], inv[3], dv[3], dv[2], dr3, dv[1], dd3, wgt, omw);
-            T.d[0][r1][bx] = dv[3];
-        }
-    };
-    auto sweep_other = [&]() {  // cells 1 and 2; neighbours of the base colour
-        float(*Do)[QuadTile<EX, EY>::WP] = T.d[0];
-        const float dr1 = (fl & 0x20u) ? Do[r0][bxr] : 0.0f, du1 = (fl & 0x20u) ? Do[rup][bx] : 0.0f;
-        const float dl2 = (fl & 0x40u) ? Do[r1][bxl] : 0.0f, dd2 = (fl & 0x40u) ? Do[rdn][bx] : 0.0f;
-        if (fl & 0x20u) {
-            dv[1] = quad_update(rc[1], T.w[1][t], inv[1], dv[1], dv[0], dr1, du1, dv[3], wgt, omw);
-            T.d[1][r0][bx] = dv[1];
-        }
-        if (fl & 0x40u) {
-            dv[2] = quad_update(rc[2], T.w[2][t], inv[2], dv[2], dl2, dv[3], dv[0], dd2, wgt, omw);
-            T.d[1][r1][bx] = dv[2];
-        }
-    };
-    auto store_d = [&]() {  // all four cells into the shared image
-        if (active) {
-            T.d[0][r0][bx] = dv[0];
-            T.d[1][r0][bx] = dv[1];
-            T.d[1][r1][bx] = dv[2];
-            T.d[0][r1][bx] = dv[3];
-        }
-    };
-
-    unsigned iters = 0, xch = 0;  // xch: correction exchanges so far
-    double2 part = quad_check<EX, EY, NT>(T, bx, by, active, fl, rc, dv, cdiv, factor);
-    if (threadIdx.x == 0) P.partials[blockIdx.x] = part;
-    bool ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
-    double r = ok ? ps_total_relative(P.partials, nblocks) : 0.0;
-    const double r0v = r;
-    bool pending = false;  // as in k_gsmix_persistent: a check's total read at the next block's first exchange
-    while (ok && (pending || (!(r <= P.tol) && iters < P.max_iters))) {
-        unsigned todo = min(P.check_interval, P.max_iters - iters);
-        unsigned done = 0;
-        bool converged = false;
-        while (ok && todo > 0) {
-            const unsigned kk = min((unsigned)KMAX, todo);
-            for (unsigned it = 0; it < kk; ++it) {
-                if (bring + 1 >= 1 + 2 * (int)it) {  // a cell of the block lies in the region still needed
-                    if (base) sweep_base();  // red ((x + y) odd) first
-                    else sweep_other();
-                }
-                __syncthreads();
-                if (bring + 1 >= 2 + 2 * (int)it) {
-                    if (base) sweep_other();
-                    else sweep_base();
-                }
-                __syncthreads();
-            }
-            todo -= kk;
-            done += kk;
-            if (todo > 0) {  // exchange the correction's halo through L2
-                // Alternate planes: a CTA that runs on to the next exchange writes the other plane, so it
-                // cannot overwrite values a slower neighbour is still reloading (two exchanges apart there
-                // is always a grid barrier).
-                const PF& db = (xch++ & 1) ? P.dbuf2 : dbuf;
-                if (owned) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if ((fl >> (16 + q)) & 1u)
-                            __stcg(&db.p[(size_t)(gy0 + 2 * by + (q >> 1)) * db.P + gx0 + 2 * bx + (q & 1)], dv[q]);
-                }
-                ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
-                if (!ok) break;
-                if (pending) {
-                    pending = false;
-                    r = ps_total_relative(P.partials, nblocks);
-                    if (r <= P.tol) {
-                        converged = true;
-                        break;
-                    }
-                }
-                if (active && !owned) {
-                    float hv[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int gx = gx0 + 2 * bx + (q & 1), gy = gy0 + 2 * by + (q >> 1);
-                        hv[q] = ((unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny)
-                                    ? __ldcg(&db.p[(size_t)gy * db.P + gx])
-                                    : 0.0f;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) dv[q] = hv[q];
-                    store_d();
-                }
-                __syncthreads();
-            }
-        }
-        if (!ok || converged) break;
-        iters += done;
-        // p += d on the owned cells (0 where the reference zeroes p), then exchange p.
-        if (owned) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if ((fl >> (16 + q)) & 1u) {
-                    const int lx = 2 * bx + (q & 1), ly = 2 * by + (q >> 1);
-                    const double pv = ((fl >> q) & 1u) ? T.p[ly][lx] + (double)dv[q] : 0.0;
-                    T.p[ly][lx] = pv;
-                    __stcg(&L.x.p[(size_t)(gy0 + ly) * L.x.P + gx0 + lx], pv);
-                }
-            }
-        }
-        ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
-        if (!ok) break;
-        if (active && !owned) {
-            double hp[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int gx = gx0 + 2 * bx + (q & 1), gy = gy0 + 2 * by + (q >> 1);
-                hp[q] = ((unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny)
-                            ? __ldcg(&L.x.p[(size_t)gy * L.x.P + gx])
-                            : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) T.p[2 * by + (q >> 1)][2 * bx + (q & 1)] = hp[q];
-        }
-        __syncthreads();
-        part = quad_check<EX, EY, NT>(T, bx, by, active, fl, rc, dv, cdiv, factor);
-        if (threadIdx.x == 0) P.partials[blockIdx.x] = part;
-        if (min(P.check_interval, P.max_iters - iters) > (unsigned)KMAX) {
-            pending = true;
-        } else {
-            ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
-            if (!ok) break;
-            r = ps_total_relative(P.partials, nblocks);
-        }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        P.result->iterations = iters;
-        P.result->converged = (ok && r <= P.tol) ? 1 : 0;
-        P.result->error = ok ? 0 : 1;
-        P.result->r0 = r0v;
-        P.result->r1 = r;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Paired-lane form of the persistent mixed solve (4 x 2 cells per thread).
 //
-// The same iterates as k_gsmix_quad (the same f32 update in the same
+// One cooperative launch = one solve (the f32 update in the same
 // operation order on every cell, the same FP64 checks), with each thread
 // owning a 4 x 2 block of the extended tile: cells c0..c3 in its upper row,
 // c4..c7 in its lower one.  A half-sweep updates four of them, in two pairs
@@ -946,8 +312,62 @@ struct OctTile {
 EFL_DEV constexpr int oct_pair(int q) { return 2 * (q >> 2) + (((q & 3) + (q >> 2)) & 1); }
 EFL_DEV constexpr int oct_lane(int q) { return (q & 3) >> 1; }
 
+// Which 32 x 8 blocks of cells hold a cell with level set < 0 (one CTA per block).
+__global__ void __launch_bounds__(256) k_wet_blocks(PF ls, unsigned char* wet) {
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+    const int any = __syncthreads_or(x < ls.w && y < ls.h && ls.at(x, y) < 0.0f);
+    if (threadIdx.x == 0 && threadIdx.y == 0) wet[blockIdx.y * gridDim.x + blockIdx.x] = any != 0;
+}
+
+// The tiles (TX x TY owned cells, multiples of 32 and 8) of a level that hold a cell with level set < 0, in tile order,
+// and after them the others: list[0 .. *n), list[*n .. ntiles).  The whole CTA calls it.
+constexpr int OCT_MAX_TILES = 1024;
+// The smallest tiles first: a CTA's sweeps cover its image, 64 x 64 cells here and 96 x 64 in the next form (0.94
+// against 1.11 us per red-black iteration on a 512^2 pool), and tiles without water need no CTA, so 32 x 32 tiles fit
+// the device up to 148 x 1024 cells of water.  The same tile by 4 x 2 blocks of cells (512 threads): 0.955 us.
+#define OCT_SMALL 64, 64, 8, 256, 4
+template <int TX, int TY, int NT>
+EFL_DEV void oct_tiles(const PersistentParams& P, unsigned short* list, int* n) {
+    static_assert(TX % 32 == 0 && TY % 8 == 0, "whole blocks");
+    __shared__ unsigned char hot[OCT_MAX_TILES];
+    const int wet_h = (P.L.ny + 7) / 8;
+    for (int t = threadIdx.x; t < P.ntiles; t += NT) {
+        const int bx = (t % P.tiles_x) * (TX / 32), by = (t / P.tiles_x) * (TY / 8);
+        unsigned any = 0;
+#pragma unroll
+        for (int j = 0; j < TY / 8; ++j)
+#pragma unroll
+            for (int i = 0; i < TX / 32; ++i)
+                any |= bx + i < P.wet_w && by + j < wet_h ? P.wet[(by + j) * P.wet_w + bx + i] : 0u;
+        hot[t] = any != 0;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int total = 0, at = 0;
+        for (int t0 = 0; t0 < P.ntiles; t0 += 32)
+            total += __popc(__ballot_sync(0xffffffffu, t0 + lane < P.ntiles && hot[t0 + lane]));
+        int cold = total;
+        for (int t0 = 0; t0 < P.ntiles; t0 += 32) {
+            const bool in = t0 + lane < P.ntiles, h = in && hot[t0 + lane];
+            const unsigned mh = __ballot_sync(0xffffffffu, h), mc = __ballot_sync(0xffffffffu, in && !h);
+            const unsigned below = (1u << lane) - 1u;
+            if (h) list[at + __popc(mh & below)] = (unsigned short)(t0 + lane);
+            else if (in) list[cold + __popc(mc & below)] = (unsigned short)(t0 + lane);
+            at += __popc(mh);
+            cold += __popc(mc);
+        }
+        if (lane == 0) *n = total;
+    }
+    __syncthreads();
+}
+
+// One simulation's solve by `nblocks` CTAs, this one being number `rank` of them and owning tile list[rank] (the
+// simulation's active tiles: a tile without a cell of level set < 0 takes no part, as its correction is 0 and no
+// weight points at its cells).  False: a grid barrier timed out.
 template <int EX, int EY, int KMAX, int NT, int ROWS>
-__global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf) {
+EFL_DEV bool oct_solve(const PersistentParams& P, const PF& dbuf, const unsigned short* list, unsigned rank,
+                       unsigned nblocks) {
     using Tile = OctTile<EX, EY, ROWS>;
     constexpr int NC = 4 * ROWS, NPAIR = 2 * ROWS;
     static_assert(KMAX >= 1 && EX % 4 == 0 && EY % ROWS == 0 && ROWS % 2 == 0, "4 x ROWS blocks");
@@ -959,9 +379,8 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
     constexpr int H = 2 * KMAX, W2 = Tile::W2, W4 = Tile::W4, NB = Tile::NB, WP = Tile::WP;
     constexpr int TXo = EX - 2 * H, TYo = EY - 2 * H;
     const Level64& L = P.L;
-    const int tile = blockIdx.x;
+    const int tile = list[rank];
     const int gx0 = (tile % P.tiles_x) * TXo - H, gy0 = (tile / P.tiles_x) * TYo - H;
-    const unsigned nblocks = gridDim.x;
     const bool active = threadIdx.x < NB;
     const int bx = active ? (int)threadIdx.x % W4 : 0, by = active ? (int)threadIdx.x / W4 : 0;
     const int base = (gx0 + gy0) & 1;  // colour of the k = 0 cells (1 = red, (x + y) odd)
@@ -974,6 +393,7 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
     // bit q: update cell; 16 + q: live (not on the outermost ring); 32 + q: counted and live; 48 + q: owned and
     // in the domain
     unsigned long long fl = 0;
+    unsigned upd_halo = 0;  // bit q: update cell, the image's outermost ring included
     f32x2 wl[NPAIR], wr[NPAIR], wu[NPAIR], wd[NPAIR], inv[NPAIR], rc[NPAIR], dv[NPAIR];
     {
         float fw[4][NC], finv[NC];
@@ -1011,6 +431,7 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
                         }
                         if (!(fabs(den) < (double)1.0e-6f)) {
                             if (live) fl |= 1ull << q;
+                            upd_halo |= 1u << q;
                             finv[q] = (float)(1.0 / den);
                         }
                     }
@@ -1151,7 +572,7 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
 
     unsigned iters = 0, xch = 0;
     double2 part = check();
-    if (threadIdx.x == 0) P.partials[blockIdx.x] = part;
+    if (threadIdx.x == 0) P.partials[rank] = part;
     bool ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
     double r = ok ? ps_total_relative(P.partials, nblocks) : 0.0;
     const double r0v = r;
@@ -1200,9 +621,8 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
 #pragma unroll
                     for (int q = 0; q < NC; ++q) {
                         const int gx = gx0 + x0 + (q & 3), gy = gy0 + y0 + (q >> 2);
-                        hv[q] = ((unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny)
-                                    ? __ldcg(&db.p[(size_t)gy * db.P + gx])
-                                    : 0.0f;
+                        // an update cell's correction; every other cell's is 0 (its tile may not take part)
+                        hv[q] = (upd_halo >> q) & 1u ? __ldcg(&db.p[(size_t)gy * db.P + gx]) : 0.0f;
                     }
 #pragma unroll
                     for (int j = 0; j < ROWS; ++j)
@@ -1238,16 +658,14 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
 #pragma unroll
             for (int q = 0; q < NC; ++q) {
                 const int gx = gx0 + x0 + (q & 3), gy = gy0 + y0 + (q >> 2);
-                hp[q] = ((unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny)
-                            ? __ldcg(&L.x.p[(size_t)gy * L.x.P + gx])
-                            : 0.0;
+                hp[q] = (upd_halo >> q) & 1u ? __ldcg(&L.x.p[(size_t)gy * L.x.P + gx]) : 0.0;
             }
 #pragma unroll
             for (int q = 0; q < NC; ++q) T.p[pix(q & 3, q >> 2)] = hp[q];
         }
         __syncthreads();
         part = check();
-        if (threadIdx.x == 0) P.partials[blockIdx.x] = part;
+        if (threadIdx.x == 0) P.partials[rank] = part;
         if (min(P.check_interval, P.max_iters - iters) > (unsigned)KMAX) {
             pending = true;
         } else {
@@ -1256,13 +674,35 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
             r = ps_total_relative(P.partials, nblocks);
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (ok && iters > 0)  // the tiles that took no part: p = 0, as on every cell that is not updated
+        for (int q = (int)(nblocks + rank); q < P.ntiles; q += (int)nblocks) {
+            const int ox = (list[q] % P.tiles_x) * TXo, oy = (list[q] / P.tiles_x) * TYo;
+            for (int i = threadIdx.x; i < TXo * TYo; i += NT) {
+                const int gx = ox + i % TXo, gy = oy + i / TXo;
+                if (gx < L.nx && gy < L.ny) L.x.p[(size_t)gy * L.x.P + gx] = 0.0;
+            }
+        }
+    if (rank == 0 && threadIdx.x == 0) {
         P.result->iterations = iters;
         P.result->converged = (ok && r <= P.tol) ? 1 : 0;
         P.result->error = ok ? 0 : 1;
         P.result->r0 = r0v;
         P.result->r1 = r;
     }
+    return ok;
+}
+
+template <int EX, int EY, int KMAX, int NT, int ROWS>
+__global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf) {
+    __shared__ unsigned short list[OCT_MAX_TILES];
+    __shared__ int n;
+    if (P.retry && P.result->error != 2) return;  // the launch before this one solved it
+    oct_tiles<EX - 4 * KMAX, EY - 4 * KMAX, NT>(P, list, &n);
+    if (n == 0 || n > (int)gridDim.x) {  // no water (b = 0: converged at once), or more tiles than CTAs
+        if (blockIdx.x == 0 && threadIdx.x == 0) *P.result = SolveResult{0, n == 0 ? 1 : 0, n ? 2 : 0, 0, 0.0, 0.0};
+        return;
+    }
+    if ((int)blockIdx.x < n) oct_solve<EX, EY, KMAX, NT, ROWS>(P, dbuf, list, blockIdx.x, (unsigned)n);
 }
 
 // The reference's fixed-count f32 sweeps (gauss_seidel.wgsl:12-88, `iters`
@@ -1757,7 +1197,7 @@ inline efl_status solve_gs32_tiled(const Level& L, const PF& alt, float dx_scale
 
 struct PersistentPlan {
     int tx = 0, ty = 0, kmax = 0, tiles_x = 0, tiles_y = 0;
-    int threads = PS_THREADS;
+    int threads = 0;
     size_t smem = 0;
     const void* kernel = nullptr;
     bool ok = false;
@@ -1784,41 +1224,9 @@ inline bool plan_resident(int threads, size_t smem) {
 }
 template <int EX, int EY, int KMAX, int NT, int ROWS>
 inline const void* oct_kernel() { return (const void*)k_gsmix_oct<EX, EY, KMAX, NT, ROWS>; }
-template <int EX, int EY, int KMAX, int NT>
-inline const void* quad_kernel() { return (const void*)k_gsmix_quad<EX, EY, KMAX, NT>; }
-
-// Plans for the mixed persistent solve (MixTile: 53 bytes per cell).
-template <int EX, int EY, int KMAX>
-inline bool try_plan_mix(const SolverWorkspace& ws, int nx, int ny, PersistentPlan* p) {
-    const int tx = EX - 4 * KMAX, ty = EY - 4 * KMAX;
-    p->kmax = KMAX;
-    p->tx = tx;
-    p->ty = ty;
-    p->tiles_x = (nx + tx - 1) / tx;
-    p->tiles_y = (ny + ty - 1) / ty;
-    p->smem = sizeof(MixTile<EX, EY>);
-    p->kernel = (const void*)k_gsmix_persistent<EX, EY, KMAX>;
-    if (p->smem + 1024 > ws.max_smem) return false;
-    if (p->tiles_x * p->tiles_y > ws.num_sms || p->tiles_x * p->tiles_y > ws.max_blocks) return false;
-    return true;
-}
-// Plans for the register-resident form (QuadTile: 44 bytes of shared memory per cell).
-template <int EX, int EY, int KMAX, int NT>
-inline bool try_plan_quad(const SolverWorkspace& ws, int nx, int ny, PersistentPlan* p) {
-    const int tx = EX - 4 * KMAX, ty = EY - 4 * KMAX;
-    p->kmax = KMAX;
-    p->tx = tx;
-    p->ty = ty;
-    p->tiles_x = (nx + tx - 1) / tx;
-    p->tiles_y = (ny + ty - 1) / ty;
-    p->smem = sizeof(QuadTile<EX, EY>);
-    p->kernel = (const void*)k_gsmix_quad<EX, EY, KMAX, NT>;
-    p->threads = NT;
-    if (p->smem + 2048 > ws.max_smem) return false;
-    if (p->tiles_x * p->tiles_y > ws.num_sms || p->tiles_x * p->tiles_y > ws.max_blocks) return false;
-    return plan_resident<quad_kernel<EX, EY, KMAX, NT>>(NT, p->smem);
-}
-// Plans for the paired-lane form (OctTile: 26 bytes of shared memory per cell).
+// Plans for the paired-lane form (OctTile: 26 bytes of shared memory per cell).  The launch holds the tiles with
+// water only, which are not known on the host: a plan whose tiles do not all fit the device at once is followed by
+// the next one, which runs if it found too many.
 template <int EX, int EY, int KMAX, int NT, int ROWS>
 inline bool try_plan_oct(const SolverWorkspace& ws, int nx, int ny, PersistentPlan* p) {
     const int tx = EX - 4 * KMAX, ty = EY - 4 * KMAX;
@@ -1830,35 +1238,22 @@ inline bool try_plan_oct(const SolverWorkspace& ws, int nx, int ny, PersistentPl
     p->smem = sizeof(OctTile<EX, EY, ROWS>);
     p->kernel = (const void*)k_gsmix_oct<EX, EY, KMAX, NT, ROWS>;
     p->threads = NT;
-    if (p->smem + 2048 > ws.max_smem) return false;
-    if (p->tiles_x * p->tiles_y > ws.num_sms || p->tiles_x * p->tiles_y > ws.max_blocks) return false;
-    return plan_resident<oct_kernel<EX, EY, KMAX, NT, ROWS>>(NT, p->smem);
+    if (p->smem + 4096 > ws.max_smem) return false;
+    if ((int64_t)p->tiles_x * p->tiles_y > OCT_MAX_TILES) return false;
+    return p->ok = plan_resident<oct_kernel<EX, EY, KMAX, NT, ROWS>>(NT, p->smem);
 }
-inline PersistentPlan plan_mix(const SolverWorkspace& ws, int nx, int ny) {
-    PersistentPlan p;
-    if (ws.use_reg && (try_plan_oct<96, 64, 8, 384, 4>(ws, nx, ny, &p) ||   // 64 x 32 owned, 8 iterations
-                       try_plan_oct<80, 48, 4, 480, 2>(ws, nx, ny, &p) ||   // 64 x 32
-                       try_plan_oct<48, 48, 4, 288, 2>(ws, nx, ny, &p) ||   // 32 x 32
-                       try_plan_oct<72, 56, 2, 512, 2>(ws, nx, ny, &p) ||   // 64 x 48
-                       try_plan_oct<40, 40, 4, 224, 2>(ws, nx, ny, &p))) {  // 24 x 24
-        p.ok = true;
-        return p;
-    }
-    if (ws.use_reg && (try_plan_quad<80, 48, 4, 960>(ws, nx, ny, &p) ||  // 64 x 32 owned
-                       try_plan_quad<48, 48, 4, 576>(ws, nx, ny, &p) ||  // 32 x 32
-                       try_plan_quad<72, 56, 2, 1024>(ws, nx, ny, &p) ||  // 64 x 48
-                       try_plan_quad<40, 40, 4, 416>(ws, nx, ny, &p))) {  // 24 x 24
-        p.ok = true;
-        return p;
-    }
-    if (try_plan_mix<80, 48, 4>(ws, nx, ny, &p) ||  // 64 x 32 owned
-        try_plan_mix<48, 48, 4>(ws, nx, ny, &p) ||  // 32 x 32
-        try_plan_mix<72, 56, 2>(ws, nx, ny, &p) ||  // 64 x 48
-        try_plan_mix<40, 40, 4>(ws, nx, ny, &p)) {  // 24 x 24
-        p.ok = true;
-        return p;
-    }
-    return PersistentPlan{};
+inline std::vector<PersistentPlan> plan_oct(const SolverWorkspace& ws, int nx, int ny) {
+    std::vector<PersistentPlan> v;
+    auto add = [&](auto try_plan) {  // true: every tile fits, no further plan is needed
+        PersistentPlan p;
+        if (!try_plan(ws, nx, ny, &p)) return false;
+        v.push_back(p);
+        return p.tiles_x * p.tiles_y <= ws.num_sms;
+    };
+    if (add(try_plan_oct<OCT_SMALL>) ||             // 32 x 32 owned, 8 iterations between exchanges
+        add(try_plan_oct<96, 64, 8, 384, 4>) ||     // 64 x 32, 8
+        add(try_plan_oct<80, 72, 4, 384, 4>)) {}    // 64 x 56, 4 (1.70 us per iteration)
+    return v;
 }
 
 // Tolerance-driven solve, one cooperative launch.  dbuf: an f32 plane of the
@@ -1868,26 +1263,10 @@ inline efl_status solve_gsmix_persistent(SolverWorkspace& ws, const Level64& L, 
                                          const Uniform& U,
                                          float weight, double tol, uint32_t max_iters, uint32_t check_interval,
                                          cudaStream_t stream, SolveResult* out, std::string* err) {
-    PersistentPlan plan = plan_mix(ws, L.nx, L.ny);
-    if (!plan.ok) return EFL_ERR_STATE;
-    if (cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        return EFL_ERR_STATE;
-    }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plan.kernel, plan.threads, plan.smem) != cudaSuccess ||
-        per_sm < 1 || plan.tiles_x * plan.tiles_y > per_sm * ws.num_sms) {
-        cudaGetLastError();
-        return EFL_ERR_STATE;
-    }
-    PersistentParams P;
+    const std::vector<PersistentPlan> plans = plan_oct(ws, L.nx, L.ny);
+    if (plans.empty()) return EFL_ERR_STATE;
+    PersistentParams P{};
     P.L = L;
-    P.tx = plan.tx;
-    P.ty = plan.ty;
-    P.kmax = plan.kmax;
-    P.halo = 2 * plan.kmax;
-    P.tiles_x = plan.tiles_x;
     const double dx = (double)U.dx;
     P.cdiv = dx * dx * (double)U.rho / (double)U.dt;
     P.factor = (double)U.dt / (double)U.rho / dx / dx;
@@ -1901,18 +1280,26 @@ inline efl_status solve_gsmix_persistent(SolverWorkspace& ws, const Level64& L, 
     P.spin_limit = ws.spin_limit > 0 ? ws.spin_limit : kBarrierSpinLimit;
     P.dbuf2 = dbuf2;
     P.one = 1.0f;
+    P.wet = ws.wet;
+    P.wet_w = (L.nx + 31) / 32;
+    k_wet_blocks<<<dim3(P.wet_w, (L.ny + 7) / 8), dim3(32, 8), count_launch(), stream>>>(L.ls, ws.wet);
     if (cudaMemsetAsync(ws.barrier, 0, sizeof(GridBarrier), stream) != cudaSuccess) {
         *err = "barrier reset failed";
         return EFL_ERR_CUDA;
     }
-    PF db = dbuf;
-    void* args[] = {&P, &db};
-    count_launch();
-    cudaError_t e = cudaLaunchCooperativeKernel(plan.kernel, dim3(plan.tiles_x * plan.tiles_y), dim3(plan.threads),
-                                                args, plan.smem, stream);
-    if (e != cudaSuccess) {
-        *err = std::string("cooperative launch of the mixed solver failed: ") + cudaGetErrorString(e);
-        return EFL_ERR_CUDA;
+    for (const PersistentPlan& plan : plans) {
+        P.tiles_x = plan.tiles_x;
+        P.ntiles = plan.tiles_x * plan.tiles_y;
+        P.retry = &plan != &plans[0];
+        PF db = dbuf;
+        void* args[] = {&P, &db};
+        count_launch();
+        const cudaError_t e = cudaLaunchCooperativeKernel(plan.kernel, dim3(std::min(P.ntiles, ws.num_sms)),
+                                                          dim3(plan.threads), args, plan.smem, stream);
+        if (e != cudaSuccess) {
+            *err = std::string("cooperative launch of the mixed solver failed: ") + cudaGetErrorString(e);
+            return EFL_ERR_CUDA;
+        }
     }
     if (cudaMemcpyAsync(ws.h_result, ws.result, sizeof(SolveResult), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
         cudaStreamSynchronize(stream) != cudaSuccess) {
@@ -1920,6 +1307,7 @@ inline efl_status solve_gsmix_persistent(SolverWorkspace& ws, const Level64& L, 
         return EFL_ERR_CUDA;
     }
     *out = *ws.h_result;
+    if (out->error == 2) return EFL_ERR_STATE;  // more tiles with water than the device holds
     if (out->error) {
         *err = "mixed solver: a grid barrier timed out";
         return EFL_ERR_CUDA;
