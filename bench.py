@@ -689,8 +689,10 @@ def batch_leg(api, torch, args, world, rank, local, dist):
             "ms_per_step": {"batched": t[0] / steps, "plain": t[1] / steps},
             "pressure_solve_ms_per_step": {"batched": t[2] / steps, "plain": t[3] / steps},
             "pressure_iterations": {"max": max(iters), "mean": round(sum(iters) / len(iters), 1)},
-            "kernel": f"k_batch_mix<{tiles[0]},{tiles[1]},{tiles[2]}> (one cooperative launch per step for all "
-                      "simulations; tile shape and iterations per round chosen by the autotuner)",
+            "kernel": (f"k_batch_mix<{tiles[0]},{tiles[1]},{tiles[2]}> (one cooperative launch per step for all "
+                       "simulations; tile shape and iterations per round chosen by the autotuner)" if any(tile_cost) else
+                       f"k_batch_gang (one cooperative launch per step, a gang of CTAs per simulation, "
+                       f"{tiles[0]} x {tiles[1]} tiles with water, {tiles[2]} iterations between exchanges)"),
             "autotuner_ns_per_cell_iteration": {"64x32x2": round(tile_cost[0], 4), "64x32x4": round(tile_cost[1], 4),
                                                 "32x32x2": round(tile_cost[2], 4), "64x32x8": round(tile_cost[3], 4)},
             "learned": ({"value": cells * steps / (t[4] / 1e3), "speedup_vs_plain": round(t[1] / t[4], 3),

@@ -1,0 +1,164 @@
+// efl_gang.cuh — the tolerance-driven pressure solves of many independent simulations in ONE cooperative launch of one
+// CTA per SM, each simulation solved by a gang of CTAs.
+//
+// A gang is as many CTAs as the simulation has tiles with water (64 x 32 cells, oct_solve), so a simulation keeps its
+// tiles in shared memory and registers for the whole solve, exchanges halos with its own CTAs only, and frees them
+// when it has converged, while the other gangs go on at their own pace.  CTAs without a gang are idle; whenever one
+// becomes idle, the largest simulation that fits the idle CTAs starts (a list in global memory behind a lock).  The
+// streamed form (efl_batch.cuh) runs every simulation in lockstep, each round reading every active tile from L2 behind
+// a barrier of the whole device: about 10 us per red-black iteration whatever the number of simulations left, against
+// 1.1 us here.  64 x 32 tiles and 8 iterations between exchanges because of the throughput per SM, 1837 cells per us
+// (64 x 56 and 4: 2108, but 1.7 us per iteration and coarser tiles; 32 x 32 and 8: 1093).
+//
+// Each simulation's iterates and iteration count are those of its own solve.  Every wait is bounded.
+#pragma once
+
+#include "efl_solver.cuh"
+
+namespace efl {
+
+#define GANG_TILE 96, 64, 8, 384, 4
+constexpr int GANG_THREADS = 384, GANG_TX = 64, GANG_TY = 32;
+constexpr int GANG_MAX_SIMS = 512, GANG_MAX_CTAS = 512;
+
+struct GangSim {
+    PersistentParams P;
+    PF dbuf;
+};
+struct GangState {  // zeroed before each launch
+    unsigned lock;
+    int arrived;    // CTAs that have been idle once
+    int nidle;
+    int started;    // simulations started or not schedulable
+    int smallest;   // no simulation left has fewer tiles
+    int error;      // a wait ran out
+    unsigned taken[GANG_MAX_SIMS / 32];
+    int idle[GANG_MAX_CTAS];
+    int2 mail[GANG_MAX_CTAS];  // (simulation + 1, rank) for a CTA; x = 0: none yet, -1: leave
+    int n[GANG_MAX_SIMS];      // tiles with water
+};
+
+EFL_DEV int gang_load(const int* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Starts simulations while one fits the idle CTAs; lets the idle CTAs go when none is left.  Under the lock.
+EFL_DEV void gang_schedule(GangState* G, int ns) {
+    volatile GangState* V = G;
+    int nidle = V->nidle, started = V->started, smallest = V->smallest;
+    while (started < ns && nidle >= smallest) {
+        int best = -1, bn = 0;
+        smallest = 1 << 30;
+#pragma unroll 8
+        for (int i = 0; i < ns; ++i) {
+            const int n = __ldcg(&G->n[i]);
+            const bool left = !((__ldcg(&G->taken[i >> 5]) >> (i & 31)) & 1u);
+            if (left && n < smallest) smallest = n;
+            if (left && n <= nidle && n > bn) {
+                bn = n;
+                best = i;
+            }
+        }
+        if (best < 0) break;
+        V->taken[best >> 5] = V->taken[best >> 5] | (1u << (best & 31));
+        __threadfence();
+        ++started;
+        for (int r = 0; r < bn; ++r) {
+            const int c = V->idle[--nidle];
+            V->mail[c].y = r;
+            __threadfence();
+            V->mail[c].x = best + 1;
+        }
+    }
+    if (started == ns)
+        while (nidle > 0) V->mail[V->idle[--nidle]].x = -1;
+    V->nidle = nidle;
+    V->started = started;
+    V->smallest = smallest;
+}
+
+// The calling CTA (its first thread) joins the idle ones and waits for its next gang: (simulation, rank), or x < 0.
+EFL_DEV int2 gang_next(GangState* G, int ns, bool first, long long limit) {
+    volatile GangState* V = G;
+    long long spins = 0;
+    while (atomicCAS(&G->lock, 0u, 1u) != 0u)
+        if (++spins >= limit || ((spins & 1023) == 0 && V->error)) {
+            atomicExch(&G->error, 1);
+            return make_int2(-1, 0);
+        }
+    __threadfence();
+    V->idle[V->nidle] = (int)blockIdx.x;
+    V->nidle = V->nidle + 1;
+    if (first) V->arrived = V->arrived + 1;
+    if (V->arrived == (int)gridDim.x) gang_schedule(G, ns);  // every simulation's tile count is known from here on
+    __threadfence();
+    atomicExch(&G->lock, 0u);
+    int seen = V->started, sim = 0;
+    spins = 0;
+    while ((sim = gang_load(&G->mail[blockIdx.x].x)) == 0) {
+        ++spins;
+        if ((spins & 1023) == 0 || spins >= limit) {
+            const int now = V->started;  // progress elsewhere: not stalled
+            if (now != seen && spins < limit) {
+                seen = now;
+                spins = 0;
+            } else if (V->error || spins >= limit) {
+                atomicExch(&G->error, 1);
+                return make_int2(-1, 0);
+            }
+        }
+        __nanosleep(100);
+    }
+    const int rank = V->mail[blockIdx.x].y;
+    V->mail[blockIdx.x].x = 0;
+    return make_int2(sim > 0 ? sim - 1 : -1, rank);
+}
+
+__global__ void __launch_bounds__(GANG_THREADS, 1) k_batch_gang(const GangSim* sims, int ns, GangState* G,
+                                                                long long limit) {
+    __shared__ unsigned short list[OCT_MAX_TILES];
+    __shared__ int n;
+    __shared__ int2 job;
+    __shared__ __align__(16) unsigned char raw[sizeof(GangSim)];
+    const GangSim& S = *reinterpret_cast<const GangSim*>(raw);
+    auto load = [&](int i) {
+        static_assert(sizeof(GangSim) % 4 == 0, "copied by words");
+        __syncthreads();
+        for (int k = threadIdx.x; k < (int)sizeof(GangSim) / 4; k += GANG_THREADS)
+            reinterpret_cast<unsigned*>(raw)[k] = reinterpret_cast<const unsigned*>(&sims[i])[k];
+        __syncthreads();
+        oct_tiles<GANG_TX, GANG_TY, GANG_THREADS>(S.P, list, &n);
+    };
+    for (int i = (int)blockIdx.x; i < ns; i += (int)gridDim.x) {
+        load(i);
+        if (threadIdx.x == 0) {
+            // No water: converged at once.  More tiles than CTAs: left to the caller (error 2).
+            const bool fits = n > 0 && n <= (int)gridDim.x;
+            if (!fits) {
+                *S.P.result = SolveResult{0, n == 0 ? 1 : 0, n ? 2 : 0, 0, 0.0, 0.0};
+                atomicOr(&G->taken[i >> 5], 1u << (i & 31));
+                atomicAdd(&G->started, 1);
+            }
+            __stcg(&G->n[i], n);
+            __threadfence();
+        }
+    }
+    bool first = true;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) job = gang_next(G, ns, first, limit);
+        first = false;
+        __syncthreads();
+        const int2 j = job;
+        if (j.x < 0) return;
+        load(j.x);
+        if (!oct_solve<GANG_TILE>(S.P, S.dbuf, list, (unsigned)j.y, (unsigned)n)) {
+            if (threadIdx.x == 0) atomicExch(&G->error, 1);
+            return;
+        }
+    }
+}
+
+}  // namespace efl

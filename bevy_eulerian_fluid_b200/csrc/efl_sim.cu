@@ -24,6 +24,7 @@
 #include "efl_solver.cuh"
 #include "efl_sweep_tma.cuh"
 #include "efl_batch.cuh"
+#include "efl_gang.cuh"
 #include "efl_mgpcg.cuh"
 #include "efl_unet.cuh"
 #include "efl_pls.cuh"
@@ -2140,10 +2141,19 @@ struct efl_batch {
     int* d_work_count = nullptr;
     BatchState* d_state = nullptr;
     BatchState* h_state = nullptr;  // pinned
+    // The gang solve (efl_gang.cuh): descriptors, scheduler state, per simulation a barrier and a result.
+    GangSim* d_gang = nullptr;
+    GangState* d_gang_state = nullptr;
+    GridBarrier* d_gang_barrier = nullptr;
+    SolveResult* d_gang_result = nullptr;
+    SolveResult* h_gang_result = nullptr;  // pinned
+    int* h_gang_error = nullptr;           // pinned
+    bool ganged = false;                   // the last solve ran by gangs alone
     GridBarrier* d_barrier = nullptr;
     int ntiles = 0;
     std::vector<int> tile_start;
     cudaEvent_t ev[2] = {nullptr, nullptr};  // around the last batched solve
+    cudaEvent_t ev_stream = nullptr;         // the start of its streamed part
     bool timed = false;
     GraphCache gc;  // the stages before and after the batched solve, all simulations
     // Autotuner of the batched solve's tile shape and iterations per round:
@@ -2238,7 +2248,13 @@ void batch_free(efl_batch* b) {
     cudaFree(b->d_state);
     cudaFree(b->d_barrier);
     if (b->h_state) cudaFreeHost(b->h_state);
-    for (cudaEvent_t e : b->ev)
+    cudaFree(b->d_gang);
+    cudaFree(b->d_gang_state);
+    cudaFree(b->d_gang_barrier);
+    cudaFree(b->d_gang_result);
+    if (b->h_gang_result) cudaFreeHost(b->h_gang_result);
+    if (b->h_gang_error) cudaFreeHost(b->h_gang_error);
+    for (cudaEvent_t e : {b->ev[0], b->ev[1], b->ev_stream})
         if (e) cudaEventDestroy(e);
     b->gc.clear();
     for (cudaStream_t w : b->work)
@@ -2275,11 +2291,102 @@ efl_status batch_fanout(efl_batch* b, F per_sim) {
     return st;
 }
 
-// One cooperative launch for the tolerance-driven solves of the batch's
-// simulations listed in `which` (equal check_interval, max_iterations and
-// tolerance), results into stats.
-efl_status batch_solve(efl_batch* b, const std::vector<int>& which, efl_step_stats* stats) {
-    if (which.empty()) return EFL_OK;
+// Which 32 x 8 blocks of a simulation hold water (oct_tiles).
+void launch_wet_blocks(efl_sim* s) {
+    k_wet_blocks<<<grid2d(s->nx, s->ny, kBlock), kBlock, count_launch(), s->stream>>>(s->ls0, s->solver.wet);
+}
+
+// The tolerance-driven solves of the simulations in `which` by gangs of CTAs (their k_wet_blocks has run); `rest`
+// gets those whose tiles with water do not fit the device.
+efl_status gang_solve(efl_batch* b, const std::vector<int>& which, efl_step_stats* stats, std::vector<int>* rest) {
+    const void* kern = (const void*)k_batch_gang;
+    const size_t smem = sizeof(OctTile<96, 64, 4>);
+    const int sms = b->sims[which[0]]->solver.num_sms;
+    int per_sm = 0;
+    if (sms > GANG_MAX_CTAS ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GANG_THREADS, smem) != cudaSuccess || per_sm < 1) {
+        cudaGetLastError();
+        *rest = which;
+        return EFL_OK;
+    }
+    cudaStream_t st = b->stream;
+    for (size_t at = 0; at < which.size();) {
+        std::vector<GangSim> hs;
+        std::vector<int> ids;
+        for (; at < which.size() && ids.size() < GANG_MAX_SIMS; ++at) {
+            efl_sim* s = b->sims[which[at]];
+            GangSim S{};
+            PersistentParams& P = S.P;
+            P.L = s->mg64[0];
+            P.tiles_x = (s->nx + GANG_TX - 1) / GANG_TX;
+            P.ntiles = P.tiles_x * ((s->ny + GANG_TY - 1) / GANG_TY);
+            if (P.ntiles > OCT_MAX_TILES) {
+                rest->push_back(which[at]);
+                continue;
+            }
+            const efl_projection& Q = s->cfg.projection;
+            const double dx = (double)s->U.dx;
+            P.cdiv = dx * dx * (double)s->U.rho / (double)s->U.dt;
+            P.factor = (double)s->U.dt / (double)s->U.rho / dx / dx;
+            P.weight = (double)Q.sor_weight;
+            P.tol = (double)Q.tolerance;
+            P.max_iters = Q.max_iterations;
+            P.check_interval = std::max<uint32_t>(1, Q.check_interval);
+            P.partials = s->solver.partials;
+            P.barrier = b->d_gang_barrier + hs.size();
+            P.result = b->d_gang_result + hs.size();
+            P.spin_limit = b->spin_limit > 0 ? b->spin_limit : kBarrierSpinLimit;
+            P.dbuf2 = s->xbuf;
+            P.one = 1.0f;
+            P.wet = s->solver.wet;
+            P.wet_w = (s->nx + 31) / 32;
+            S.dbuf = s->r0;
+            hs.push_back(S);
+            ids.push_back(which[at]);
+        }
+        int ns = (int)ids.size();
+        if (!ns) continue;
+        if (cudaMemcpyAsync(b->d_gang, hs.data(), ns * sizeof(GangSim), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+            cudaMemsetAsync(b->d_gang_barrier, 0, ns * sizeof(GridBarrier), st) != cudaSuccess ||
+            cudaMemsetAsync(b->d_gang_state, 0, sizeof(GangState), st) != cudaSuccess)
+            return batch_err(b, EFL_ERR_CUDA, "batch upload failed");
+        long long limit = b->spin_limit > 0 ? b->spin_limit : kBarrierSpinLimit;
+        const GangSim* dg = b->d_gang;
+        GangState* gs = b->d_gang_state;
+        void* args[] = {&dg, &ns, &gs, &limit};
+        count_launch();
+        const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(sms), dim3(GANG_THREADS), args, smem, st);
+        if (e != cudaSuccess)
+            return batch_err(b, EFL_ERR_CUDA, std::string("batched solver launch failed: ") + cudaGetErrorString(e));
+        if (cudaMemcpyAsync(b->h_gang_result, b->d_gang_result, ns * sizeof(SolveResult), cudaMemcpyDeviceToHost, st) !=
+                cudaSuccess ||
+            cudaMemcpyAsync(b->h_gang_error, &gs->error, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+            return batch_err(b, EFL_ERR_CUDA, "batch read-back failed");
+        cudaEventRecord(b->ev[1], st);  // the solve's end, whatever follows
+        if (cudaStreamSynchronize(st) != cudaSuccess)
+            return batch_err(b, EFL_ERR_CUDA, std::string("batched solver failed: ") + cudaGetErrorString(cudaGetLastError()));
+        if (*b->h_gang_error) return batch_err(b, EFL_ERR_CUDA, "batched solver: a grid barrier timed out");
+        for (int i = 0; i < ns; ++i) {
+            const SolveResult& r = b->h_gang_result[i];
+            if (r.error == 2) {
+                rest->push_back(ids[i]);
+                continue;
+            }
+            if (!stats) continue;
+            efl_step_stats& o = stats[ids[i]];
+            o.pressure_iterations = r.iterations;
+            o.converged = r.converged;
+            o.residual = r.r1;
+            o.residual_initial = r.r0;
+        }
+    }
+    return EFL_OK;
+}
+
+// The tolerance-driven solves of the batch's simulations listed in `which` by the streamed form: one cooperative
+// launch for all of them (equal check_interval, max_iterations and tolerance), results into stats.
+efl_status stream_solve(efl_batch* b, const std::vector<int>& which, efl_step_stats* stats) {
     if ((int)b->tune_cost.size() != kBatchConfigs) b->tune_cost.assign(kBatchConfigs, 0.0);
     const int ci = b->tile_fixed >= 0 ? b->tile_fixed : (b->tile_cfg >= 0 ? b->tile_cfg : b->tune_next);
     const BatchTileConfig& cfg = batch_configs(ci);
@@ -2346,12 +2453,9 @@ efl_status batch_solve(efl_batch* b, const std::vector<int>& which, efl_step_sta
                              std::to_string(BT_MAX_OWN * grid) + " per cooperative launch");
     void* args[] = {&Pm};
     count_launch();
-    if (!b->ev[0] && (cudaEventCreate(&b->ev[0]) != cudaSuccess || cudaEventCreate(&b->ev[1]) != cudaSuccess))
-        return batch_err(b, EFL_ERR_CUDA, "event creation failed");
-    cudaEventRecord(b->ev[0], st);
+    cudaEventRecord(b->ev_stream, st);
     cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(BT_THREADS), args, smem, st);
     cudaEventRecord(b->ev[1], st);
-    b->timed = true;
     if (e != cudaSuccess)
         return batch_err(b, EFL_ERR_CUDA, std::string("batched solver launch failed: ") + cudaGetErrorString(e));
     GridBarrier hb{};
@@ -2367,7 +2471,7 @@ efl_status batch_solve(efl_batch* b, const std::vector<int>& which, efl_step_sta
         work += (double)s->nx * s->ny * b->h_state[i].iterations;
     }
     float ms = 0.0f;
-    if (work > 0.0 && cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]) == cudaSuccess) {
+    if (work > 0.0 && cudaEventElapsedTime(&ms, b->ev_stream, b->ev[1]) == cudaSuccess) {
         const double cost = ms * 1e6 / work;
         if (b->tune_cost[ci] == 0.0 || cost < b->tune_cost[ci]) b->tune_cost[ci] = cost;
         if (b->tile_fixed < 0 && b->tile_cfg < 0) {
@@ -2388,6 +2492,26 @@ efl_status batch_solve(efl_batch* b, const std::vector<int>& which, efl_step_sta
         o->residual_initial = b->h_state[i].r0;
     }
     return EFL_OK;
+}
+
+// The solves of the simulations in `which`: by gangs, and streamed where a simulation's tiles with water do not fit
+// the device or the caller fixed the streamed form's tiles (efl_batch_set_tiles).
+efl_status batch_solve(efl_batch* b, const std::vector<int>& which, efl_step_stats* stats) {
+    if (which.empty()) return EFL_OK;
+    if (!b->ev_stream && (cudaEventCreate(&b->ev[0]) != cudaSuccess || cudaEventCreate(&b->ev[1]) != cudaSuccess ||
+                          cudaEventCreate(&b->ev_stream) != cudaSuccess))
+        return batch_err(b, EFL_ERR_CUDA, "event creation failed");
+    cudaEventRecord(b->ev[0], b->stream);
+    b->timed = true;
+    std::vector<int> rest;
+    if (b->tile_fixed >= 0) {
+        rest = which;
+    } else {
+        const efl_status st = gang_solve(b, which, stats, &rest);
+        if (st != EFL_OK) return st;
+    }
+    b->ganged = rest.empty();
+    return rest.empty() ? EFL_OK : stream_solve(b, rest, stats);
 }
 }  // namespace
 
@@ -2421,7 +2545,8 @@ efl_status efl_batch_create(const efl_config* cfgs, uint32_t n, efl_batch** out)
         s->stream = b->stream;
         s->owns_stream = false;
         b->sims.push_back(s);
-        if (ensure_mix_planes(s) != EFL_OK) {
+        if (ensure_mix_planes(s) != EFL_OK ||
+            (!s->xbuf.p && alloc_plane(s, s->xbuf, s->nx, s->ny, s->P, s->ny + 1) != EFL_OK)) {
             std::string m = s->err;
             batch_free(b);
             return batch_err(nullptr, EFL_ERR_OUT_OF_MEMORY, m);
@@ -2447,6 +2572,12 @@ efl_status efl_batch_create(const efl_config* cfgs, uint32_t n, efl_batch** out)
         cudaMalloc(&b->d_work_count, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&b->d_state, n * sizeof(BatchState)) != cudaSuccess ||
         cudaMalloc(&b->d_barrier, sizeof(GridBarrier)) != cudaSuccess ||
+        cudaMalloc(&b->d_gang, n * sizeof(GangSim)) != cudaSuccess ||
+        cudaMalloc(&b->d_gang_state, sizeof(GangState)) != cudaSuccess ||
+        cudaMalloc(&b->d_gang_barrier, n * sizeof(GridBarrier)) != cudaSuccess ||
+        cudaMalloc(&b->d_gang_result, n * sizeof(SolveResult)) != cudaSuccess ||
+        cudaMallocHost(&b->h_gang_result, n * sizeof(SolveResult)) != cudaSuccess ||
+        cudaMallocHost(&b->h_gang_error, sizeof(int)) != cudaSuccess ||
         cudaMallocHost(&b->h_state, n * sizeof(BatchState)) != cudaSuccess) {
         batch_free(b);
         return batch_err(nullptr, EFL_ERR_OUT_OF_MEMORY, "batch workspace allocation failed");
@@ -2481,6 +2612,11 @@ efl_status efl_batch_tiles(const efl_batch* b, int32_t* tx, int32_t* ty, int32_t
     if (tx) *tx = c ? c->tx : 0;
     if (ty) *ty = c ? c->ty : 0;
     if (k) *k = c ? c->k : 0;
+    if (!c && b->ganged) {  // the gang solve's tiles
+        if (tx) *tx = GANG_TX;
+        if (ty) *ty = GANG_TY;
+        if (k) *k = 8;
+    }
     if (ns_per_cell_iteration)
         for (int i = 0; i < kBatchConfigs; ++i)
             ns_per_cell_iteration[i] = i < (int)b->tune_cost.size() ? b->tune_cost[i] : 0.0;
@@ -2723,6 +2859,7 @@ efl_status efl_batch_step(efl_batch* b, float dt, efl_step_stats* stats) {
         efl_status st = run_segment(b->gc, b->stream, sig_pre | 1, SEG_PRE, [&]() -> efl_status {
             TRY(batch_fanout(b, [&](size_t i, efl_sim* s) -> efl_status {
                 TRY(run_stages(s, EFL_STAGE_UPDATE_SOLID, EFL_STAGE_DIVERGENCE, nullptr));
+                launch_wet_blocks(s);
                 if (on_canvas(s))  // its residual kernel widens p and b
                     return unet_features(s, b->canvas->X0 + ((size_t)b->corigin[i].y * b->cw + b->corigin[i].x) * 16,
                                          b->cw, true);
@@ -2791,6 +2928,7 @@ efl_status efl_batch_step(efl_batch* b, float dt, efl_step_stats* stats) {
                                P.check_interval == Q.check_interval;
         if (batchable) {
             const Level64& L = s->mg64[0];
+            launch_wet_blocks(s);
             if (s->unet && (s->unet_flags & EFL_UNET_WARM_START)) {
                 efl_status st = unet_before_solve(s, true);  // its residual kernel widens p and b
                 if (st != EFL_OK) return fail(s, st);

@@ -440,8 +440,9 @@ EFL_API efl_status efl_pls_run_phase(efl_sim* sim, int32_t phase, float dt);
  * (the reference steps each fluid entity with its own dispatches,
  * render_node.rs:205-217; examples/multiple.rs spawns several).  The
  * simulations share one CUDA stream.  Their tolerance-driven red-black
- * pressure solves run as ONE cooperative launch over a packed list of
- * (simulation, tile) items; each simulation's result and iteration count are
+ * pressure solves run as ONE cooperative launch, each by a gang of CTAs of
+ * its own (those with more water than the device holds at once run streamed,
+ * tile by tile); each simulation's result and iteration count are
  * those of its own efl_step.  Simulations whose projection is not the
  * tolerance-driven Gauss-Seidel solve are projected one by one. */
 typedef struct efl_batch efl_batch;
@@ -453,16 +454,17 @@ EFL_API const char* efl_batch_last_error(const efl_batch* batch);
 EFL_API efl_status efl_batch_sim(efl_batch* batch, uint32_t i, efl_sim** sim);
 /* One frame for every simulation (efl_step semantics); stats: n entries or NULL. */
 EFL_API efl_status efl_batch_step(efl_batch* batch, float dt, efl_step_stats* stats);
-/* Tile configurations of the batched solve (owned tile and red-black
- * iterations per streamed round): 0 = 64 x 32 x 2, 1 = 64 x 32 x 4,
- * 2 = 32 x 32 x 2, 3 = 64 x 32 x 8.  By default (config = -1) an autotuner
- * runs the first four batched solves with one configuration each, timing
- * device ns per
- * cell-iteration, and keeps the fastest; every configuration gives the same
- * iterates and iteration counts.  No reference counterpart. */
+/* Tile configurations of the streamed form of the batched solve (owned tile
+ * and red-black iterations per streamed round): 0 = 64 x 32 x 2,
+ * 1 = 64 x 32 x 4, 2 = 32 x 32 x 2, 3 = 64 x 32 x 8; fixing one makes every
+ * solve streamed.  By default (config = -1) the solves run by gangs, and an
+ * autotuner picks the configuration of those that do not fit: its first four
+ * streamed solves run one configuration each, timing device ns per
+ * cell-iteration, and the fastest stays; every form and configuration gives
+ * the same iterates and iteration counts.  No reference counterpart. */
 EFL_API efl_status efl_batch_set_tiles(efl_batch* batch, int32_t config);
-/* The configuration in use (0, 0, 0 while tuning) and the measured cost of
- * each (ns_per_cell_iteration: 4 entries or NULL; 0 = not tried). */
+/* The configuration in use (64, 32, 8 where the last solve ran by gangs
+ * alone; 0, 0, 0 while tuning) and the measured cost of each (ns_per_cell_iteration: 4 entries or NULL; 0 = not tried). */
 EFL_API efl_status efl_batch_tiles(const efl_batch* batch, int32_t* tx, int32_t* ty, int32_t* k,
                                    double* ns_per_cell_iteration);
 /* Grid-barrier poll limit of the batched solve (efl_set_wait_limits'

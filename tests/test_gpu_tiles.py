@@ -80,3 +80,39 @@ def test_jacobi_tiles_bit_exact(oracle_api, gpu_api, nx, ny):
         o.step(scenes.DT)
         g.step(scenes.DT)
     assert not compare_fields(g, o)
+
+
+def test_batch_gangs_of_every_kind(gpu_api):
+    """A batch with a simulation without water, one with more tiles of water than the device holds (streamed), ragged
+    ones, ones of a single tile, and more simulations than fit at once: each as its own solve, bit for bit."""
+    shapes = [(128, 128), (1024, 640), (64, 64), (200, 72), (16, 16), (256, 256), (520, 96)] + [(96, 64)] * 30
+    scs = []
+    for i, (nx, ny) in enumerate(shapes):
+        sc = scenes.batch(1, seed=100 + i, shapes=[(nx, ny)]).scenes[0]
+        if i == 0:
+            sc.oneshot = []
+        if i == 1:  # full of water
+            sc.oneshot = [scenes.aabb_source((0.0, 0.0), (0.5 * nx, 0.49 * ny))]
+        sc.cfg.projection.max_iterations = 400
+        scs.append(sc)
+    alone = [sc.make(gpu_api) for sc in scs]
+    with capi.Batch(gpu_api, [sc.cfg for sc in scs]) as batch:
+        scenes.BatchScene("kinds", scs, 0).setup(batch.sims)
+        for _ in range(4):
+            sb = batch.step(scenes.DT)
+            sa = [s.step(scenes.DT) for s in alone]
+            assert [(x.pressure_iterations, x.converged) for x in sb] == [(x.pressure_iterations, x.converged) for x in sa]
+        for i, (g, a) in enumerate(zip(batch.sims, alone)):
+            assert not compare_fields(g, a), shapes[i]
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 64), (16, 200), (200, 136), (352, 320), (1024, 256)])
+def test_solve_on_tiles_with_water(oracle_api, gpu_api, nx, ny):
+    """The tolerance-driven solve on the tiles with water only (32 x 32; 64 x 32 where those are too many)."""
+    sc = _splash(nx, ny)
+    sc.cfg.projection.tolerance = 1e-4
+    o, g = make_pair(sc, oracle_api, gpu_api)
+    for _ in range(4):
+        so, sg = o.step(scenes.DT), g.step(scenes.DT)
+        assert so.pressure_iterations == sg.pressure_iterations
+    assert not compare_fields(g, o)
