@@ -404,6 +404,49 @@ __global__ void k_divergence(PF u1, PF v1, PF us, PF vs, PF fu, PF fv, PF div, f
     div.st(x, y, -(du_f + dv_f + du_s + dv_s) / dx);
 }
 
+// Which 32 x 8 blocks of cells hold a cell with level set < 0 (one CTA per block).  The large solves skip the others
+// (dam breaks and pools are half air or more): their correction, residual and weights are 0.
+__global__ void __launch_bounds__(256) k_wet_blocks(PF ls, unsigned char* wet) {
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+    const int any = __syncthreads_or(x < ls.w && y < ls.h && ls.at(x, y) < 0.0f);
+    if (threadIdx.x == 0 && threadIdx.y == 0) wet[blockIdx.y * gridDim.x + blockIdx.x] = any != 0;
+}
+// The same for the next coarser level, from the finer one's (fw x fh blocks): a coarse cell is water only if one of its
+// children is (restriction.wgsl takes a child's level set).
+__global__ void k_wet_coarsen(const unsigned char* fine, int fw, int fh, unsigned char* wet, int w, int h) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= w || y >= h) return;
+    unsigned any = 0;
+    for (int j = 0; j < 2; ++j)
+        for (int i = 0; i < 2; ++i)
+            if (2 * x + i < fw && 2 * y + j < fh) any |= fine[(2 * y + j) * fw + 2 * x + i];
+    wet[y * w + x] = any != 0;
+}
+// The tiles of 64 x 32 cells with a wet block, list[0 .. count), and the others, list[count .. ntiles), each in any
+// order.  counts[2] = 0 before.
+__global__ void k_wet_tiles(const unsigned char* wet, int w, int h, int tiles_x, int ntiles, int* list, int* counts) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    bool any = false;
+    if (t < ntiles) {
+        const int bx = (t % tiles_x) * 2, by = (t / tiles_x) * 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) any |= bx + i < w && by + j < h && wet[(by + j) * w + bx + i];
+    }
+    const unsigned hot = __ballot_sync(0xffffffffu, any), cold = __ballot_sync(0xffffffffu, t < ntiles && !any);
+    int at[2] = {0, 0};
+    if (lane == 0) {
+        if (hot) at[0] = atomicAdd(&counts[0], __popc(hot));
+        if (cold) at[1] = atomicAdd(&counts[1], __popc(cold));
+    }
+    at[0] = __shfl_sync(0xffffffffu, at[0], 0);
+    at[1] = __shfl_sync(0xffffffffu, at[1], 0);
+    const unsigned below = (1u << lane) - 1u;
+    if (any) list[at[0] + __popc(hot & below)] = t;
+    else if (t < ntiles) list[ntiles - 1 - (at[1] + __popc(cold & below))] = t;
+}
+
 // One level of the pressure system: iterate x, right-hand side b and
 // residual r of type T (f32: the reference's fixed-count solve; f64: the
 // tolerance-driven solve), with the level's f32 air level set and face
@@ -459,10 +502,15 @@ EFL_DEV T gs_cdiv(float dx_scaled, float rho, float dt) {
     return d * d * (T)rho / (T)dt;
 }
 // gauss_seidel.wgsl:12-42: colour 1 = red ((x+y) odd), 0 = black.  One
-// thread per cell of the colour.
+// thread per cell of the colour.  wet (or null): blocks without water are skipped (their iterate is 0 already).
 template <class T>
-__global__ void k_gs_color(LevelT<T> L, float dx_scaled, float rho, float dt, float weight, int color) {
+__global__ void k_gs_color(LevelT<T> L, float dx_scaled, float rho, float dt, float weight, int color,
+                           const unsigned char* wet = nullptr) {
     int tx = gx(), y = gy();
+    if (wet) {  // a CTA's 64 x 8 cells
+        const int w = (L.nx + 31) / 32, b = blockIdx.y * w + 2 * blockIdx.x;
+        if (!wet[b] && !(2 * (int)blockIdx.x + 1 < w && wet[b + 1])) return;
+    }
     int x = 2 * tx + ((y + color) & 1);
     if (x >= L.nx || y >= L.ny) return;
     L.x.at(x, y) = gs_update(L, gs_cdiv<T>(dx_scaled, rho, dt), (T)weight, x, y);
@@ -551,10 +599,13 @@ EFL_DEV void restrict_cell(const LevelT<T>& F, const LevelT<T>& C, int x, int y)
 }
 // The residual (k_residual) and the restriction in one pass: each coarse cell computes its four children's
 // residuals (residual_at, 0 outside the level, as the residual plane reads there) and restricts them, so the
-// fine residual plane is neither written nor read back.  The same values, in the same order.
+// fine residual plane is neither written nor read back.  The same values, in the same order.  wet: C's wet blocks in a
+// solve's later V-cycles (null in the first one), when C's geometry is known and blocks without water hold zeros.
 template <class T>
-__global__ void k_residual_restrict(LevelT<T> F, LevelT<T> C, float dt, float rho, float dx_scaled) {
+__global__ void k_residual_restrict(LevelT<T> F, LevelT<T> C, float dt, float rho, float dx_scaled,
+                                    const unsigned char* wet = nullptr) {
     int x = gx(), y = gy();
+    if (wet && !wet[blockIdx.y * gridDim.x + blockIdx.x]) return;
     if (x >= C.nx || y >= C.ny) return;
     const T fac = residual_factor<T>(dt, rho, dx_scaled);
     auto rr = [&](int ax, int ay) -> T {
@@ -563,6 +614,11 @@ __global__ void k_residual_restrict(LevelT<T> F, LevelT<T> C, float dt, float rh
     };
     const int fx = 2 * x, fy = 2 * y;
     const T r00 = rr(fx, fy), r01 = rr(fx, fy + 1), r10 = rr(fx + 1, fy), r11 = rr(fx + 1, fy + 1);
+    if (wet) {
+        C.b.at(x, y) = T(0.25) * (r00 + r01 + r10 + r11);
+        C.x.at(x, y) = T(0);
+        return;
+    }
     restrict_from(F, C, x, y, r00, r01, r10, r11);
 }
 // prolongation.wgsl:5-34
@@ -577,8 +633,9 @@ EFL_DEV void prolong_cell(const LevelT<T>& F, const LevelT<T>& C, int x, int y) 
     }
 }
 template <class T>
-__global__ void k_prolongation(LevelT<T> F, LevelT<T> C) {
+__global__ void k_prolongation(LevelT<T> F, LevelT<T> C, const unsigned char* wet = nullptr) {  // wet: C's blocks
     int x = gx(), y = gy();
+    if (wet && !wet[blockIdx.y * gridDim.x + blockIdx.x]) return;
     if (x >= C.nx || y >= C.ny) return;
     prolong_cell(F, C, x, y);
 }
@@ -744,15 +801,23 @@ __global__ void k_div_norm_finalize(const double2* partials, int n, double* out)
     out[0] = a2;
     out[1] = m;
 }
-__global__ void k_norm_finalize(const double2* partials, int n, double* out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double r = 0.0, b = 0.0;
-    for (int i = 0; i < n; ++i) {
-        r += partials[i].x;
-        b += partials[i].y;
+// The partials in block order, r and b by a thread each (one CTA of NORM_THREADS; n <= 1024).  The sums are one chain of
+// dependent additions; the loads are not (one thread for all took 50 us at 1024 partials, 76 times a solve).
+__global__ void __launch_bounds__(NORM_THREADS) k_norm_finalize(const double2* partials, int n, double* out) {
+    __shared__ double sp[2][1024];
+    for (int i = threadIdx.x; i < n; i += NORM_THREADS) {
+        const double2 v = partials[i];
+        sp[0][i] = v.x;
+        sp[1][i] = v.y;
     }
-    out[0] = r;
-    out[1] = b;
+    __syncthreads();
+    if (threadIdx.x == 0 || threadIdx.x == 32) {
+        const double* p = sp[threadIdx.x >> 5];
+        double a = 0.0;
+#pragma unroll 8
+        for (int i = 0; i < n; ++i) a += p[i];
+        out[threadIdx.x >> 5] = a;
+    }
 }
 // f32 <-> f64 transfers of the tolerance-driven solve.
 __global__ void k_widen(PF p0, PF div, Plane<double> x, Plane<double> b) {

@@ -94,10 +94,23 @@ struct TermNorm {  // (r^2, b^2) over counted cells, r = b - A x (true residual)
 constexpr int RS_CHUNK = 32, RS_THREADS = 256;
 
 // part[y * nch + cx] = sum over the 32 columns of chunk cx, in x order, of term(x, y).
+// A chunk without water adds +0 (the terms are 0 there).
 template <class Term>
-__global__ void __launch_bounds__(RS_THREADS) k_chunk_sums(Term term, int nx, int ny, int nch, double2* part) {
+__global__ void __launch_bounds__(RS_THREADS) k_chunk_sums(Term term, int nx, int ny, int nch, double2* part,
+                                                           const unsigned char* wet) {
     __shared__ double2 tile[RS_CHUNK][RS_CHUNK + 1];
     const int x0 = blockIdx.x * RS_CHUNK, y0 = blockIdx.y * RS_CHUNK;
+    if (wet) {  // four 32 x 8 blocks, as many across as chunks
+        unsigned any = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (y0 + 8 * j < ny) any |= wet[(4 * blockIdx.y + j) * nch + blockIdx.x];
+        if (!any) {
+            if (threadIdx.x < RS_CHUNK && y0 + (int)threadIdx.x < ny)
+                part[(size_t)(y0 + threadIdx.x) * nch + blockIdx.x] = make_double2(0.0, 0.0);
+            return;
+        }
+    }
     for (int i = threadIdx.x; i < RS_CHUNK * RS_CHUNK; i += RS_THREADS) {
         const int ly = i / RS_CHUNK, lx = i % RS_CHUNK;
         const int gx = x0 + lx, gy = y0 + ly;
@@ -192,8 +205,10 @@ __global__ void k_cg_scalar(int op, const double2* totals, CgScalars* sc) {
 }
 // x += alpha p, r -= alpha ap on the unknowns; r32 = f32(r).  Nothing moves
 // after a breakdown.
+// wet: blocks without water hold no unknowns.
 __global__ void k_cg_axpy(Plane<double> x, Plane<double> r, PF r32, Plane<double> p, Plane<double> ap, MixPlanes M,
-                          const CgScalars* sc, int nx, int ny) {
+                          const CgScalars* sc, int nx, int ny, const unsigned char* wet) {
+    if (!wet[blockIdx.y * gridDim.x + blockIdx.x]) return;
     const int gx = blockIdx.x * blockDim.x + threadIdx.x, gy = blockIdx.y * blockDim.y + threadIdx.y;
     if (gx >= nx || gy >= ny || !(M.mode.at(gx, gy) & MODE_UPDATE) || sc->breakdown) return;
     const double alpha = sc->alpha;
@@ -203,7 +218,10 @@ __global__ void k_cg_axpy(Plane<double> x, Plane<double> r, PF r32, Plane<double
     r32.at(gx, gy) = (float)rv;
 }
 // p = z (first) or z + beta p on the unknowns, 0 elsewhere (z widened from f32).
-__global__ void k_cg_direction(Plane<double> p, PF z, MixPlanes M, const CgScalars* sc, int first, int nx, int ny) {
+// wet (null in a solve's first call): blocks without water keep p = 0.
+__global__ void k_cg_direction(Plane<double> p, PF z, MixPlanes M, const CgScalars* sc, int first, int nx, int ny,
+                               const unsigned char* wet) {
+    if (wet && !wet[blockIdx.y * gridDim.x + blockIdx.x]) return;
     const int gx = blockIdx.x * blockDim.x + threadIdx.x, gy = blockIdx.y * blockDim.y + threadIdx.y;
     if (gx >= nx || gy >= ny) return;
     double v = 0.0;

@@ -140,6 +140,9 @@ struct efl_sim {
     SweepTma tma_pre1;   // TMA maps of the preconditioner's level 1 (error flag shared with tma)
     const float* tma_pre1_x = nullptr;  // level 1's iterate plane the maps were built over
     SweepTma tma_pre;    // TMA maps of the preconditioner's level 0 (error flag shared with tma)
+    std::vector<unsigned char*> wet_lv;  // wet blocks of the levels above the cluster's (level 0: solver.wet)
+    int* wet_list[2] = {nullptr, nullptr};  // tiles of levels 0 and 1 for the TMA sweep, wet ones first
+    int* wet_count = nullptr;               // their counts, 2 per level
     DevBuf vc_image[2];           // the coarse levels' geometry in a solve's V-cycles (f32, f64 levels); owned by bufs
     GraphCache gc;                // captured step segments
     uint64_t graph_epoch = 1;     // counts the setters that change kernel arguments
@@ -566,7 +569,7 @@ template <class T>
 efl_status launch_norms(efl_sim* s, const LevelT<T>& L0) {
     k_residual_norm<T><<<s->n_partials, NORM_THREADS, count_launch(), s->stream>>>(L0, s->U.dt, s->U.rho, s->U.dx,
                                                                       s->d_partials);
-    k_norm_finalize<<<1, 32, count_launch(), s->stream>>>(s->d_partials, s->n_partials, s->d_norms);
+    k_norm_finalize<<<1, NORM_THREADS, count_launch(), s->stream>>>(s->d_partials, s->n_partials, s->d_norms);
     LAUNCH_CHECK();
     return EFL_OK;
 }
@@ -590,15 +593,66 @@ efl_status relative_residual(efl_sim* s, const LevelT<T>& L0, double* rel) {
     return EFL_OK;
 }
 
+// What the solves skip: wet blocks (32 x 8 cells) of level 0 and of the first `levels` - 1 coarse ones, and the tile
+// lists of the TMA sweep on levels 0 and 1.  The buffers are made on first use, outside any stream capture.
+const unsigned char* wet_map(const efl_sim* s, size_t level) {
+    return level == 0 ? s->solver.wet : level <= s->wet_lv.size() ? s->wet_lv[level - 1] : nullptr;
+}
+WetList wet_tiles_of(const efl_sim* s, int level, bool zero) {
+    return s->wet_list[level] ? WetList{s->wet_list[level], s->wet_count + 2 * level, zero ? 1 : 0} : WetList{};
+}
+efl_status wet_alloc(efl_sim* s, size_t levels, bool lists) {
+    auto blocks = [&](size_t l) { return (size_t)(((s->nx >> l) + 31) / 32) * (((s->ny >> l) + 7) / 8); };
+    while (s->wet_lv.size() + 1 < levels) {
+        unsigned char* q = nullptr;
+        TRY(alloc_raw(s, q, blocks(s->wet_lv.size() + 1)));
+        s->wet_lv.push_back(q);
+    }
+    if (!lists) return EFL_OK;
+    if (!s->wet_count) TRY(alloc_raw(s, s->wet_count, 4));
+    for (int l = 0; l < 2 && (size_t)l < levels; ++l) {
+        const int nx = s->nx >> l, ny = s->ny >> l, nt = ((nx + TS_TX - 1) / TS_TX) * ((ny + TS_TY - 1) / TS_TY);
+        // a list pays where a CTA has several tiles
+        if (nt > s->solver.num_sms && !s->wet_list[l]) TRY(alloc_raw(s, s->wet_list[l], nt));
+    }
+    return EFL_OK;
+}
+efl_status wet_update(efl_sim* s, size_t levels, bool lists) {
+    k_wet_blocks<<<grid2d(s->nx, s->ny, kBlock), kBlock, count_launch(), s->stream>>>(s->ls0, s->solver.wet);
+    auto w = [&](size_t l) { return ((s->nx >> l) + 31) / 32; };
+    auto h = [&](size_t l) { return ((s->ny >> l) + 7) / 8; };
+    for (size_t l = 1; l < levels; ++l)
+        k_wet_coarsen<<<grid2d(w(l), h(l), kBlock), kBlock, count_launch(), s->stream>>>(
+            wet_map(s, l - 1), w(l - 1), h(l - 1), s->wet_lv[l - 1], w(l), h(l));
+    if (lists && (s->wet_list[0] || s->wet_list[1])) {
+        CU(cudaMemsetAsync(s->wet_count, 0, 4 * sizeof(int), s->stream));
+        for (int l = 0; l < 2 && (size_t)l < levels; ++l)
+            if (s->wet_list[l]) {
+                const int tx = ((s->nx >> l) + TS_TX - 1) / TS_TX, nt = tx * (((s->ny >> l) + TS_TY - 1) / TS_TY);
+                k_wet_tiles<<<(nt + 255) / 256, 256, count_launch(), s->stream>>>(wet_map(s, l), w(l), h(l), tx, nt,
+                                                                                 s->wet_list[l], s->wet_count + 2 * l);
+            }
+    }
+    LAUNCH_CHECK();
+    return EFL_OK;
+}
+// The levels of a V-cycle that run as launches of their own, 1 more than the cluster's first (at least 1).
+template <class T>
+size_t launched_levels(const std::vector<LevelT<T>>& mg) {
+    size_t l = 0;
+    while (l < mg.size() && (int64_t)mg[l].nx * mg[l].ny > VC_MAX_CELLS) ++l;
+    return std::min(l + 1, mg.size());
+}
+
 template <class T>
 efl_status gs_iterations(efl_sim* s, const LevelT<T>& L, float weight, float res_scale, uint32_t n,
-                         bool black_first = false) {
+                         bool black_first = false, const unsigned char* wet = nullptr) {
     float dxs = res_scale * s->U.dx;  // gauss_seidel.wgsl:57
     dim3 g = grid2d((L.nx + 1) / 2, L.ny, kBlock);
     const int c0 = black_first ? 0 : 1;  // the reference sweeps red ((x+y) odd) first
     for (uint32_t k = 0; k < n; ++k) {
-        k_gs_color<T><<<g, kBlock, count_launch(), s->stream>>>(L, dxs, s->U.rho, s->U.dt, weight, c0);
-        k_gs_color<T><<<g, kBlock, count_launch(), s->stream>>>(L, dxs, s->U.rho, s->U.dt, weight, 1 - c0);
+        k_gs_color<T><<<g, kBlock, count_launch(), s->stream>>>(L, dxs, s->U.rho, s->U.dt, weight, c0, wet);
+        k_gs_color<T><<<g, kBlock, count_launch(), s->stream>>>(L, dxs, s->U.rho, s->U.dt, weight, 1 - c0, wet);
     }
     LAUNCH_CHECK();
     return EFL_OK;
@@ -669,16 +723,19 @@ efl_status v_cycle(efl_sim* s, std::vector<LevelT<T>>& mg, size_t i, bool symmet
         return EFL_OK;
     }
     float scale = (float)(1u << i);
-    if (i == mg.size() - 1) return gs_iterations(s, L, 1.0f, scale, P.mg_coarsest);
-    TRY(gs_iterations(s, L, 1.0f, scale, P.mg_pre));
+    // A solve's first V-cycle visits every cell (geometry, zeros in the air), the later ones the blocks with water.
+    const bool skip = geom == VC_GEOM_LOAD;
+    const unsigned char *wet = skip ? wet_map(s, i) : nullptr, *wetc = skip ? wet_map(s, i + 1) : nullptr;
+    if (i == mg.size() - 1) return gs_iterations(s, L, 1.0f, scale, P.mg_coarsest, false, wet);
+    TRY(gs_iterations(s, L, 1.0f, scale, P.mg_pre, false, wet));
     const LevelT<T>& C = mg[i + 1];
     k_residual_restrict<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(L, C, s->U.dt, s->U.rho,
-                                                                                          scale * s->U.dx);
+                                                                                          scale * s->U.dx, wetc);
     LAUNCH_CHECK();
     TRY(v_cycle(s, mg, i + 1, symmetric, geom));
-    k_prolongation<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(L, C);
+    k_prolongation<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(L, C, wetc);
     LAUNCH_CHECK();
-    return gs_iterations(s, L, 1.0f, scale, P.mg_post, symmetric);
+    return gs_iterations(s, L, 1.0f, scale, P.mg_post, symmetric, wet);
 }
 
 // n reference (f32) red-black iterations on the pressure field: the TMA
@@ -695,8 +752,12 @@ efl_status sweeps_f32(efl_sim* s, float weight, uint32_t n) {
         return EFL_OK;
     }
     if (st != EFL_ERR_STATE) return set_err(s, st, "%s", e.c_str());
+    // Grids of more tiles than SMs: the tiles with water only.  The list's buffers are made by the first call, which is
+    // never inside a capture (run_segment's first run is eager).
+    TRY(wet_alloc(s, 1, true));
+    TRY(wet_update(s, 1, true));
     st = solve_gs32_tma(s->tma, s->mg[0], s->p1, s->solver.num_sms, s->U.dx, s->U.rho, s->U.dt, weight, n,
-                        s->stream, &e);
+                        s->stream, &e, wet_tiles_of(s, 0, true));
     if (st == EFL_ERR_STATE) {
         if (solve_gs32_tiled(s->mg[0], s->p1, s->U.dx, s->U.rho, s->U.dt, weight, n, s->stream) != EFL_OK)
             return set_err(s, EFL_ERR_CUDA, "tiled Gauss-Seidel launch failed: %s",
@@ -821,10 +882,10 @@ efl_status run_segment(efl_sim* s, int seg, F body) {
 // A fixed-order reduction (k_chunk_sums, k_chunk_rows, k_rows_total) into
 // C.totals[slot], enqueued on the simulation's stream.
 template <class Term>
-void cg_sum_enqueue(efl_sim* s, const Term& term, int slot) {
+void cg_sum_enqueue(efl_sim* s, const Term& term, int slot) {  // (wet blocks known)
     const int nch = (s->nx + RS_CHUNK - 1) / RS_CHUNK;
     k_chunk_sums<Term><<<dim3(nch, (s->ny + RS_CHUNK - 1) / RS_CHUNK), RS_THREADS, count_launch(), s->stream>>>(
-        term, s->nx, s->ny, nch, s->cg.part);
+        term, s->nx, s->ny, nch, s->cg.part, s->solver.wet);
     k_chunk_rows<<<(s->ny + 127) / 128, 128, count_launch(), s->stream>>>(s->cg.part, nch, s->ny, s->cg.rowsum);
     k_rows_total<<<1, 1024, count_launch(), s->stream>>>(s->cg.rowsum, s->ny, s->cg.totals + slot);
 }
@@ -840,6 +901,10 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
     const efl_projection& P = s->cfg.projection;
     const int nx = s->nx, ny = s->ny;
     TRY(ensure_mix_planes(s));
+    const size_t nlv = launched_levels(s->mg);
+    TRY(wet_alloc(s, std::max<size_t>(nlv, 2), true));
+    TRY(wet_update(s, std::max<size_t>(nlv, 2), true));
+    const unsigned char* wet0 = wet_map(s, 0);
     if (!s->cg_ready) {
         const int R = ny + 1;
         TRY(alloc_plane(s, s->cg.r, nx, ny, s->P, R));
@@ -897,39 +962,43 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
     const bool tma0 = s->tma_pre.ok && P.mg_pre == 2 && P.mg_post == 2 && pre.size() > 1;
     const bool tma1 = tma0 && s->tma_pre1.ok && s->tma_pre1_x == pre[1].x.p && pre.size() > 2;
     auto precondition = [&](int geom) -> efl_status {  // z = M r, then r . z into totals[2]
+        // Tiles and blocks without water hold zeros after the solve's first V-cycle and are skipped from the second on.
+        const bool skip = geom == VC_GEOM_LOAD;
+        const WetList wl0 = wet_tiles_of(s, 0, !skip), wl1 = skip ? wet_tiles_of(s, 1, false) : WetList{};
+        const unsigned char *wet1 = skip ? wet_map(s, 1) : nullptr, *wet2 = skip && nlv > 2 ? wet_map(s, 2) : nullptr;
         CU(cudaMemset2DAsync(C.z32.p, (size_t)C.z32.P * sizeof(float), 0, (size_t)nx * sizeof(float), ny, s->stream));
         if (tma0) {
             const float dxs = s->U.dx;  // resolution scale 1 at level 0
             TRY(tma_sweep_pass(s->tma_pre, nx, ny, s->alt32, 0, s->solver.num_sms, dxs, s->U.rho, s->U.dt, 1.0f, 2,
-                               1, s->tma.d_err, s->stream));
+                               1, s->tma.d_err, s->stream, wl0));
             Level L0 = pre[0];
             L0.x = s->alt32;
             const Level& C1 = pre[1];
             k_residual_restrict<float><<<grid2d(C1.nx, C1.ny, kBlock), kBlock, count_launch(), s->stream>>>(
-                L0, C1, s->U.dt, s->U.rho, dxs);
+                L0, C1, s->U.dt, s->U.rho, dxs, wet1);
             LAUNCH_CHECK();
             if (tma1) {  // level 1 as at level 0: x (zero) -> alt32_1 red first, coarse correction, back black first
                 const float dxs1 = 2.0f * s->U.dx;  // resolution scale 2 (multi_grid.rs:268-270)
                 TRY(tma_sweep_pass(s->tma_pre1, C1.nx, C1.ny, s->alt32_1, 0, s->solver.num_sms, dxs1, s->U.rho,
-                                   s->U.dt, 1.0f, 2, 1, s->tma.d_err, s->stream));
+                                   s->U.dt, 1.0f, 2, 1, s->tma.d_err, s->stream, wl1));
                 Level L1 = C1;
                 L1.x = s->alt32_1;
                 const Level& C2 = pre[2];
                 k_residual_restrict<float><<<grid2d(C2.nx, C2.ny, kBlock), kBlock, count_launch(), s->stream>>>(
-                    L1, C2, s->U.dt, s->U.rho, dxs1);
+                    L1, C2, s->U.dt, s->U.rho, dxs1, wet2);
                 LAUNCH_CHECK();
                 TRY(v_cycle(s, pre, 2, true, geom));
-                k_prolongation<float><<<grid2d(C2.nx, C2.ny, kBlock), kBlock, count_launch(), s->stream>>>(L1, C2);
+                k_prolongation<float><<<grid2d(C2.nx, C2.ny, kBlock), kBlock, count_launch(), s->stream>>>(L1, C2, wet2);
                 LAUNCH_CHECK();
                 TRY(tma_sweep_pass(s->tma_pre1, C1.nx, C1.ny, C1.x, 1, s->solver.num_sms, dxs1, s->U.rho, s->U.dt,
-                                   1.0f, 2, 0, s->tma.d_err, s->stream));
+                                   1.0f, 2, 0, s->tma.d_err, s->stream, wl1));
             } else {
                 TRY(v_cycle(s, pre, 1, true, geom));
             }
-            k_prolongation<float><<<grid2d(C1.nx, C1.ny, kBlock), kBlock, count_launch(), s->stream>>>(L0, C1);
+            k_prolongation<float><<<grid2d(C1.nx, C1.ny, kBlock), kBlock, count_launch(), s->stream>>>(L0, C1, wet1);
             LAUNCH_CHECK();
             TRY(tma_sweep_pass(s->tma_pre, nx, ny, C.z32, 1, s->solver.num_sms, dxs, s->U.rho, s->U.dt, 1.0f, 2,
-                               0, s->tma.d_err, s->stream));
+                               0, s->tma.d_err, s->stream, wl0));
         } else {
             TRY(v_cycle(s, pre, 0, true, geom));
         }
@@ -948,7 +1017,7 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
         k_cg_residual<<<g, kBlock, count_launch(), s->stream>>>(L.x, L.b, C.r, C.r32, M, factor, nx, ny);
         TRY(precondition(VC_GEOM_STORE));
         k_cg_scalar<<<1, 1, count_launch(), s->stream>>>(CG_RZ, C.totals, C.sc);
-        k_cg_direction<<<g, kBlock, count_launch(), s->stream>>>(C.p, C.z32, M, C.sc, 1, nx, ny);
+        k_cg_direction<<<g, kBlock, count_launch(), s->stream>>>(C.p, C.z32, M, C.sc, 1, nx, ny, nullptr);
         LAUNCH_CHECK();
         // One iteration: ap = A p and p . ap; alpha = rz / p.ap (0 and a
         // breakdown flag unless p.ap > 0); x += alpha p, r -= alpha ap; the
@@ -957,11 +1026,11 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
         auto iteration = [&]() -> efl_status {
             cg_sum_enqueue(s, TermMatvecDot{C.p, C.ap, M, factor, nx, ny}, 0);
             k_cg_scalar<<<1, 1, count_launch(), s->stream>>>(CG_ALPHA, C.totals, C.sc);
-            k_cg_axpy<<<g, kBlock, count_launch(), s->stream>>>(L.x, C.r, C.r32, C.p, C.ap, M, C.sc, nx, ny);
+            k_cg_axpy<<<g, kBlock, count_launch(), s->stream>>>(L.x, C.r, C.r32, C.p, C.ap, M, C.sc, nx, ny, wet0);
             cg_sum_enqueue(s, TermNorm{L.x, L.b, M, factor, nx, ny}, 1);
             TRY(precondition(VC_GEOM_LOAD));
             k_cg_scalar<<<1, 1, count_launch(), s->stream>>>(CG_BETA, C.totals, C.sc);
-            k_cg_direction<<<g, kBlock, count_launch(), s->stream>>>(C.p, C.z32, M, C.sc, 0, nx, ny);
+            k_cg_direction<<<g, kBlock, count_launch(), s->stream>>>(C.p, C.z32, M, C.sc, 0, nx, ny, wet0);
             LAUNCH_CHECK();
             return read_back();
         };
@@ -1137,6 +1206,10 @@ efl_status st_projection(efl_sim* s, efl_step_stats* st) {
         if (!done) {  // multigrid: FP64 V-cycles with a host-side residual test
             TRY(relative_residual(s, L, &r));
             r0 = r;
+            if (!(r <= (double)P.tolerance)) {
+                TRY(wet_alloc(s, launched_levels(s->mg64), false));
+                TRY(wet_update(s, launched_levels(s->mg64), false));
+            }
             while (!(r <= (double)P.tolerance) && iters < P.max_iterations) {
                 TRY(v_cycle(s, s->mg64, 0, false, iters == 0 ? VC_GEOM_STORE : VC_GEOM_LOAD));
                 ++iters;

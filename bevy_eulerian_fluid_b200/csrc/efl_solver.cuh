@@ -312,13 +312,6 @@ struct OctTile {
 EFL_DEV constexpr int oct_pair(int q) { return 2 * (q >> 2) + (((q & 3) + (q >> 2)) & 1); }
 EFL_DEV constexpr int oct_lane(int q) { return (q & 3) >> 1; }
 
-// Which 32 x 8 blocks of cells hold a cell with level set < 0 (one CTA per block).
-__global__ void __launch_bounds__(256) k_wet_blocks(PF ls, unsigned char* wet) {
-    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
-    const int any = __syncthreads_or(x < ls.w && y < ls.h && ls.at(x, y) < 0.0f);
-    if (threadIdx.x == 0 && threadIdx.y == 0) wet[blockIdx.y * gridDim.x + blockIdx.x] = any != 0;
-}
-
 // The tiles (TX x TY owned cells, multiples of 32 and 8) of a level that hold a cell with level set < 0, in tile order,
 // and after them the others: list[0 .. *n), list[*n .. ntiles).  The whole CTA calls it.
 constexpr int OCT_MAX_TILES = 1024;

@@ -148,7 +148,7 @@ EFL_DEV void ts_sweep_half(GsTile32<TS_EX, TS_EY>& T, int c, int base, float wei
 __global__ void __launch_bounds__(TS_THREADS, 1)
     k_gs32_tma(const __grid_constant__ SweepMaps maps, int nx, int ny, PF out, int pin, float dx_scaled, float rho,
                float dt, float weight, int tiles_x, int ntiles, int iters, int* err, int first,
-               long long wait_limit) {
+               long long wait_limit, const int* list, const int* count, int zero_dry) {
     extern __shared__ __align__(128) unsigned char sm[];
     GsTile32<TS_EX, TS_EY>& T = *reinterpret_cast<GsTile32<TS_EX, TS_EY>*>(sm + TS_TILE_OFF);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + TS_BAR_OFF);
@@ -173,15 +173,18 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
     // Tile n is staged in buffer n & 1.  Tiles 0 and 1 are issued up front; tile n + 2 goes into
     // buffer n & 1 as soon as tile n's coefficients are built (the stage is not read after that),
     // so every load has about two tiles of work to complete behind.
-    int t = blockIdx.x;
+    // With a list, its first *count tiles (those with water) are swept and the others' pressure is 0.
+    const int nsweep = list ? *count : ntiles, G = (int)gridDim.x;
+    auto tile = [&](int i) { return i >= nsweep ? -1 : list ? __ldg(&list[i]) : i; };
+    int t = tile(blockIdx.x), t1 = tile(blockIdx.x + G), t2 = tile(blockIdx.x + 2 * G);
     if (threadIdx.x == 0) {
-        if (t < ntiles) issue(t, 0);
-        if (t + (int)gridDim.x < ntiles) issue(t + gridDim.x, 1);
+        if (t >= 0) issue(t, 0);
+        if (t1 >= 0) issue(t1, 1);
     }
-    for (int n = 0; t < ntiles; t += gridDim.x, ++n) {
+    for (int n = 0; t >= 0; ++n) {
         const int b = n & 1;
-        const bool next = t + (int)gridDim.x < ntiles;
-        const bool after = t + 2 * (int)gridDim.x < ntiles;
+        const bool next = t1 >= 0, after = t2 >= 0;
+        const int t3 = tile(blockIdx.x + (n + 3) * G);  // on its way while this tile is swept
         // Warp 0 waits for the copies; the barrier then orders the other warps' reads after its
         // acquire (the other 31 warps sleep in the barrier instead of spinning on the mbarrier).
         const bool got = threadIdx.x < 32 ? mbar_wait(&bars[b], (n >> 1) & 1, wait_limit) : true;
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
         __syncthreads();
         if (threadIdx.x == 0 && after) {
             fence_proxy_async();  // the generic reads of stage[b] above before the async writes
-            issue(t + 2 * gridDim.x, b);
+            issue(t2, b);
         }
         for (int it = 0; it < iters; ++it) {
 #pragma unroll
@@ -273,8 +276,26 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
                 out.at(gx, gy) = T.p[(base + lx + ly) & 1][ly * TS_W2 + (lx >> 1)];
         }
         __syncthreads();  // the tile image and stage[b] are free again
+        t = t1;
+        t1 = t2;
+        t2 = t3;
     }
+    if (zero_dry)
+        for (int i = nsweep + (int)blockIdx.x; i < ntiles; i += G) {
+            const int q = __ldg(&list[i]), ox = (q % tiles_x) * TS_TX, oy = (q / tiles_x) * TS_TY;
+            for (int k = threadIdx.x; k < TS_TX * TS_TY; k += TS_THREADS) {
+                const int gx = ox + k % TS_TX, gy = oy + k / TS_TX;
+                if (gx < nx && gy < ny) out.at(gx, gy) = 0.0f;
+            }
+        }
 }
+
+// The tiles of a level to sweep: those with water first (k_wet_tiles).  Null: all.
+struct WetList {
+    const int* list = nullptr;
+    const int* count = nullptr;
+    int zero = 0;  // 0 into the others' pressure
+};
 
 // Host side: tensor maps of the five planes, created once per simulation.
 struct SweepTma {
@@ -352,11 +373,12 @@ inline bool tma_kernel_ready() {
 // writing `out`.
 inline efl_status tma_sweep_pass(const SweepTma& st, int nx, int ny, const PF& out, int pin, int num_sms,
                                  float dx_scaled, float rho, float dt, float weight, int iters, int first, int* err,
-                                 cudaStream_t stream) {
+                                 cudaStream_t stream, const WetList& wet) {
     if (!st.ok || iters < 1 || iters > TS_K || !tma_kernel_ready()) return EFL_ERR_STATE;
     const int tiles_x = (nx + TS_TX - 1) / TS_TX, ntiles = tiles_x * ((ny + TS_TY - 1) / TS_TY);
     k_gs32_tma<<<std::min(ntiles, num_sms), TS_THREADS, TS_SMEM + count_launch(), stream>>>(
-        st.maps, nx, ny, out, pin, dx_scaled, rho, dt, weight, tiles_x, ntiles, iters, err, first, st.wait_limit);
+        st.maps, nx, ny, out, pin, dx_scaled, rho, dt, weight, tiles_x, ntiles, iters, err, first, st.wait_limit, wet.list,
+        wet.count, wet.zero);
     return cudaGetLastError() == cudaSuccess ? EFL_OK : EFL_ERR_CUDA;
 }
 
@@ -365,7 +387,7 @@ inline efl_status tma_sweep_pass(const SweepTma& st, int nx, int ny, const PF& o
 // L.x.  Returns EFL_ERR_STATE when the TMA path is unavailable.
 inline efl_status solve_gs32_tma(SweepTma& st, const Level& L, const PF& alt, int num_sms, float dx_scaled,
                                  float rho, float dt, float weight, uint32_t n, cudaStream_t stream,
-                                 std::string* err) {
+                                 std::string* err, const WetList& wet) {
     if (!st.ok || !tma_kernel_ready()) return EFL_ERR_STATE;
     const int tiles_x = (L.nx + TS_TX - 1) / TS_TX, tiles_y = (L.ny + TS_TY - 1) / TS_TY;
     const int ntiles = tiles_x * tiles_y;
@@ -378,7 +400,8 @@ inline efl_status solve_gs32_tma(SweepTma& st, const Level& L, const PF& alt, in
         PF out = pin == 0 ? alt : L.x;
         k_gs32_tma<<<grid, TS_THREADS, TS_SMEM + count_launch(), stream>>>(st.maps, L.nx, L.ny, out, pin, dx_scaled,
                                                                            rho, dt, weight, tiles_x, ntiles, k,
-                                                                           st.d_err, 1, st.wait_limit);
+                                                                           st.d_err, 1, st.wait_limit, wet.list,
+                                                                           wet.count, wet.zero);
         pin ^= 1;
         done += (uint32_t)k;
         ++launches;
