@@ -39,14 +39,22 @@ struct CgPlanes {
     double2* part = nullptr;    // chunk sums, ny x ceil(nx / 32)
     double2* rowsum = nullptr;  // one per row
     double2* totals = nullptr;  // [0] p . ap, [1] norms, [2] r . z
+    unsigned* done = nullptr;   // k_chunk_rows' block count
     CgScalars* sc = nullptr;
     CgRead* h_read = nullptr;   // pinned
 };
 
 // A v on update cells (0 elsewhere), v = 0 off the unknowns.
 EFL_DEV double cg_apply(const Plane<double>& v, const MixPlanes& M, double factor, int x, int y, int nx, int ny) {
-    const float4 wk = M.w.at(x, y);
     const double* row = v.p + (size_t)y * v.P + x;
+    if (M.mode.at(x, y) & MODE_STD) {  // w = 1 and den = 4 (1 * v is v): 24 bytes of coefficients not read
+        double sum = row[-1];
+        sum = sum + row[1];
+        sum = sum + row[-(ptrdiff_t)v.P];
+        sum = sum + row[v.P];
+        return factor * (4.0 * row[0] - sum);
+    }
+    const float4 wk = M.w.at(x, y);
     double sum = (double)wk.x * (x > 0 ? row[-1] : 0.0);
     sum = sum + (double)wk.y * (x + 1 < nx ? row[1] : 0.0);
     sum = sum + (double)wk.z * (y > 0 ? row[-(ptrdiff_t)v.P] : 0.0);
@@ -126,42 +134,60 @@ __global__ void __launch_bounds__(RS_THREADS) k_chunk_sums(Term term, int nx, in
         part[(size_t)(y0 + threadIdx.x) * nch + blockIdx.x] = acc;
     }
 }
-// rowsum[y] = sum over chunks in order of part[y][.]
-__global__ void k_chunk_rows(const double2* part, int nch, int ny, double2* rowsum) {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= ny) return;
+// rowsum[y] = sum over chunks in order of part[y][.]; the last block to finish then adds the rows: total = sum over
+// groups of 32 rows, in group order, of each group's rows summed in row order.  A block takes 32 rows, staged 64 chunks
+// at a time so that the loads are coalesced (a thread per row read them 16 bytes at a stride of a row: 18 us at 4096^2,
+// and 6 us for the rows' launch; 14 us now).  done: zero before the first call, and left zero.
+constexpr int RR_ROWS = 32, RR_CH = 64, RR_THREADS = 256;
+__global__ void __launch_bounds__(RR_THREADS) k_chunk_rows(const double2* part, int nch, int ny, double2* rowsum,
+                                                           double2* total, unsigned* done) {
+    __shared__ double2 tile[RR_ROWS][RR_CH + 1];
+    __shared__ int last;
+    const int y0 = blockIdx.x * RR_ROWS, rows = min(RR_ROWS, ny - y0);
     double2 acc = make_double2(0.0, 0.0);
-#pragma unroll 8
-    for (int c = 0; c < nch; ++c) {
-        const double2 v = part[(size_t)y * nch + c];
-        acc.x = acc.x + v.x;
-        acc.y = acc.y + v.y;
-    }
-    rowsum[y] = acc;
-}
-
-// total = sum over groups of 32 rows, in group order, of each group's rows
-// summed in row order (one block: thread g adds group g, thread 0 the groups).
-__global__ void __launch_bounds__(1024) k_rows_total(const double2* rowsum, int ny, double2* total) {
-    __shared__ double2 grp[1024];
-    const int ngroups = (ny + 31) / 32;  // ny <= 32768
-    for (int g = threadIdx.x; g < ngroups; g += blockDim.x) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int y = 32 * g; y < min(ny, 32 * g + 32); ++y) {
-            const double2 v = rowsum[y];
-            acc.x = acc.x + v.x;
-            acc.y = acc.y + v.y;
+    for (int c0 = 0; c0 < nch; c0 += RR_CH) {
+        const int n = min(RR_CH, nch - c0);
+        for (int i = threadIdx.x; i < rows * RR_CH; i += RR_THREADS) {
+            const int r = i / RR_CH, c = i % RR_CH;
+            if (c < n) tile[r][c] = part[(size_t)(y0 + r) * nch + c0 + c];
         }
-        grp[g] = acc;
+        __syncthreads();
+        if ((int)threadIdx.x < rows)
+            for (int c = 0; c < n; ++c) {
+                acc.x = acc.x + tile[threadIdx.x][c].x;
+                acc.y = acc.y + tile[threadIdx.x][c].y;
+            }
+        __syncthreads();
+    }
+    if ((int)threadIdx.x < rows) {
+        rowsum[y0 + threadIdx.x] = acc;
+        __threadfence();
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int g = 0; g < ngroups; ++g) {
-            acc.x = acc.x + grp[g].x;
-            acc.y = acc.y + grp[g].y;
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double2* const grp = &tile[0][0];  // 1024 groups fit
+    const int ngroups = (ny + 31) / 32;  // ny <= 32768
+    for (int g = threadIdx.x; g < ngroups; g += RR_THREADS) {
+        double2 a = make_double2(0.0, 0.0);
+#pragma unroll 8
+        for (int y = 32 * g; y < min(ny, 32 * g + 32); ++y) {
+            const double2 v = __ldcg(&rowsum[y]);
+            a.x = a.x + v.x;
+            a.y = a.y + v.y;
         }
-        *total = acc;
+        grp[g] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 || threadIdx.x == 32) {  // the two sums side by side
+        const int k = threadIdx.x >> 5;
+        double a = 0.0;
+#pragma unroll 8
+        for (int g = 0; g < ngroups; ++g) a = a + (k ? grp[g].y : grp[g].x);
+        (k ? total->y : total->x) = a;
+        if (k == 0) *done = 0u;
     }
 }
 

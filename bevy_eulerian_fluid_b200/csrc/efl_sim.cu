@@ -886,8 +886,8 @@ void cg_sum_enqueue(efl_sim* s, const Term& term, int slot) {  // (wet blocks kn
     const int nch = (s->nx + RS_CHUNK - 1) / RS_CHUNK;
     k_chunk_sums<Term><<<dim3(nch, (s->ny + RS_CHUNK - 1) / RS_CHUNK), RS_THREADS, count_launch(), s->stream>>>(
         term, s->nx, s->ny, nch, s->cg.part, s->solver.wet);
-    k_chunk_rows<<<(s->ny + 127) / 128, 128, count_launch(), s->stream>>>(s->cg.part, nch, s->ny, s->cg.rowsum);
-    k_rows_total<<<1, 1024, count_launch(), s->stream>>>(s->cg.rowsum, s->ny, s->cg.totals + slot);
+    k_chunk_rows<<<(s->ny + RR_ROWS - 1) / RR_ROWS, RR_THREADS, count_launch(), s->stream>>>(
+        s->cg.part, nch, s->ny, s->cg.rowsum, s->cg.totals + slot, s->cg.done);
 }
 
 // EFL_PROJECTION_MGPCG on the FP64 level 0 (x = iterate, b = widened div):
@@ -915,6 +915,7 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
         TRY(alloc_raw(s, s->cg.part, (size_t)ny * ((nx + RS_CHUNK - 1) / RS_CHUNK)));
         TRY(alloc_raw(s, s->cg.rowsum, (size_t)ny));
         TRY(alloc_raw(s, s->cg.totals, 3));
+        TRY(alloc_raw(s, s->cg.done, 1));
         TRY(alloc_raw(s, s->cg.sc, 1));
         CU(cudaMallocHost(&s->cg.h_read, sizeof(CgRead)));
         TRY(alloc_plane(s, s->alt32, nx, ny, s->P, R));
@@ -943,7 +944,7 @@ efl_status mgpcg(efl_sim* s, SolveResult* res) {
     const dim3 g = grid2d(nx, ny, kBlock);
     const double dx = (double)s->U.dx;
     const double factor = (double)s->U.dt / (double)s->U.rho / dx / dx;
-    k_mix_coefficients<<<g, kBlock, count_launch(), s->stream>>>(L, M);
+    k_mix_coefficients<true><<<g, kBlock, count_launch(), s->stream>>>(L, M);
     LAUNCH_CHECK();
     auto read_back = [&]() -> efl_status {  // C.h_read <- (norm totals, breakdown flag)
         CU(cudaMemcpyAsync(&C.h_read->norm, C.totals + 1, sizeof(double2), cudaMemcpyDeviceToHost, s->stream));

@@ -942,6 +942,8 @@ struct MixPlanes {
     Plane<double> den;
     Plane<unsigned char> mode;
 };
+// CG: the conjugate gradients imply a standard cell's coefficients and use none of a cell that is not counted.
+template <bool CG>
 __global__ void k_mix_coefficients(Level64 L, MixPlanes M) {
     const int gx = blockIdx.x * blockDim.x + threadIdx.x, gy = blockIdx.y * blockDim.y + threadIdx.y;
     if (gx >= L.nx || gy >= L.ny) return;
@@ -973,13 +975,15 @@ __global__ void k_mix_coefficients(Level64 L, MixPlanes M) {
             if (!(fabs(den) < (double)1.0e-6f)) {
                 m = (unsigned char)((m & MODE_COUNTED) | MODE_UPDATE);
                 inv = (float)(1.0 / den);
+                if (wk.x == 1.0f && wk.y == 1.0f && wk.z == 1.0f && wk.w == 1.0f) m |= MODE_STD;
             }
         }
     }
     M.mode.at(gx, gy) = m;
+    if (CG && ((m & MODE_STD) || !(m & MODE_COUNTED))) return;
     M.den.at(gx, gy) = den;
-    M.inv.at(gx, gy) = inv;
     M.w.at(gx, gy) = wk;
+    if (!CG) M.inv.at(gx, gy) = inv;
 }
 __global__ void __launch_bounds__(NORM_THREADS) k_mix_residual(Level64 L, MixPlanes M, double cdiv, double factor,
                                                                double2* partials) {
@@ -1320,7 +1324,7 @@ inline efl_status solve_gsmix_global(SolverWorkspace& ws, const Level64& L, cons
     const double cdiv = dx * dx * (double)U.rho / (double)U.dt;
     const double factor = (double)U.dt / (double)U.rho / dx / dx;
     const int nblocks = std::min(ws.max_blocks, std::max(1, (L.nx * L.ny + NORM_THREADS - 1) / NORM_THREADS));
-    k_mix_coefficients<<<g, b, count_launch(), stream>>>(L, M);
+    k_mix_coefficients<false><<<g, b, count_launch(), stream>>>(L, M);
     auto residual = [&](double* rel) -> efl_status {
         k_mix_residual<<<nblocks, NORM_THREADS, count_launch(), stream>>>(L, M, cdiv, factor, ws.partials);
         std::vector<double2> h(nblocks);
