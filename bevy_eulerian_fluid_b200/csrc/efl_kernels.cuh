@@ -278,22 +278,39 @@ __global__ void k_area_fraction(PF ls_s, PF fu, PF fv, Dom d) {
     if (y == d.ny - 1) fv.st(x, y + 1, f.w);
 }
 
+// (i, j), (i + 1, j), (i, j + 1), (i + 1, j + 1), 0 outside: one test for the interior instead of four.
+EFL_DEV void load_2x2(const PF& a, int i, int j, float (&q)[4]) {
+    if (i >= 0 && j >= 0 && i < a.w - 1 && j < a.h - 1) {
+        const float* c = a.p + (size_t)j * a.P + i;
+        q[0] = c[0];
+        q[1] = c[1];
+        q[2] = c[a.P];
+        q[3] = c[a.P + 1];
+    } else {
+        q[0] = a.ld(i, j);
+        q[1] = a.ld(i + 1, j);
+        q[2] = a.ld(i, j + 1);
+        q[3] = a.ld(i + 1, j + 1);
+    }
+}
 // utils/coordinate.wgsl:51-94
 EFL_DEV float interp_edge_x(const PF& u, float px, float py) {
     int i = f2i(rintf(px));
     int j = f2i(floorf(py));
     float fi = px + 0.5f - (float)i;
     float fj = py - (float)j;
-    float u00 = u.ld(i, j), u10 = u.ld(i + 1, j), u01 = u.ld(i, j + 1), u11 = u.ld(i + 1, j + 1);
-    return wmix(wmix(u00, u10, fi), wmix(u01, u11, fi), fj);
+    float q[4];
+    load_2x2(u, i, j, q);
+    return wmix(wmix(q[0], q[1], fi), wmix(q[2], q[3], fi), fj);
 }
 EFL_DEV float interp_edge_y(const PF& v, float px, float py) {
     int i = f2i(floorf(px));
     int j = f2i(rintf(py));
     float fi = px - (float)i;
     float fj = py + 0.5f - (float)j;
-    float v00 = v.ld(i, j), v10 = v.ld(i + 1, j), v01 = v.ld(i, j + 1), v11 = v.ld(i + 1, j + 1);
-    return wmix(wmix(v00, v10, fi), wmix(v01, v11, fi), fj);
+    float q[4];
+    load_2x2(v, i, j, q);
+    return wmix(wmix(q[0], q[1], fi), wmix(q[2], q[3], fi), fj);
 }
 EFL_DEV float2 runge_kutta(const PF& u, const PF& v, float px, float py, float dt) {
     float vx = interp_edge_x(u, px, py), vy = interp_edge_y(v, px, py);
@@ -303,30 +320,33 @@ EFL_DEV float2 runge_kutta(const PF& u, const PF& v, float px, float py, float d
     return make_float2(px - dt * wx, py - dt * wy);
 }
 // advect_velocity.wgsl:11-27 (x-major) and :29-45 (y-major)
-EFL_DEV void advect_u_at(const PF& u0, const PF& v0, const PF& u1, float dt, const Dom& d) {
-    int x = gx(), y = gy();
-    if (x > d.nx || y >= d.xrows()) return;
+EFL_DEV float advected_u(const PF& u0, const PF& v0, float dt, int x, int y) {
     float px = (float)x + -0.5f, py = (float)y + 0.0f;
     float2 b = runge_kutta(u0, v0, px, py, dt);
     float dimx = (float)u0.w, dimy = (float)u0.h;
     bool inside = b.x >= 0.0f && b.y >= 0.0f && b.x <= dimx - 1.0f && b.y <= dimy - 1.0f;
-    u1.st(x, y, inside ? interp_edge_x(u0, b.x, b.y) : u0.ld(x, y));
+    return inside ? interp_edge_x(u0, b.x, b.y) : u0.ld(x, y);
 }
-EFL_DEV void advect_v_at(const PF& u0, const PF& v0, const PF& v1, float dt, const Dom& d) {
-    int x = gx(), y = gy();
-    if (x >= d.ycols() || y > d.ny) return;
+EFL_DEV float advected_v(const PF& u0, const PF& v0, float dt, int x, int y) {
     float px = (float)x + 0.0f, py = (float)y + -0.5f;
     float2 b = runge_kutta(u0, v0, px, py, dt);
     float dimx = (float)v0.w, dimy = (float)v0.h;
     bool inside = b.x >= 0.0f && b.y >= 0.0f && b.x <= dimx - 1.0f && b.y <= dimy - 1.0f;
-    v1.st(x, y, inside ? interp_edge_y(v0, b.x, b.y) : v0.ld(x, y));
+    return inside ? interp_edge_y(v0, b.x, b.y) : v0.ld(x, y);
+}
+// The faces of each component's dispatch (pipeline.rs:175-186).
+template <int COMP>
+EFL_DEV bool face_covered(const Dom& d, int x, int y) {
+    return COMP == 0 ? x <= d.nx && y < d.xrows() : x < d.ycols() && y <= d.ny;
 }
 // Both passes in one launch over the larger of their grids: blockIdx.z 0 the x-major faces, 1 the y-major ones.
 __global__ void k_advect_uv(PF u0, PF v0, PF u1, PF v1, float dt, Dom d) {
-    if (blockIdx.z == 0)
-        advect_u_at(u0, v0, u1, dt, d);
-    else
-        advect_v_at(u0, v0, v1, dt, d);
+    const int x = gx(), y = gy();
+    if (blockIdx.z == 0) {
+        if (face_covered<0>(d, x, y)) u1.st(x, y, advected_u(u0, v0, dt, x, y));
+    } else {
+        if (face_covered<1>(d, x, y)) v1.st(x, y, advected_v(u0, v0, dt, x, y));
+    }
 }
 
 // exp for the Gaussian force splat.  WGSL's exp is implementation-defined
@@ -356,28 +376,51 @@ EFL_DEV float gaussian_2d(float x, float y, float x0, float y0, float sigma) {
     float dx = x - x0, dy = y - y0;
     return efl_exp(b * (dx * dx + dy * dy));
 }
-// apply_forces.wgsl:17-43 / 45-71 (comp 0 = u, x-major; comp 1 = v, y-major)
+// area_fraction(l0, l1) == 1, without the division: with m = max(l0, l1) and a = |l0 - l1|, m < a leaves m / a at most
+// 1 - 2^-24 (a float below 1), and m >= a > 0 rounds to 1 or above; 0 / 0, inf / inf and NaN give the fraction 0.
+EFL_DEV bool area_fraction_one(float l0, float l1) {
+    const float m = fmaxf(l0, l1);
+    return m >= fabsf(l0 - l1) && m > 0.0f && m < INFINITY;
+}
+// apply_forces.wgsl:17-43 / 45-71 (comp 0 = u, x-major; comp 1 = v, y-major): whether a face's velocity becomes 0 (all
+// air, or solid) ...
 template <int COMP>
-EFL_DEV void apply_forces_at(const PF& vel, const PF& ls0, const PF& face_frac, const efl_force* __restrict__ forces,
-                             int n_forces, const Uniform& U, const Dom& d) {
-    int x = gx(), y = gy();
-    if (COMP == 0 ? (x > d.nx || y >= d.xrows()) : (x >= d.ycols() || y > d.ny)) return;
-    float4 f = area_fractions(ls0, x, y);
-    float fair = COMP == 0 ? f.x : f.z;
+EFL_DEV bool face_still(const PF& ls0, const PF& face_frac, int x, int y, const Dom& d) {
     // af(idx).x / af(idx).z; outside the cell texture the reference reads 0,
     // and the face planes hold 0 there too (border faces of the solid ring).
-    float fs = (x < d.nx && y < d.ny) ? face_frac.ld(x, y) : 0.0f;
-    if (fair == 1.0f || fs == 0.0f) {
-        vel.st(x, y, 0.0f);
-        return;
+    if (!(x < d.nx && y < d.ny) || face_frac.at(x, y) == 0.0f) return true;
+    // The corners of the face (area_fractions): u faces use the columns x - 1 and x, v faces the rows y - 1 and y.
+    float m0, m1;
+    if (COMP == 0) {
+        const float c0 = ls0.ld(x - 1, y - 1), c1 = ls0.ld(x, y - 1), c3 = ls0.ld(x - 1, y), c4 = ls0.at(x, y);
+        const float c6 = ls0.ld(x - 1, y + 1), c7 = ls0.ld(x, y + 1);
+        m0 = 0.25f * (c0 + c1 + c3 + c4);
+        m1 = 0.25f * (c3 + c4 + c6 + c7);
+    } else {
+        const float c0 = ls0.ld(x - 1, y - 1), c1 = ls0.ld(x, y - 1), c2 = ls0.ld(x + 1, y - 1);
+        const float c3 = ls0.ld(x - 1, y), c4 = ls0.at(x, y), c5 = ls0.ld(x + 1, y);
+        m0 = 0.25f * (c0 + c1 + c3 + c4);
+        m1 = 0.25f * (c1 + c2 + c4 + c5);
     }
+    return area_fraction_one(m0, m1);
+}
+// ... and the velocity of the others.
+template <int COMP>
+EFL_DEV float forced(float val, const efl_force* __restrict__ forces, int n_forces, const Uniform& U, int x, int y) {
     float net = U.g[COMP];
     for (int n = n_forces; n > 0; --n) {
         const efl_force F = forces[n - 1];
         net = net + F.force[COMP] * gaussian_2d((float)x, (float)y, F.position[0], F.position[1], 10.0f);
     }
-    float val = vel.ld(x, y);
-    vel.st(x, y, val + net * U.dt / U.dx);
+    return val + net * U.dt / U.dx;
+}
+template <int COMP>
+EFL_DEV void apply_forces_at(const PF& vel, const PF& ls0, const PF& face_frac, const efl_force* __restrict__ forces,
+                             int n_forces, const Uniform& U, const Dom& d) {
+    const int x = gx(), y = gy();
+    if (!face_covered<COMP>(d, x, y)) return;
+    vel.st(x, y, face_still<COMP>(ls0, face_frac, x, y, d) ? 0.0f
+                                                           : forced<COMP>(vel.ld(x, y), forces, n_forces, U, x, y));
 }
 // Both components in one launch over the larger of their grids (blockIdx.z: 0 = u, 1 = v).
 __global__ void k_apply_forces_uv(PF u, PF v, PF ls0, PF fu, PF fv, const efl_force* __restrict__ forces, int n_forces,
@@ -386,6 +429,25 @@ __global__ void k_apply_forces_uv(PF u, PF v, PF ls0, PF fu, PF fv, const efl_fo
         apply_forces_at<0>(u, ls0, fu, forces, n_forces, U, d);
     else
         apply_forces_at<1>(v, ls0, fv, forces, n_forces, U, d);
+}
+
+// Advection and forces in one pass, as a step runs them one after the other: the advected velocity is neither written
+// nor read back, and faces that the forces set to 0 (air and solid: most of a dam break) are not advected at all
+// (4096^2: 329 + 247 us before).
+__global__ void k_advect_forces_uv(PF u0, PF v0, PF u1, PF v1, PF ls0, PF fu, PF fv,
+                                   const efl_force* __restrict__ forces, int n_forces, Uniform U, Dom d) {
+    const int x = gx(), y = gy();
+    if (blockIdx.z == 0) {
+        if (!face_covered<0>(d, x, y)) return;
+        u1.st(x, y, face_still<0>(ls0, fu, x, y, d)
+                        ? 0.0f
+                        : forced<0>(advected_u(u0, v0, U.dt, x, y), forces, n_forces, U, x, y));
+    } else {
+        if (!face_covered<1>(d, x, y)) return;
+        v1.st(x, y, face_still<1>(ls0, fv, x, y, d)
+                        ? 0.0f
+                        : forced<1>(advected_v(u0, v0, U.dt, x, y), forces, n_forces, U, x, y));
+    }
 }
 
 // divergence.wgsl:16-42 (fractions of levelset_solid = the face planes)
@@ -1255,17 +1317,27 @@ EFL_DEV float cubic1d_x(const PF& t, int bx, int by, float tx) {
     return cubic1d(t.ld(bx - 1, by), t.ld(bx, by), t.ld(bx + 1, by), t.ld(bx + 2, by), tx);
 }
 // advect_levelset.wgsl:11-34 (CUBIC defined, advect_levelset.rs:62)
-__global__ void k_advect_levelset(PF u0, PF v0, PF ls0, PF ls1, float dt, Dom d) {
-    int x = gx(), y = gy();
-    if (x >= d.cx() || y >= d.cy()) return;
+EFL_DEV float advected_level(const PF& u0, const PF& v0, const PF& ls0, float dt, const Dom& d, int x, int y) {
     float2 xn = runge_kutta(u0, v0, (float)x, (float)y, dt);
     xn.x = fclampf(xn.x, 0.0f, (float)d.nx - 1.0f);
     xn.y = fclampf(xn.y, 0.0f, (float)d.ny - 1.0f);
     int bx = f2i(xn.x), by = f2i(xn.y);
     float tx = xn.x - (float)bx, ty = xn.y - (float)by;
-    float y0 = cubic1d_x(ls0, bx, by - 1, tx), y1 = cubic1d_x(ls0, bx, by, tx);
-    float y2 = cubic1d_x(ls0, bx, by + 1, tx), y3 = cubic1d_x(ls0, bx, by + 2, tx);
-    float nl = cubic1d(y0, y1, y2, y3, ty);
+    float r[4];
+    if (bx >= 1 && by >= 1 && bx + 2 < d.nx && by + 2 < d.ny) {  // one test for the interior
+        const float* c = ls0.p + (size_t)(by - 1) * ls0.P + bx;
+#pragma unroll
+        for (int k = 0; k < 4; ++k, c += ls0.P) r[k] = cubic1d(c[-1], c[0], c[1], c[2], tx);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k] = cubic1d_x(ls0, bx, by - 1 + k, tx);
+    }
+    return cubic1d(r[0], r[1], r[2], r[3], ty);
+}
+__global__ void k_advect_levelset(PF u0, PF v0, PF ls0, PF ls1, float dt, Dom d) {
+    const int x = gx(), y = gy();
+    if (x >= d.cx() || y >= d.cy()) return;
+    const float nl = advected_level(u0, v0, ls0, dt, d, x, y);
     if (fabsf(nl) < 1000.0f) ls1.st(x, y, nl);
 }
 

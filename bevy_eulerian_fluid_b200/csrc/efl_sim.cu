@@ -306,6 +306,7 @@ efl_status st_init(efl_sim* s) {  // render_node.rs:219-277
 }
 
 efl_status st_fluid_source(efl_sim* s, const std::vector<efl_source>& src) {  // update_fluid_source.wgsl
+    if (src.empty()) return EFL_OK;  // no cell's level set and no face's velocity changes
     Dom d = s->dom();
     Sources S;
     std::memset(&S, 0, sizeof(S));
@@ -553,6 +554,16 @@ efl_status st_apply_forces(efl_sim* s) {
     g.z = 2;  // u and v faces
     k_apply_forces_uv<<<g, kBlock, count_launch(), s->stream>>>(s->u1, s->v1, s->ls0, s->fu, s->fv, s->d_forces,
                                                                  s->n_forces, s->U, d);
+    LAUNCH_CHECK();
+    return EFL_OK;
+}
+// st_advect and st_apply_forces in one pass (a step's only; the stages stay apart).
+efl_status st_advect_forces(efl_sim* s) {
+    Dom d = s->dom();
+    dim3 g = grid2d(d.nx + 1, d.ny + 1, kBlock);
+    g.z = 2;  // u and v faces
+    k_advect_forces_uv<<<g, kBlock, count_launch(), s->stream>>>(s->u0, s->v0, s->u1, s->v1, s->ls0, s->fu, s->fv,
+                                                                  s->d_forces, s->n_forces, s->U, d);
     LAUNCH_CHECK();
     return EFL_OK;
 }
@@ -1699,7 +1710,13 @@ namespace {
 efl_status run_stages(efl_sim* s, int first, int last, efl_step_stats* st) {
     efl_status ret = EFL_OK;
     for (int stage = first; stage <= last; ++stage) {
-        efl_status r = run_stage(s, stage, st);
+        efl_status r;
+        if (stage == EFL_STAGE_ADVECT_VELOCITY && last > stage) {
+            r = st_advect_forces(s);
+            ++stage;
+        } else {
+            r = run_stage(s, stage, st);
+        }
         if (r == EFL_NOT_CONVERGED) ret = r;
         else if (r != EFL_OK) return r;
     }
