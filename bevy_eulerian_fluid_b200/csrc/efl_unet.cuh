@@ -48,6 +48,11 @@ EFL_DEV uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
+// The same with both operands MN-major: in shared memory a core matrix is 8 k-rows of 8 consecutive m (or n) elements
+// (16 bytes); the descriptor's stride offset leads to the next 8 of m / n, its leading offset to the next 8 of k.
+__host__ __device__ constexpr uint32_t umma_idesc_bf16_mn(int m, int n) {
+    return umma_idesc_bf16(m, n) | (1u << 15) | (1u << 16);
+}
 EFL_DEV void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -500,14 +505,22 @@ __global__ void __launch_bounds__(CV_THREADS * TILES) k_conv3x3_rows(ConvArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// Weight gradient: dW[tap][co][ci] = sum_p dy[p][co] * x[p + tap][ci].
+// Weight gradient: dW[tap][co][ci] = sum_p dy[p][co] * x[p + tap][ci], and the bias gradient sum_p dy[p][co].
 // GEMM D[(tap, ci)][co] over K = pixels: A rows r = tap * cin + ci (M tiles of
-// 128 rows; rows beyond 9 * cin are zero), B rows co.  Each CTA reduces one
-// chunk of pixels for one M tile and writes its partial D; k_wgrad_reduce
-// sums the chunks in order.
-
-constexpr int WG_THREADS = 128, WG_K = 64;  // pixels per staged block
-constexpr int WG_SMEM = 128 * WG_K * 2 + CV_MAX_COUT * WG_K * 2 + 64;
+// 128 rows), then a row of ones (the bias; where 9 * cin leaves one), then
+// zeros; B rows co.  Each CTA reduces one chunk of pixels for one M tile and
+// writes its partial D; k_wgrad_reduce sums the chunks in order.
+//
+// Pixels are the rows of both tensors in memory, channels consecutive: the
+// operands are MN-major, so a pixel's 8 channels are one 16-byte asynchronous
+// copy to their place, four blocks of 64 pixels in flight.  (K-major operands
+// took eight 2-byte stores per copy and a barrier, a load and an MMA in turn per
+// block: 69 us a layer at 256^2, half of a training step; 1024 pixels per CTA
+// whatever the layer left the deep levels with 5 CTAs.)
+constexpr int WG_THREADS = 128, WG_K = 64, WG_STAGES = 4;  // pixels per staged block
+constexpr int WG_A = 128 * WG_K * 2;
+constexpr int wg_smem(int cout) { return WG_STAGES * (WG_A + cout * WG_K * 2) + 64; }
+constexpr int WG_SMEM = wg_smem(64);  // the widest layer
 
 struct WgradArgs {
     const bf16* x;  // forward input [H*W][xs] at xo
@@ -520,10 +533,9 @@ struct WgradArgs {
 };
 
 __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(WgradArgs a) {
-    extern __shared__ __align__(128) unsigned char wg_smem[];
-    unsigned char* As = wg_smem;                  // 128 x WG_K
-    unsigned char* Bs = wg_smem + 128 * WG_K * 2;  // cout x WG_K
-    uint64_t* bar = reinterpret_cast<uint64_t*>(wg_smem + 128 * WG_K * 2 + CV_MAX_COUT * WG_K * 2);
+    extern __shared__ __align__(128) unsigned char wg_smem_raw[];
+    const int stage_bytes = WG_A + a.cout * WG_K * 2;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(wg_smem_raw + WG_STAGES * stage_bytes);
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int npix = a.H * a.W;
@@ -531,63 +543,81 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(WgradArgs a) {
     const uint32_t ncols = tmem_cols(a.cout);
     if (warp == 0) tmem_alloc(&s_tmem, ncols);
     if (tid == 0) {
-        mbar_init(bar, 1);
+        for (int i = 0; i < WG_STAGES; ++i) mbar_init(&bar[i], 1);
         fence_mbar_init();
     }
+    // Row groups of 8 (tap, ci) rows in this tile; the one after the last holds the row of ones, the rest are zero.
+    const int groups = min(16, (9 * a.cin >> 3) - 16 * tile), og = a.cout >> 3;
+    for (int i = tid; i < WG_STAGES * (16 - groups) * WG_K; i += WG_THREADS) {
+        const int st = i / ((16 - groups) * WG_K), q = i - st * (16 - groups) * WG_K, g = groups + q / WG_K, k = q % WG_K;
+        const bool ones = g == groups && 8 * (16 * tile + g) == 9 * a.cin;
+        *reinterpret_cast<uint4*>(wg_smem_raw + st * stage_bytes + g * WG_K * 16 + k * 16) =
+            make_uint4(ones ? 0x3F80u : 0u, 0u, 0u, 0u);
+    }
+    fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    const uint32_t idesc = umma_idesc_bf16(128, a.cout);
-    const uint32_t sbo = (WG_K / 8) * 128;
-    const int og = a.cout >> 3;
+    const uint32_t idesc = umma_idesc_bf16_mn(128, a.cout);
     const int pbeg = chunk * a.pix_per_cta, pend = min(npix, pbeg + a.pix_per_cta);
+    const int nst = (pend - pbeg + WG_K - 1) / WG_K;
+    // This thread copies pixel k of every second group, from g0 on.
+    const int k = tid % WG_K, g0 = tid / WG_K;
+    int off[8], dyx[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int r0 = tile * 128 + 8 * (g0 + 2 * j), tap = r0 / a.cin, dy = tap / 3 - 1, dx = tap % 3 - 1;
+        off[j] = (dy * a.W + dx) * a.xs + a.xo + r0 - tap * a.cin;
+        dyx[j] = (dy + 1) * 4 + dx + 1;
+    }
+    auto load = [&](int st) {
+        unsigned char* As = wg_smem_raw + (st % WG_STAGES) * stage_bytes;
+        unsigned char* Bs = As + WG_A;
+        const int pp = pbeg + st * WG_K + k;
+        const bool in = pp < pend;
+        const int py = pp / a.W, px = pp - py * a.W;
+        const bf16* xp = a.x + (ptrdiff_t)pp * a.xs;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int g = g0 + 2 * j, sy = py + (dyx[j] >> 2) - 1, sx = px + (dyx[j] & 3) - 1;
+            if (g >= groups) break;
+            const bool full = in && (unsigned)sy < (unsigned)a.H && (unsigned)sx < (unsigned)a.W;
+            cp_async16(As + (g * WG_K + k) * 16, full ? xp + off[j] : a.x, full);
+        }
+        for (int g = g0; g < og; g += 2)
+            cp_async16(Bs + (g * WG_K + k) * 16, in ? a.dy + (size_t)pp * a.cout + 8 * g : a.dy, in);
+    };
+    for (int st = 0; st < WG_STAGES - 1; ++st) {
+        if (st < nst) load(st);
+        cp_async_commit();
+    }
     bool ok = true;
-    int stage = 0;
-    for (int pb = pbeg; pb < pend && ok; pb += WG_K, ++stage) {
-        // A: 16 row groups of 8 (tap, ci) rows x WG_K pixels; one 16-byte load = 8 channels of one pixel.
-        for (int i = tid; i < 16 * WG_K; i += WG_THREADS) {
-            const int g = i / WG_K, k = i - g * WG_K;
-            const int r0 = tile * 128 + 8 * g;  // first row of the group
-            const int tap = r0 / a.cin, ci0 = r0 - tap * a.cin;
-            const int pp = pb + k;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (tap < 9 && pp < pend) {
-                const int py = pp / a.W, px = pp - py * a.W;
-                const int sy = py + tap / 3 - 1, sx = px + tap % 3 - 1;
-                if ((unsigned)sy < (unsigned)a.H && (unsigned)sx < (unsigned)a.W)
-                    v = __ldg(reinterpret_cast<const uint4*>(a.x + (size_t)(sy * a.W + sx) * a.xs + a.xo + ci0));
-            }
-            const bf16* e = reinterpret_cast<const bf16*>(&v);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) *reinterpret_cast<bf16*>(As + kmajor_off(8 * g + q, k, WG_K)) = e[q];
-        }
-        // B: cout rows x WG_K pixels.
-        for (int i = tid; i < og * WG_K; i += WG_THREADS) {
-            const int g = i / WG_K, k = i - g * WG_K;
-            const int pp = pb + k;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (pp < pend) v = __ldg(reinterpret_cast<const uint4*>(a.dy + (size_t)pp * a.cout + 8 * g));
-            const bf16* e = reinterpret_cast<const bf16*>(&v);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) *reinterpret_cast<bf16*>(Bs + kmajor_off(8 * g + q, k, WG_K)) = e[q];
-        }
+    for (int st = 0; st < nst; ++st) {
+        cp_async_wait<WG_STAGES - 2>();
         fence_proxy_async();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t sa = smem_u32(As), sb = smem_u32(Bs);
+            const uint32_t sa = smem_u32(wg_smem_raw + (st % WG_STAGES) * stage_bytes), sb = sa + WG_A;
             for (int kc = 0; kc < WG_K / 16; ++kc)
-                umma_bf16(tmem, umma_desc(sa + kc * 256, 128, sbo), umma_desc(sb + kc * 256, 128, sbo), idesc,
-                          (stage | kc) != 0);
-            umma_commit(bar);
+                umma_bf16(tmem, umma_desc(sa + kc * 256, 128, WG_K * 16), umma_desc(sb + kc * 256, 128, WG_K * 16), idesc,
+                          (st | kc) != 0);
+            umma_commit(&bar[st % WG_STAGES]);
         }
-        ok = mbar_wait(bar, stage & 1);
-        if (__syncthreads_or(!ok)) ok = false;
+        // The buffer of block st - 1 takes block st + 3 once its MMAs are done.
+        if (st > 0 && ok) ok = mbar_wait(&bar[(st - 1) % WG_STAGES], ((st - 1) / WG_STAGES) & 1);
+        if (st + WG_STAGES - 1 < nst && ok) load(st + WG_STAGES - 1);
+        cp_async_commit();
     }
-    if (!ok) {
-        if (tid == 0) atomicExch(a.err, 1);
-        mbar_wait(bar, 0);
+    cp_async_wait<0>();
+    if (ok && nst > 0) ok = mbar_wait(&bar[(nst - 1) % WG_STAGES], ((nst - 1) / WG_STAGES) & 1);
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) {
+            atomicExch(a.err, 1);
+            if (nst > 0) mbar_wait(&bar[(nst - 1) % WG_STAGES], ((nst - 1) / WG_STAGES) & 1);  // copies of the MMAs in flight
+        }
+        __syncthreads();
     }
     tc_fence_after();
     const int row = 32 * warp + lane;
@@ -597,22 +627,44 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(WgradArgs a) {
         float v[16];
         tmem_ld16(taddr + (uint32_t)c0, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) dst[c0 + i] = (ok && stage > 0) ? v[i] : 0.0f;
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<float4*>(dst + c0 + 4 * i) =
+                nst > 0 ? make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]) : make_float4(0, 0, 0, 0);
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, ncols);
 }
 
-// dw[tap][co][ci] = sum over chunks in order of part[chunk][tile][r][co], r = tap * cin + ci - 128 * tile.
-__global__ void k_wgrad_reduce(const float* part, int chunks, int mtiles, int cin, int cout, float* dw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;  // over 9 * cout * cin
-    if (i >= 9 * cout * cin) return;
-    const int tap = i / (cout * cin), rem = i - tap * cout * cin, co = rem / cin, ci = rem - co * cin;
-    const int r = tap * cin + ci, tile = r >> 7, row = r & 127;
+// dw[tap][co][ci] = sum over chunks of part[chunk][tile][r][co], r = tap * cin + ci - 128 * tile, and db[co] from the
+// row of ones (db null: there is none).  32 threads along co, as the partials lie, by 8 slices of the chunks (slice q
+// adds the chunks q, q + 8, .. in order); the slices are then added in order.  (A thread for all chunks: 9.3 us a layer.)
+constexpr int WR_SLICES = 8;
+__global__ void __launch_bounds__(32 * WR_SLICES) k_wgrad_reduce(const float* part, int chunks, int mtiles, int cin,
+                                                                 int cout, float* dw, float* db) {
+    __shared__ float sums[WR_SLICES][32];
+    const int i = blockIdx.x * 32 + threadIdx.x;  // over (9 cin [+ 1]) * cout
+    const int r = i / cout, co = i - r * cout;
+    const bool in = r < 9 * cin + (db ? 1 : 0);
+    const size_t step = (size_t)mtiles * 128 * cout;
     float s = 0.0f;
-    for (int c = 0; c < chunks; ++c) s += part[(((size_t)c * mtiles + tile) * 128 + row) * cout + co];
-    dw[i] = s;
+    if (in) {
+        const float* p = part + (size_t)r * cout + co;
+#pragma unroll 4
+        for (int c = threadIdx.y; c < chunks; c += WR_SLICES) s += p[c * step];
+    }
+    sums[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y != 0 || !in) return;
+    s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < WR_SLICES; ++q) s += sums[q][threadIdx.x];
+    if (r == 9 * cin) {
+        db[co] = s;
+    } else {
+        const int tap = r / cin, ci = r - tap * cin;
+        dw[(tap * cout + co) * cin + ci] = s;
+    }
 }
 
 // db[co] = sum over pixels of dy[p][co]: per block of pix_per_block pixels,
@@ -1653,16 +1705,24 @@ inline void unet_conv_bwd(UNet& n, int i, const bf16* x, int xs, int xo, const b
     w.W = W;
     w.cin = cin;
     w.cout = cout;
-    w.pix_per_cta = 1024;
     w.part = n.wpart;
     w.err = n.err;
-    const int chunks = (npix + 1023) / 1024, mtiles = (9 * cin + 127) / 128;
-    k_wgrad_tc<<<dim3(chunks, mtiles), WG_THREADS, WG_SMEM + count_launch(), st>>>(w);
-    k_wgrad_reduce<<<lin_grid((size_t)9 * cin * cout), 256, count_launch(), st>>>(n.wpart, chunks, mtiles, cin, cout,
-                                                                                  n.grads + n.woff[i]);
-    const int bblocks = (npix + 1023) / 1024;
-    k_bgrad_partial<<<bblocks, 256, count_launch(), st>>>(n.dym, npix, cout, 1024, n.bpart);
-    k_bgrad_reduce<<<1, 64, count_launch(), st>>>(n.bpart, bblocks, cout, n.grads + n.boff[i]);
+    // About two CTAs per SM, as far as the partials' buffer goes.
+    const int mtiles = (9 * cin + 127) / 128;
+    int pix = ((int)((int64_t)npix * mtiles / 296) + WG_K - 1) / WG_K * WG_K;
+    pix = std::min(1024, std::max(WG_K, pix));
+    while ((size_t)((npix + pix - 1) / pix) * mtiles * 128 * cout > n.wpart_elems) pix *= 2;
+    w.pix_per_cta = pix;
+    const int chunks = (npix + pix - 1) / pix;
+    const bool ones = 9 * cin % 128 != 0;  // a row is left for the bias gradient
+    k_wgrad_tc<<<dim3(chunks, mtiles), WG_THREADS, wg_smem(cout) + count_launch(), st>>>(w);
+    k_wgrad_reduce<<<((9 * cin + 1) * cout + 31) / 32, dim3(32, WR_SLICES), count_launch(), st>>>(
+        n.wpart, chunks, mtiles, cin, cout, n.grads + n.woff[i], ones ? n.grads + n.boff[i] : nullptr);
+    if (!ones) {
+        const int bblocks = (npix + 1023) / 1024;
+        k_bgrad_partial<<<bblocks, 256, count_launch(), st>>>(n.dym, npix, cout, 1024, n.bpart);
+        k_bgrad_reduce<<<1, 64, count_launch(), st>>>(n.bpart, bblocks, cout, n.grads + n.boff[i]);
+    }
     if (gx) {
         ConvArgs a;
         a.x = n.dym;

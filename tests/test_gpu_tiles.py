@@ -116,3 +116,26 @@ def test_solve_on_tiles_with_water(oracle_api, gpu_api, nx, ny):
         so, sg = o.step(scenes.DT), g.step(scenes.DT)
         assert so.pressure_iterations == sg.pressure_iterations
     assert not compare_fields(g, o)
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 16), (104, 72), (48, 200), (264, 64)])
+def test_weight_gradients_of_ragged_images(gpu_api, nx, ny):
+    """The weight- and bias-gradient GEMMs where the last block of 64 pixels, the last chunk and the last tile of 128
+    rows are partial; bounds as for the network's other gradients (ReLU and bf16 flips reach a few percent)."""
+    from oracle import unet_ref
+
+    from .test_unet import _random_case, _rel
+    params, feats, target, mask = _random_case(21, n=ny, nx=nx)
+    net = capi.UNet(gpu_api, nx, ny)
+    net.set_params(params)
+    loss, g = net.gradients(feats, target, mask)
+    ref = unet_ref.Net(params)
+    ref.forward(feats)
+    rloss, rg = ref.backward(target, mask)
+    cos = float(g.astype(np.float64) @ rg / (np.linalg.norm(g) * np.linalg.norm(rg)))
+    assert loss == pytest.approx(rloss, rel=2e-3) and cos > 0.998 and _rel(g, rg) < 0.06
+    off = 0
+    for ci, co, _ in unet_ref.SPEC:  # each layer's bias gradient: a row of its own in the GEMM
+        off += 9 * ci * co
+        assert _rel(g[off:off + co], rg[off:off + co]) < 0.08
+        off += co
