@@ -72,6 +72,13 @@ EFL_DEV float div_any(float a, float b) {
     asm volatile("" : "+f"(a));
     return a / b;
 }
+// The same for numerators that may be zero themselves: the quotient of a zero is that zero with the product's sign
+// (NaN from a NaN or zero b).
+EFL_DEV float div_zero(float a, float b) {
+    const float q = div_any(a == 0.0f ? 1.0f : a, b);
+    const float z = __uint_as_float((__float_as_uint(a) ^ __float_as_uint(b)) & 0x80000000u);
+    return a != 0.0f || b != b ? q : b != 0.0f ? z : __int_as_float(0x7fc00000);
+}
 EFL_DEV float wmix(float a, float b, float t) { return a * (1.0f - t) + b * t; }
 EFL_DEV int f2i(float v) { return __float2int_rz(v); }  // truncate, saturate, NaN -> 0
 EFL_DEV float2 mat_xy(const float* m, float x, float y) {

@@ -700,13 +700,22 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
 
 // The reference's fixed-count f32 sweeps (gauss_seidel.wgsl:12-88, `iters`
 // red-black iterations, red first) as ONE cooperative launch for grids of at
-// most one 64 x 32 tile per SM (C1's 256^2, 512^2): the 2 x 2-block layout
-// of k_gsmix_quad on the pressure itself.  Per cell, with the reference's f32
+// most one tile per SM: a thread holds a 2 x 2 block of the tile and its halo.
+// Per cell, with the reference's f32
 // coefficients: update cells p = w (nume / den) + (1 - w) p, zero cells
 // (air, fully solid, |den| < 1e-6) p = 0, the outermost ring untouched.  The
-// owned cells are exchanged through L2 every 4 iterations (alternating
-// planes) and stored to `out` after a last grid barrier (no CTA may still be
-// loading its first image from `out`).
+// owned cells are exchanged through L2 every KMAX iterations (alternating
+// planes) and stored to `out` once no CTA may still be loading its first
+// image from `out`: after an exchange, or a grid barrier of its own.
+//
+// Bound by the latency of the slowest warp between two block barriers, and by
+// the exchanges (2.4 us each).  So: both cells of a colour side by side, no
+// weights and no division in warps of standard cells, and no lane that divides
+// by zero or divides a zero (the division's slow path: a warp with such a lane
+// took 1000 cycles for a half-sweep, the others 200), and every load of the
+// first image in flight at once.  20 iterations: 41.3 -> 30.4 us at 64 x 64,
+// 44.0 -> 32.7 us at 256 x 256, 41.6 -> 33.0 us at 512 x 512 on tiles of
+// 64 x 32 cells, and 20.0 and 21.5 us (64 x 64, 256 x 256) on the small tiles.
 template <int EX, int EY>
 struct Quad32Tile {
     static constexpr int W2 = EX / 2, NB = (EX / 2) * (EY / 2);
@@ -723,19 +732,36 @@ struct Gs32Params {
     long long spin_limit;
     int* err;  // set to 2 if a grid barrier timed out (reported with the TMA sweep's flag)
 };
-EFL_DEV float gs32_update(float cb, float4 w, float den, float p, float pl, float pr, float pu, float pd, float wgt,
-                          float omw, unsigned upd, unsigned zero) {
-    float nume = cb;
-    nume = nume + w.x * pl;
-    nume = nume + w.y * pr;
-    nume = nume + w.z * pu;
-    nume = nume + w.w * pd;
-    const float pn = div_any(upd ? nume : 1.0f, den);
-    const float v = wgt * pn + omw * p;
-    return upd ? v : (zero ? 0.0f : p);
+// Two cells of one colour.  general: some update cell of the warp is not standard (w = 1, den = 4: nume / 4 is
+// nume * 0.25 exactly, without the weights and the division).
+EFL_DEV void gs32_update2(bool general, float cb0, const float4* w0, float den0, float& p0, float l0, float r0, float u0,
+                          float d0, unsigned upd0, unsigned zero0, float cb1, const float4* w1, float den1, float& p1,
+                          float l1, float r1, float u1, float d1, unsigned upd1, unsigned zero1, float wgt, float omw) {
+    float n0 = cb0, n1 = cb1;
+    if (general) {
+        const float4 a = *w0, b = *w1;
+        n0 = n0 + a.x * l0;
+        n1 = n1 + b.x * l1;
+        n0 = n0 + a.y * r0;
+        n1 = n1 + b.y * r1;
+        n0 = n0 + a.z * u0;
+        n1 = n1 + b.z * u1;
+        n0 = n0 + a.w * d0;
+        n1 = n1 + b.w * d1;
+        n0 = div_zero(upd0 ? n0 : 1.0f, den0);
+        n1 = div_zero(upd1 ? n1 : 1.0f, den1);
+    } else {
+        n0 = (((n0 + l0) + r0) + u0) + d0;
+        n1 = (((n1 + l1) + r1) + u1) + d1;
+        n0 = n0 * 0.25f;
+        n1 = n1 * 0.25f;
+    }
+    const float v0 = wgt * n0 + omw * p0, v1 = wgt * n1 + omw * p1;
+    p0 = upd0 ? v0 : (zero0 ? 0.0f : p0);
+    p1 = upd1 ? v1 : (zero1 ? 0.0f : p1);
 }
 template <int EX, int EY, int KMAX, int NT>
-__global__ void __launch_bounds__(NT, 1) k_gs32_quad(Gs32Params P) {
+__global__ void __launch_bounds__(NT, NT < 512 ? 2 : 1) k_gs32_quad(Gs32Params P) {
     static_assert((EX / 2) * (EY / 2) <= NT && NT % 32 == 0 && EX % 2 == 0 && EY % 2 == 0, "2 x 2 blocks");
     extern __shared__ __align__(16) unsigned char q32_raw[];
     Quad32Tile<EX, EY>& T = *reinterpret_cast<Quad32Tile<EX, EY>*>(q32_raw);
@@ -752,82 +778,103 @@ __global__ void __launch_bounds__(NT, 1) k_gs32_quad(Gs32Params P) {
     float pv[4], cb[4], den[4];
     unsigned fl = 0;  // bit q: update; bit 4 + q: zero; bit 8 + q: live (in the domain, not the outer ring);
                       // bit 16 + q: owned and in the domain
+    unsigned gen = 0;  // a live update cell that is not standard; then: one in the warp
+    // Every load of the block first, at clamped places (three dependent rounds per cell otherwise).
+    const int bgx = gx0 + 2 * bx, bgy = gy0 + 2 * by;
+    float lv[4][4], fu[2][3], fv[3][2], xb0[4], bb[4];
+    {
+        const int xs[4] = {min(max(bgx - 1, 0), L.nx - 1), min(max(bgx, 0), L.nx - 1), min(max(bgx + 1, 0), L.nx - 1),
+                           min(max(bgx + 2, 0), L.nx - 1)};
+        const int ys[4] = {min(max(bgy - 1, 0), L.ny - 1), min(max(bgy, 0), L.ny - 1), min(max(bgy + 1, 0), L.ny - 1),
+                           min(max(bgy + 2, 0), L.ny - 1)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if ((i == 1 || i == 2) || (j == 1 || j == 2)) lv[j][i] = L.ls.at(xs[i], ys[j]);
+        const int fx[3] = {xs[1], min(max(bgx + 1, 0), L.nx), min(max(bgx + 2, 0), L.nx)};
+        const int fy[3] = {ys[1], min(max(bgy + 1, 0), L.ny), min(max(bgy + 2, 0), L.ny)};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                xb0[2 * j + i] = L.x.at(xs[1 + i], ys[1 + j]);
+                bb[2 * j + i] = L.b.at(xs[1 + i], ys[1 + j]);
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                fu[j][i] = L.fu.at(fx[i], ys[1 + j]);
+                fv[i][j] = L.fv.at(xs[1 + j], fy[i]);
+            }
+        }
+    }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const int lx = 2 * bx + (q & 1), ly = 2 * by + (q >> 1);
-        const int gx = gx0 + lx, gy = gy0 + ly;
-        const bool edge = (ring0x && ((q & 1) == (bx == 0 ? 0 : 1))) || (ring0y && ((q >> 1) == (by == 0 ? 0 : 1)));
+        const int qx = q & 1, qy = q >> 1;
+        const int gx = bgx + qx, gy = bgy + qy;
+        const bool edge = (ring0x && (qx == (bx == 0 ? 0 : 1))) || (ring0y && (qy == (by == 0 ? 0 : 1)));
         float4 wk = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         pv[q] = 0.0f;
         cb[q] = 0.0f;
-        den[q] = 0.0f;
+        den[q] = 1.0f;  // of every lane that divides: a zero would take the slow path
         if (active && (unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny) {
-            pv[q] = L.x.at(gx, gy);
+            pv[q] = xb0[q];
             if (owned) fl |= 1u << (16 + q);
-            const float lij = L.ls.at(gx, gy);
+            const float lij = lv[1 + qy][1 + qx];
             bool update = false;
             float dn = 0.0f;
-            if (lij < 0.0f) {
-                const float f[4] = {L.fu.at(gx, gy), L.fu.at(gx + 1, gy), L.fv.at(gx, gy), L.fv.at(gx, gy + 1)};
-                if (!(f[0] == 0.0f && f[1] == 0.0f && f[2] == 0.0f && f[3] == 0.0f)) {
-                    cb[q] = P.cdiv * L.b.at(gx, gy);
-                    const int ox[4] = {-1, 1, 0, 0}, oy[4] = {0, 0, -1, 1};
-                    float wv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const float f[4] = {fu[qy][qx], fu[qy][qx + 1], fv[qy][qx], fv[qy + 1][qx]};
+            if (lij < 0.0f && !(f[0] == 0.0f && f[1] == 0.0f && f[2] == 0.0f && f[3] == 0.0f)) {
+                cb[q] = P.cdiv * bb[q];
+                const float ln[4] = {lv[1 + qy][qx], lv[1 + qy][qx + 2], lv[qy][1 + qx], lv[qy + 2][1 + qx]};
+                const bool in[4] = {gx > 0, gx + 1 < L.nx, gy > 0, gy + 1 < L.ny};
+                float wv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int jx = gx + ox[k], jy = gy + oy[k];
-                        if ((unsigned)jx < (unsigned)L.nx && (unsigned)jy < (unsigned)L.ny) {
-                            const float level = L.ls.at(jx, jy);
-                            if (level < 0.0f) {
-                                dn += f[k];
-                                wv[k] = f[k];
-                            } else {
-                                dn += f[k] * (1.0f - level / lij);
-                            }
-                        }
+                for (int k = 0; k < 4; ++k) {
+                    if (!in[k]) continue;
+                    if (ln[k] < 0.0f) {
+                        dn += f[k];
+                        wv[k] = f[k];
+                    } else {
+                        dn += f[k] * (1.0f - ln[k] / lij);
                     }
-                    wk = make_float4(wv[0], wv[1], wv[2], wv[3]);
-                    update = !(fabsf(dn) < 1.0e-6f);
                 }
+                wk = make_float4(wv[0], wv[1], wv[2], wv[3]);
+                update = !(fabsf(dn) < 1.0e-6f);
             }
             den[q] = update ? dn : 1.0f;
             if (!edge) fl |= (update ? 1u << q : 1u << (4 + q)) | (1u << (8 + q));
+            if (!edge && update && !(wk.x == 1.0f && wk.y == 1.0f && wk.z == 1.0f && wk.w == 1.0f)) gen = 1u;
         }
         if (active) {
             T.w[q][threadIdx.x] = wk;
-            T.p[(q == 0 || q == 3) ? 0 : 1][ly][bx] = pv[q];
+            T.p[(q == 0 || q == 3) ? 0 : 1][2 * by + qy][bx] = pv[q];
         }
     }
     __syncthreads();
+    gen = __reduce_or_sync(0xffffffffu, gen);
     const float wgt = P.weight, omw = 1.0f - P.weight;
     const int t = active ? (int)threadIdx.x : 0;
     const int r0 = 2 * by, r1 = 2 * by + 1;
     const int bxl = bx > 0 ? bx - 1 : 0, bxr = bx < W2 - 1 ? bx + 1 : bx;
     const int rup = r0 > 0 ? r0 - 1 : 0, rdn = r1 < EY - 1 ? r1 + 1 : r1;
     const int bring = min(min(2 * bx + 1, EX - 2 * bx), min(2 * by + 1, EY - 2 * by)) - 1;
+    // both cells of a colour side by side, stored under a predicate
     auto sweep_base = [&]() {  // cells 0 and 3; neighbours of the other colour
         float(*Po)[WP] = T.p[1];
         const float pl0 = Po[r0][bxl], pu0 = Po[rup][bx], pr3 = Po[r1][bxr], pd3 = Po[rdn][bx];
-        if (fl & 0x100u) {
-            pv[0] = gs32_update(cb[0], T.w[0][t], den[0], pv[0], pl0, pv[1], pu0, pv[2], wgt, omw, fl & 1u, fl & 0x10u);
-            T.p[0][r0][bx] = pv[0];
-        }
-        if (fl & 0x800u) {
-            pv[3] = gs32_update(cb[3], T.w[3][t], den[3], pv[3], pv[2], pr3, pv[1], pd3, wgt, omw, fl & 8u, fl & 0x80u);
-            T.p[0][r1][bx] = pv[3];
-        }
+        gs32_update2(gen, cb[0], &T.w[0][t], den[0], pv[0], pl0, pv[1], pu0, pv[2], fl & 1u, fl & 0x10u, cb[3],
+                     &T.w[3][t], den[3], pv[3], pv[2], pr3, pv[1], pd3, fl & 8u, fl & 0x80u, wgt, omw);
+        if (fl & 0x100u) T.p[0][r0][bx] = pv[0];
+        if (fl & 0x800u) T.p[0][r1][bx] = pv[3];
     };
     auto sweep_other = [&]() {  // cells 1 and 2; neighbours of the base colour
         float(*Po)[WP] = T.p[0];
         const float pr1 = Po[r0][bxr], pu1 = Po[rup][bx], pl2 = Po[r1][bxl], pd2 = Po[rdn][bx];
-        if (fl & 0x200u) {
-            pv[1] = gs32_update(cb[1], T.w[1][t], den[1], pv[1], pv[0], pr1, pu1, pv[3], wgt, omw, fl & 2u, fl & 0x20u);
-            T.p[1][r0][bx] = pv[1];
-        }
-        if (fl & 0x400u) {
-            pv[2] = gs32_update(cb[2], T.w[2][t], den[2], pv[2], pl2, pv[3], pv[0], pd2, wgt, omw, fl & 4u, fl & 0x40u);
-            T.p[1][r1][bx] = pv[2];
-        }
+        gs32_update2(gen, cb[1], &T.w[1][t], den[1], pv[1], pv[0], pr1, pu1, pv[3], fl & 2u, fl & 0x20u, cb[2],
+                     &T.w[2][t], den[2], pv[2], pl2, pv[3], pv[0], pd2, fl & 4u, fl & 0x40u, wgt, omw);
+        if (fl & 0x200u) T.p[1][r0][bx] = pv[1];
+        if (fl & 0x400u) T.p[1][r1][bx] = pv[2];
     };
     bool ok = true;
     int xch = 0;
@@ -875,7 +922,8 @@ __global__ void __launch_bounds__(NT, 1) k_gs32_quad(Gs32Params P) {
             __syncthreads();
         }
     }
-    if (ok) ok = grid_barrier(P.barrier, nblocks, P.spin_limit);  // every CTA has read its first image of x
+    // every CTA has read its first image of x: an exchange said so already
+    if (ok && xch == 0) ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
     if (!ok && threadIdx.x == 0) atomicExch(P.err, 2);
     if (ok && owned) {
 #pragma unroll
@@ -884,17 +932,12 @@ __global__ void __launch_bounds__(NT, 1) k_gs32_quad(Gs32Params P) {
     }
 }
 
-// n fixed f32 red-black iterations at level 0 as one cooperative launch, when
-// the grid fits one 64 x 32 tile per SM.  EFL_ERR_STATE: it does not (use the
-// TMA-streamed sweeps).
-inline efl_status solve_gs32_persistent(SolverWorkspace& ws, const Level& L, const PF& xa, const PF& xb,
-                                        float dx_scaled, float rho, float dt, float weight, uint32_t n,
-                                        int* dev_err, cudaStream_t stream, std::string* err) {
-    constexpr int EX = 80, EY = 48, KMAX = 4, NT = 960;
+template <int EX, int EY, int KMAX, int NT>
+inline efl_status launch_gs32_quad(SolverWorkspace& ws, Gs32Params P, cudaStream_t stream, std::string* err) {
     constexpr int TXo = EX - 4 * KMAX, TYo = EY - 4 * KMAX;
-    const int tiles_x = (L.nx + TXo - 1) / TXo, tiles_y = (L.ny + TYo - 1) / TYo;
-    if (n == 0) return EFL_OK;
+    const int tiles_x = (P.L.nx + TXo - 1) / TXo, tiles_y = (P.L.ny + TYo - 1) / TYo;
     if (tiles_x * tiles_y > ws.num_sms) return EFL_ERR_STATE;
+    P.tiles_x = tiles_x;
     const void* kern = (const void*)k_gs32_quad<EX, EY, KMAX, NT>;
     const size_t smem = sizeof(Quad32Tile<EX, EY>);
     static bool attr_done[64] = {};
@@ -908,18 +951,6 @@ inline efl_status solve_gs32_persistent(SolverWorkspace& ws, const Level& L, con
         }
         attr_done[dev] = true;
     }
-    Gs32Params P;
-    P.L = L;
-    P.xb[0] = xa;
-    P.xb[1] = xb;
-    P.tiles_x = tiles_x;
-    P.iters = (int)n;
-    P.cdiv = dx_scaled * dx_scaled * rho / dt;  // gauss_seidel.wgsl:58
-    P.weight = weight;
-    P.barrier = ws.barrier;
-    P.spin_limit = ws.spin_limit > 0 ? ws.spin_limit : kBarrierSpinLimit;
-    P.err = dev_err;
-    if (!dev_err) return EFL_ERR_STATE;
     if (cudaMemsetAsync(ws.barrier, 0, sizeof(GridBarrier), stream) != cudaSuccess) {
         *err = "barrier reset failed";
         return EFL_ERR_CUDA;
@@ -932,6 +963,34 @@ inline efl_status solve_gs32_persistent(SolverWorkspace& ws, const Level& L, con
         return EFL_ERR_CUDA;
     }
     return EFL_OK;
+}
+
+// n fixed f32 red-black iterations at level 0 as one cooperative launch, when
+// the grid fits one tile per SM: tiles of 32 x 16 cells, exchanged every 5
+// iterations, where they do (256 x 256, 20 iterations: 21.5 us, against 32.7 us
+// on the larger ones), else 64 x 32, every 4 (512 x 512: 33 us).  32 x 16 cells
+// every 4, 6 and 7 iterations took 22.3, 23.0 and 22.4 us at 256 x 256.
+// Two blocks of the small kernel fit an SM, so that simulations in flight together run side by side (three of
+// 256 x 256: 45 us a frame; 54 us with one block per SM, 45 us on the larger tiles, whose frame alone takes 9 us more).
+// EFL_ERR_STATE: it fits neither (use the TMA-streamed sweeps).
+inline efl_status solve_gs32_persistent(SolverWorkspace& ws, const Level& L, const PF& xa, const PF& xb,
+                                        float dx_scaled, float rho, float dt, float weight, uint32_t n,
+                                        int* dev_err, cudaStream_t stream, std::string* err) {
+    if (n == 0) return EFL_OK;
+    if (!dev_err) return EFL_ERR_STATE;
+    Gs32Params P;
+    P.L = L;
+    P.xb[0] = xa;
+    P.xb[1] = xb;
+    P.tiles_x = 0;
+    P.iters = (int)n;
+    P.cdiv = dx_scaled * dx_scaled * rho / dt;  // gauss_seidel.wgsl:58
+    P.weight = weight;
+    P.barrier = ws.barrier;
+    P.spin_limit = ws.spin_limit > 0 ? ws.spin_limit : kBarrierSpinLimit;
+    P.err = dev_err;
+    const efl_status st = launch_gs32_quad<52, 36, 5, 480>(ws, P, stream, err);
+    return st == EFL_ERR_STATE ? launch_gs32_quad<80, 48, 4, 960>(ws, P, stream, err) : st;
 }
 
 // Global-memory form of the same solve for grids the persistent scheme

@@ -139,3 +139,17 @@ def test_weight_gradients_of_ragged_images(gpu_api, nx, ny):
         off += 9 * ci * co
         assert _rel(g[off:off + co], rg[off:off + co]) < 0.08
         off += co
+
+
+@pytest.mark.parametrize("nx,ny,iterations", [(16, 16, 1), (32, 16, 5), (64, 64, 6), (72, 40, 10), (200, 136, 11),
+                                              (256, 256, 20), (384, 192, 4), (392, 200, 20), (512, 512, 9)])
+def test_fixed_count_sweeps_on_both_tiles(oracle_api, gpu_api, nx, ny, iterations):
+    """Fixed-count red-black sweeps in one launch: 32 x 16 tiles, exchanged every 5 iterations, where one per SM holds
+    the grid, else 64 x 32 every 4."""
+    sc = _splash(nx, ny)
+    sc.cfg.projection.gs_iterations = iterations
+    o, g = make_pair(sc, oracle_api, gpu_api)
+    for _ in range(5):
+        o.step(scenes.DT)
+        g.step(scenes.DT)
+    assert not compare_fields(g, o)
