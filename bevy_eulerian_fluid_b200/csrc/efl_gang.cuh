@@ -7,8 +7,9 @@
 // becomes idle, the largest simulation that fits the idle CTAs starts (a list in global memory behind a lock).  The
 // streamed form (efl_batch.cuh) runs every simulation in lockstep, each round reading every active tile from L2 behind
 // a barrier of the whole device: about 10 us per red-black iteration whatever the number of simulations left, against
-// 1.1 us here.  64 x 32 tiles and 8 iterations between exchanges because of the throughput per SM, 1837 cells per us
-// (64 x 56 and 4: 2108, but 1.7 us per iteration and coarser tiles; 32 x 32 and 8: 1093).
+// 0.9 us here.  64 x 32 tiles because of the throughput per SM, 2190 cells per us (32 x 32: 1380; 64 x 56: 2108, but
+// 1.7 us per iteration and coarser tiles).  A step of 32 pools of 128^2 to 768^2: 91 ms; with an exchange every 8
+// iterations instead of 4, by 4 x 4 blocks that spill, 134 ms.
 //
 // Each simulation's iterates and iteration count are those of its own solve.  Every wait is bounded.
 #pragma once
@@ -17,13 +18,12 @@
 
 namespace efl {
 
-#define GANG_TILE 96, 64, 8, 384, 4
-constexpr int GANG_THREADS = 384, GANG_TX = 64, GANG_TY = 32;
+#define GANG_TILE OCT_MEDIUM
+constexpr int GANG_THREADS = 480, GANG_TX = 64, GANG_TY = 32;
 constexpr int GANG_MAX_SIMS = 512, GANG_MAX_CTAS = 512;
 
 struct GangSim {
     PersistentParams P;
-    PF dbuf;
 };
 struct GangState {  // zeroed before each launch
     unsigned lock;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_batch_gang(const GangSim* s
         const int2 j = job;
         if (j.x < 0) return;
         load(j.x);
-        if (!oct_solve<GANG_TILE>(S.P, S.dbuf, list, (unsigned)j.y, (unsigned)n)) {
+        if (!oct_solve<GANG_TILE>(S.P, list, (unsigned)j.y, (unsigned)n)) {
             if (threadIdx.x == 0) atomicExch(&G->error, 1);
             return;
         }

@@ -800,9 +800,7 @@ efl_status ensure_mix_planes(efl_sim* s) {
 efl_status gs_mixed(efl_sim* s, float weight, double tol, uint32_t max_iters, uint32_t check, SolveResult* res) {
     const Level64& L = s->mg64[0];
     std::string perr;
-    if (!s->xbuf.p) TRY(alloc_plane(s, s->xbuf, s->nx, s->ny, s->P, s->ny + 1));
-    efl_status ps = solve_gsmix_persistent(s->solver, L, s->r0, s->xbuf, s->U, weight, tol, max_iters, check,
-                                           s->stream, res, &perr);
+    efl_status ps = solve_gsmix_persistent(s->solver, L, s->U, weight, tol, max_iters, check, s->stream, res, &perr);
     if (ps == EFL_OK) return EFL_OK;
     if (ps != EFL_ERR_STATE) return set_err(s, ps, "%s", perr.c_str());
     TRY(ensure_mix_planes(s));
@@ -2391,7 +2389,7 @@ void launch_wet_blocks(efl_sim* s) {
 // gets those whose tiles with water do not fit the device.
 efl_status gang_solve(efl_batch* b, const std::vector<int>& which, efl_step_stats* stats, std::vector<int>* rest) {
     const void* kern = (const void*)k_batch_gang;
-    const size_t smem = sizeof(OctTile<96, 64, 4>);
+    const size_t smem = sizeof(OctTile<80, 48, 2>);
     const int sms = b->sims[which[0]]->solver.num_sms;
     int per_sm = 0;
     if (sms > GANG_MAX_CTAS ||
@@ -2428,11 +2426,10 @@ efl_status gang_solve(efl_batch* b, const std::vector<int>& which, efl_step_stat
             P.barrier = b->d_gang_barrier + hs.size();
             P.result = b->d_gang_result + hs.size();
             P.spin_limit = b->spin_limit > 0 ? b->spin_limit : kBarrierSpinLimit;
-            P.dbuf2 = s->xbuf;
+            P.xch = s->solver.xch;
             P.one = 1.0f;
             P.wet = s->solver.wet;
             P.wet_w = (s->nx + 31) / 32;
-            S.dbuf = s->r0;
             hs.push_back(S);
             ids.push_back(which[at]);
         }
@@ -2641,6 +2638,11 @@ efl_status efl_batch_create(const efl_config* cfgs, uint32_t n, efl_batch** out)
             std::string m = s->err;
             batch_free(b);
             return batch_err(nullptr, EFL_ERR_OUT_OF_MEMORY, m);
+        }
+        const int gang_tiles = ((s->nx + GANG_TX - 1) / GANG_TX) * ((s->ny + GANG_TY - 1) / GANG_TY);
+        if (!oct_reserve(s->solver, oct_xch_bytes(std::min(gang_tiles, s->solver.num_sms), GANG_TX * GANG_TY))) {
+            batch_free(b);
+            return batch_err(nullptr, EFL_ERR_OUT_OF_MEMORY, "batch workspace allocation failed");
         }
         total_tiles += ((s->nx + kMinTile - 1) / kMinTile) * ((s->ny + kMinTile - 1) / kMinTile);
     }

@@ -55,6 +55,8 @@ struct SolverWorkspace {
     int max_blocks = 0;
     long long spin_limit = 0;  // grid-barrier polls before giving up (0: kBarrierSpinLimit)
     unsigned char* wet = nullptr;  // per 32 x 8 block: holds a cell with level set < 0 (k_wet_blocks)
+    ulonglong2* xch = nullptr;     // the persistent solve's exchanges (its first solve allocates them)
+    size_t xch_bytes = 0;
 };
 
 
@@ -112,7 +114,7 @@ struct PersistentParams {
     GridBarrier* barrier;
     SolveResult* result;
     long long spin_limit;  // grid-barrier polls before giving up
-    PF dbuf2;              // the exchanges alternate between the correction planes dbuf and dbuf2
+    ulonglong2* xch;       // the exchanges' tagged words (oct_xch_bytes)
     float one;             // 1.0f, passed at run time (see x2_add1)
     const unsigned char* wet;  // per 32 x 8 block of cells (row pitch wet_w): holds a cell with level set < 0
     int wet_w, ntiles;
@@ -190,6 +192,7 @@ inline void solver_free(SolverWorkspace& ws) {
     if (ws.barrier) cudaFree(ws.barrier);
     if (ws.result) cudaFree(ws.result);
     if (ws.partials) cudaFree(ws.partials);
+    if (ws.xch) cudaFree(ws.xch);
     if (ws.wet) cudaFree(ws.wet);
     if (ws.h_result) cudaFreeHost(ws.h_result);
     ws = SolverWorkspace{};
@@ -312,13 +315,81 @@ struct OctTile {
 EFL_DEV constexpr int oct_pair(int q) { return 2 * (q >> 2) + (((q & 3) + (q >> 2)) & 1); }
 EFL_DEV constexpr int oct_lane(int q) { return (q & 3) >> 1; }
 
+// Exchanges between the CTAs of a solve: words of 32 bits of data under a 32-bit tag, written and polled as 64-bit
+// relaxed accesses, which are indivisible.  The receiver waits for the tag of the exchange on the data itself, so an
+// exchange costs a store and a load of L2 and no fence, no flag and no barrier (a grid barrier and the loads behind it
+// took 3 us of every 8 iterations: 0.94 us per iteration on a 512^2 pool).  Tags only grow within a solve and the
+// words are cleared before its first barrier; two buffers alternate, which suffices because every CTA waits in each
+// exchange for all the CTAs that read its words.
+EFL_DEV void xch_store(ulonglong2* p, uint32_t a, uint32_t b, uint32_t tag) {
+    const unsigned long long t = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | a), "l"(t | b) : "memory");
+}
+// N pairs of words `stride` apart, when all carry the tag.  False: `limit` polls, or another CTA's, ran out.
+template <int N>
+EFL_DEV bool xch_poll(const ulonglong2* p, int stride, uint32_t tag, ulonglong2 (&w)[N], GridBarrier* gb,
+                      long long limit) {
+    for (long long spins = 0;;) {
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
+                         : "=l"(w[k].x), "=l"(w[k].y)
+                         : "l"(p + (size_t)k * stride)
+                         : "memory");
+        bool got = true;
+#pragma unroll
+        for (int k = 0; k < N; ++k) got = got && (uint32_t)(w[k].x >> 32) == tag && (uint32_t)(w[k].y >> 32) == tag;
+        if (got) return true;
+        if ((++spins & 1023) == 0 || spins >= limit) {
+            int e;
+            asm volatile("ld.acquire.gpu.s32 %0, [%1];" : "=r"(e) : "l"(&gb->error) : "memory");
+            if (e || spins >= limit) {
+                atomicExch(&gb->error, 1);
+                return false;
+            }
+        }
+    }
+}
+EFL_DEV double xch_double(ulonglong2 w) {
+    return __longlong_as_double((long long)((w.x & 0xffffffffull) | (w.y << 32)));
+}
+EFL_DEV void xch_store(ulonglong2* p, double v, uint32_t tag) {
+    xch_store(p, (uint32_t)__double2loint(v), (uint32_t)__double2hiint(v), tag);
+}
+
 // The tiles (TX x TY owned cells, multiples of 32 and 8) of a level that hold a cell with level set < 0, in tile order,
 // and after them the others: list[0 .. *n), list[*n .. ntiles).  The whole CTA calls it.
 constexpr int OCT_MAX_TILES = 1024;
-// The smallest tiles first: a CTA's sweeps cover its image, 64 x 64 cells here and 96 x 64 in the next form (0.94
-// against 1.11 us per red-black iteration on a 512^2 pool), and tiles without water need no CTA, so 32 x 32 tiles fit
-// the device up to 148 x 1024 cells of water.  The same tile by 4 x 2 blocks of cells (512 threads): 0.955 us.
+constexpr size_t OCT_XCH_SUMS = 2 * 2 * OCT_MAX_TILES;  // the residual sums of every CTA, then its cells
+// Bytes of the exchanges of `ctas` CTAs that own `cells` cells each.
+inline size_t oct_xch_bytes(int ctas, int cells) { return (OCT_XCH_SUMS + 2 * (size_t)ctas * cells) * sizeof(ulonglong2); }
+// ps_total_relative of the sums of check `tag`, in the first warp (every lane); false: a wait ran out.
+EFL_DEV bool oct_total_relative(const ulonglong2* sums, uint32_t tag, int nblocks, GridBarrier* gb, long long limit,
+                                double* rel) {
+    double r = 0.0, b = 0.0;
+    bool got = true;
+    for (int i = threadIdx.x; i < nblocks && got; i += 32) {
+        ulonglong2 w[2];
+        got = xch_poll(sums + ((tag & 1) * OCT_MAX_TILES + i) * 2, 1, tag, w, gb, limit);
+        r += xch_double(w[0]);
+        b += xch_double(w[1]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        r += __shfl_xor_sync(0xffffffffu, r, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    *rel = b > 0.0 ? sqrt(r) / sqrt(b) : (r > 0.0 ? __longlong_as_double(0x7ff0000000000000ll) : 0.0);
+    return got;
+}
+// The smallest tiles first: a CTA's sweeps cover its image, 64 x 64 cells here, and tiles without water need no CTA, so
+// 32 x 32 tiles fit the device up to 148 x 1024 cells of water.  0.74 us per red-black iteration on a 512^2 pool; the
+// same tile by 4 x 2 blocks of cells (512 threads) 0.79, exchanged every 6 iterations 0.86, every 4 iterations 0.91
+// (0.80 by 4 x 2 blocks), every 2 iterations 1.20.
 #define OCT_SMALL 64, 64, 8, 256, 4
+// Twice the cells per CTA, by 4 x 2 blocks so that a thread's coefficients stay in its registers: 0.93 us on a full
+// 768 x 640 pool; by 4 x 4 blocks 1.00 (256 threads), and exchanged every 8 iterations 1.40 (384 threads, spilled).
+#define OCT_MEDIUM 80, 48, 4, 480, 2
 template <int TX, int TY, int NT>
 EFL_DEV void oct_tiles(const PersistentParams& P, unsigned short* list, int* n) {
     static_assert(TX % 32 == 0 && TY % 8 == 0, "whole blocks");
@@ -359,8 +430,7 @@ EFL_DEV void oct_tiles(const PersistentParams& P, unsigned short* list, int* n) 
 // simulation's active tiles: a tile without a cell of level set < 0 takes no part, as its correction is 0 and no
 // weight points at its cells).  False: a grid barrier timed out.
 template <int EX, int EY, int KMAX, int NT, int ROWS>
-EFL_DEV bool oct_solve(const PersistentParams& P, const PF& dbuf, const unsigned short* list, unsigned rank,
-                       unsigned nblocks) {
+EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, unsigned rank, unsigned nblocks) {
     using Tile = OctTile<EX, EY, ROWS>;
     constexpr int NC = 4 * ROWS, NPAIR = 2 * ROWS;
     static_assert(KMAX >= 1 && EX % 4 == 0 && EY % ROWS == 0 && ROWS % 2 == 0, "4 x ROWS blocks");
@@ -379,6 +449,26 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const PF& dbuf, const unsigned
     const int base = (gx0 + gy0) & 1;  // colour of the k = 0 cells (1 = red, (x + y) odd)
     const bool owned = active && bx >= H / 4 && bx < (H + TXo) / 4 && by >= H / ROWS && by < (H + TYo) / ROWS;
     const int x0 = 4 * bx, y0 = ROWS * by;
+    // The words of this thread's block in its owner's part of an exchange: pair pi of corrections, or cell q of p, at
+    // [k][block], k = pi or q.  part: this CTA's; null: the block is outside, or its tile takes no part.
+    constexpr int NBLK = (TXo / 4) * (TYo / ROWS), XP = NC * NBLK;
+    ulonglong2* part_of = nullptr;
+    {
+        const int gx = gx0 + x0, gy = gy0 + y0;
+        const int tx = gx / TXo, ty = gy / TYo, t = ty * P.tiles_x + tx;
+        if (active && gx >= 0 && gy >= 0 && tx < P.tiles_x && t < P.ntiles) {
+            int lo = 0, hi = (int)nblocks;  // the tile's place among the first nblocks of the list (ascending)
+            while (lo < hi) {
+                const int m = (lo + hi) / 2;
+                if (list[m] < t) lo = m + 1;
+                else hi = m;
+            }
+            if (lo < (int)nblocks && list[lo] == t)
+                part_of = P.xch + OCT_XCH_SUMS + (size_t)lo * (2 * XP) + (gy - ty * TYo) / ROWS * (TXo / 4) + (gx - tx * TXo) / 4;
+        }
+    }
+    for (int i = threadIdx.x; i < 2 * XP; i += NT) P.xch[OCT_XCH_SUMS + (size_t)rank * (2 * XP) + i] = make_ulonglong2(0, 0);
+    if (threadIdx.x < 4) P.xch[((threadIdx.x >> 1) * OCT_MAX_TILES + rank) * 2 + (threadIdx.x & 1)] = make_ulonglong2(0, 0);
     // FP64 plane index of the cell (x0 + i, y0 + j), i in -1 .. 4 and j in -1 .. ROWS (constants once unrolled)
     const int pbase = y0 * Tile::RS + bx;
     auto pix = [&](int i, int j) { return pbase + j * Tile::RS + (i & 3) * W4 + (i >> 2); };
@@ -563,13 +653,20 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const PF& dbuf, const unsigned
     const std::integral_constant<int, 0> c0{};
     const std::integral_constant<int, 1> c1{};
 
-    unsigned iters = 0, xch = 0;
+    __shared__ double s_rel;
+    unsigned iters = 0, seq = 0, checks = 0;  // exchanges and checks so far: their tags
     double2 part = check();
     if (threadIdx.x == 0) P.partials[rank] = part;
     bool ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
     double r = ok ? ps_total_relative(P.partials, nblocks) : 0.0;
     const double r0v = r;
     bool pending = false;  // a check's total, read at the next block's first exchange
+    auto total = [&]() {
+        double rel;
+        const bool got = oct_total_relative(P.xch, checks, (int)nblocks, P.barrier, P.spin_limit, &rel);
+        if (threadIdx.x == 0) s_rel = rel;
+        return got;
+    };
     while (ok && (pending || (!(r <= P.tol) && iters < P.max_iters))) {
         unsigned todo = min(P.check_interval, P.max_iters - iters);
         unsigned done = 0;
@@ -590,83 +687,98 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const PF& dbuf, const unsigned
             }
             todo -= kk;
             done += kk;
-            if (todo > 0) {  // exchange the correction's halo through L2, alternating planes
-                const PF& db = (xch++ & 1) ? P.dbuf2 : dbuf;
+            if (todo > 0) {  // exchange the correction's halo
+                ++seq;
+                ulonglong2* const at = part_of + (seq & 1) * XP;
+                bool got = true;
                 if (owned) {
 #pragma unroll
-                    for (int q = 0; q < NC; ++q)
-                        if ((fl >> (48 + q)) & 1ull)
-                            __stcg(&db.p[(size_t)(gy0 + y0 + (q >> 2)) * db.P + gx0 + x0 + (q & 3)],
-                                   x2_lane(dv[oct_pair(q)], oct_lane(q)));
+                    for (int i = 0; i < NPAIR; ++i)
+                        xch_store(at + i * NBLK, __float_as_uint(x2_lane(dv[i], 0)), __float_as_uint(x2_lane(dv[i], 1)),
+                                  seq);
                 }
-                ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
+                if (pending && threadIdx.x < 32) got = total();
+                if (active && !owned) {
+                    ulonglong2 w[NPAIR];
+                    const bool from = part_of != nullptr;
+                    if (from) got = xch_poll(at, NBLK, seq, w, P.barrier, P.spin_limit) && got;
+#pragma unroll
+                    for (int j = 0; j < ROWS; ++j)
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            // an update cell's correction; every other cell's is 0 (its tile may not take part)
+                            const int pi = 2 * j + k, qa = 4 * j + ((k + j) & 1);
+                            const float a = from && ((upd_halo >> qa) & 1u) ? __uint_as_float((uint32_t)w[pi].x) : 0.0f;
+                            const float b =
+                                from && ((upd_halo >> (qa + 2)) & 1u) ? __uint_as_float((uint32_t)w[pi].y) : 0.0f;
+                            dv[pi] = x2_pack(a, b);
+                            *reinterpret_cast<f32x2*>(&T.d[k][y0 + j][2 * bx]) = dv[pi];
+                        }
+                }
+                ok = __syncthreads_and(got);
                 if (!ok) break;
                 if (pending) {
                     pending = false;
-                    r = ps_total_relative(P.partials, nblocks);
+                    r = s_rel;
                     if (r <= P.tol) {
                         converged = true;
                         break;
                     }
                 }
-                if (active && !owned) {
-                    float hv[NC];
-#pragma unroll
-                    for (int q = 0; q < NC; ++q) {
-                        const int gx = gx0 + x0 + (q & 3), gy = gy0 + y0 + (q >> 2);
-                        // an update cell's correction; every other cell's is 0 (its tile may not take part)
-                        hv[q] = (upd_halo >> q) & 1u ? __ldcg(&db.p[(size_t)gy * db.P + gx]) : 0.0f;
-                    }
-#pragma unroll
-                    for (int j = 0; j < ROWS; ++j)
-#pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            const int qa = 4 * j + ((k + j) & 1);
-                            dv[2 * j + k] = x2_pack(hv[qa], hv[qa + 2]);
-                            *reinterpret_cast<f32x2*>(&T.d[k][y0 + j][2 * bx]) = dv[2 * j + k];
-                        }
-                }
-                __syncthreads();
             }
         }
         if (!ok || converged) break;
         iters += done;
         // p += d on the owned cells (0 where the reference zeroes p), then exchange p.
+        ++seq;
+        ulonglong2* const at = part_of + (seq & 1) * XP;
+        bool got = true;
         if (owned) {
 #pragma unroll
             for (int q = 0; q < NC; ++q) {
-                if ((fl >> (48 + q)) & 1ull) {
-                    const int lx = x0 + (q & 3), ly = y0 + (q >> 2);
-                    const double pv =
-                        ((fl >> q) & 1ull) ? T.p[pix(q & 3, q >> 2)] + (double)x2_lane(dv[oct_pair(q)], oct_lane(q)) : 0.0;
-                    T.p[pix(q & 3, q >> 2)] = pv;
-                    __stcg(&L.x.p[(size_t)(gy0 + ly) * L.x.P + gx0 + lx], pv);
+                double pv = 0.0;
+                if ((fl >> q) & (fl >> (48 + q)) & 1ull)
+                    pv = T.p[pix(q & 3, q >> 2)] + (double)x2_lane(dv[oct_pair(q)], oct_lane(q));
+                T.p[pix(q & 3, q >> 2)] = pv;
+                xch_store(at + q * NBLK, pv, seq);
+            }
+        } else if (active) {
+            constexpr int PART = NC / 2;  // cells polled together
+#pragma unroll
+            for (int q0 = 0; q0 < NC; q0 += PART) {
+                ulonglong2 w[PART];
+                const bool from = part_of != nullptr;
+                if (from) got = xch_poll(at + q0 * NBLK, NBLK, seq, w, P.barrier, P.spin_limit) && got;
+#pragma unroll
+                for (int k = 0; k < PART; ++k) {
+                    const int q = q0 + k;
+                    T.p[pix(q & 3, q >> 2)] = from && ((upd_halo >> q) & 1u) ? xch_double(w[k]) : 0.0;
                 }
             }
         }
-        ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
+        ok = __syncthreads_and(got);
         if (!ok) break;
-        if (active && !owned) {
-            double hp[NC];
-#pragma unroll
-            for (int q = 0; q < NC; ++q) {
-                const int gx = gx0 + x0 + (q & 3), gy = gy0 + y0 + (q >> 2);
-                hp[q] = (upd_halo >> q) & 1u ? __ldcg(&L.x.p[(size_t)gy * L.x.P + gx]) : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < NC; ++q) T.p[pix(q & 3, q >> 2)] = hp[q];
-        }
-        __syncthreads();
         part = check();
-        if (threadIdx.x == 0) P.partials[rank] = part;
+        ++checks;
+        if (threadIdx.x == 0) {
+            ulonglong2* const sum = P.xch + ((checks & 1) * OCT_MAX_TILES + rank) * 2;
+            xch_store(sum, part.x, checks);
+            xch_store(sum + 1, part.y, checks);
+        }
         if (min(P.check_interval, P.max_iters - iters) > (unsigned)KMAX) {
             pending = true;
         } else {
-            ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
+            ok = __syncthreads_and(threadIdx.x < 32 ? total() : true);
             if (!ok) break;
-            r = ps_total_relative(P.partials, nblocks);
+            r = s_rel;
+            __syncthreads();  // before the next total
         }
     }
+    if (ok && iters > 0 && owned)
+#pragma unroll
+        for (int q = 0; q < NC; ++q)
+            if ((fl >> (48 + q)) & 1ull)
+                L.x.at(gx0 + x0 + (q & 3), gy0 + y0 + (q >> 2)) = T.p[pix(q & 3, q >> 2)];
     if (ok && iters > 0)  // the tiles that took no part: p = 0, as on every cell that is not updated
         for (int q = (int)(nblocks + rank); q < P.ntiles; q += (int)nblocks) {
             const int ox = (list[q] % P.tiles_x) * TXo, oy = (list[q] / P.tiles_x) * TYo;
@@ -686,7 +798,7 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const PF& dbuf, const unsigned
 }
 
 template <int EX, int EY, int KMAX, int NT, int ROWS>
-__global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf) {
+__global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P) {
     __shared__ unsigned short list[OCT_MAX_TILES];
     __shared__ int n;
     if (P.retry && P.result->error != 2) return;  // the launch before this one solved it
@@ -695,7 +807,7 @@ __global__ void __launch_bounds__(NT, 1) k_gsmix_oct(PersistentParams P, PF dbuf
         if (blockIdx.x == 0 && threadIdx.x == 0) *P.result = SolveResult{0, n == 0 ? 1 : 0, n ? 2 : 0, 0, 0.0, 0.0};
         return;
     }
-    if ((int)blockIdx.x < n) oct_solve<EX, EY, KMAX, NT, ROWS>(P, dbuf, list, blockIdx.x, (unsigned)n);
+    if ((int)blockIdx.x < n) oct_solve<EX, EY, KMAX, NT, ROWS>(P, list, blockIdx.x, (unsigned)n);
 }
 
 // The reference's fixed-count f32 sweeps (gauss_seidel.wgsl:12-88, `iters`
@@ -1307,16 +1419,28 @@ inline std::vector<PersistentPlan> plan_oct(const SolverWorkspace& ws, int nx, i
         return p.tiles_x * p.tiles_y <= ws.num_sms;
     };
     if (add(try_plan_oct<OCT_SMALL>) ||             // 32 x 32 owned, 8 iterations between exchanges
-        add(try_plan_oct<96, 64, 8, 384, 4>) ||     // 64 x 32, 8
+        add(try_plan_oct<OCT_MEDIUM>) ||            // 64 x 32, 4
         add(try_plan_oct<80, 72, 4, 384, 4>)) {}    // 64 x 56, 4 (1.70 us per iteration)
     return v;
 }
 
-// Tolerance-driven solve, one cooperative launch.  dbuf: an f32 plane of the
-// level's extent for the correction's halo exchange.  EFL_ERR_STATE: the grid
+// The exchanges' words for the largest of the plans (never inside a capture: the solve ends in a synchronisation).
+inline bool oct_reserve(SolverWorkspace& ws, size_t bytes) {
+    if (ws.xch_bytes >= bytes) return true;
+    cudaFree(ws.xch);
+    ws.xch = nullptr;
+    ws.xch_bytes = 0;
+    if (cudaMalloc(&ws.xch, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    ws.xch_bytes = bytes;
+    return true;
+}
+
+// Tolerance-driven solve, one cooperative launch.  EFL_ERR_STATE: the grid
 // does not fit the persistent scheme.
-inline efl_status solve_gsmix_persistent(SolverWorkspace& ws, const Level64& L, const PF& dbuf, const PF& dbuf2,
-                                         const Uniform& U,
+inline efl_status solve_gsmix_persistent(SolverWorkspace& ws, const Level64& L, const Uniform& U,
                                          float weight, double tol, uint32_t max_iters, uint32_t check_interval,
                                          cudaStream_t stream, SolveResult* out, std::string* err) {
     const std::vector<PersistentPlan> plans = plan_oct(ws, L.nx, L.ny);
@@ -1334,7 +1458,14 @@ inline efl_status solve_gsmix_persistent(SolverWorkspace& ws, const Level64& L, 
     P.barrier = ws.barrier;
     P.result = ws.result;
     P.spin_limit = ws.spin_limit > 0 ? ws.spin_limit : kBarrierSpinLimit;
-    P.dbuf2 = dbuf2;
+    size_t bytes = 0;
+    for (const PersistentPlan& plan : plans)
+        bytes = std::max(bytes, oct_xch_bytes(std::min(plan.tiles_x * plan.tiles_y, ws.num_sms), plan.tx * plan.ty));
+    if (!oct_reserve(ws, bytes)) {
+        *err = "out of device memory for the solve's exchanges";
+        return EFL_ERR_OUT_OF_MEMORY;
+    }
+    P.xch = ws.xch;
     P.one = 1.0f;
     P.wet = ws.wet;
     P.wet_w = (L.nx + 31) / 32;
@@ -1347,8 +1478,7 @@ inline efl_status solve_gsmix_persistent(SolverWorkspace& ws, const Level64& L, 
         P.tiles_x = plan.tiles_x;
         P.ntiles = plan.tiles_x * plan.tiles_y;
         P.retry = &plan != &plans[0];
-        PF db = dbuf;
-        void* args[] = {&P, &db};
+        void* args[] = {&P};
         count_launch();
         const cudaError_t e = cudaLaunchCooperativeKernel(plan.kernel, dim3(std::min(P.ntiles, ws.num_sms)),
                                                           dim3(plan.threads), args, plan.smem, stream);

@@ -153,3 +153,33 @@ def test_fixed_count_sweeps_on_both_tiles(oracle_api, gpu_api, nx, ny, iteration
         o.step(scenes.DT)
         g.step(scenes.DT)
     assert not compare_fields(g, o)
+
+
+@pytest.mark.parametrize("nx,ny,interval,limit", [(64, 32, 1, 7), (72, 40, 4, 40), (96, 96, 8, 37), (200, 136, 9, 100),
+                                                  (136, 264, 16, 64), (264, 72, 33, 200), (640, 512, 20, 45)])
+def test_exchanges_of_every_check_interval(oracle_api, gpu_api, nx, ny, interval, limit):
+    """The persistent solve's exchanges by tagged words: checks more often than exchanges, on them and between them, a
+    limit that cuts an interval short, one tile and many, and a second solve over the words of the first."""
+    sc = _splash(nx, ny)
+    sc.cfg.projection.tolerance = 1e-6
+    sc.cfg.projection.check_interval = interval
+    sc.cfg.projection.max_iterations = limit
+    o, g = make_pair(sc, oracle_api, gpu_api)
+    for _ in range(4):
+        so, sg = o.step(scenes.DT), g.step(scenes.DT)
+        assert (so.pressure_iterations, so.converged) == (sg.pressure_iterations, sg.converged)
+    assert not compare_fields(g, o)
+
+
+def test_exchanges_of_the_larger_tiles(oracle_api, gpu_api):
+    """More 32 x 32 tiles with water than the device holds: 64 x 32 tiles of 4 x 2 blocks, an exchange every 4."""
+    nx, ny = 704, 360
+    sc = _splash(nx, ny)
+    sc.oneshot = [scenes.aabb_source((0.0, 0.0), (0.5 * nx, 0.45 * ny))]
+    sc.cfg.projection.tolerance = 1e-6
+    sc.cfg.projection.max_iterations = 50
+    o, g = make_pair(sc, oracle_api, gpu_api)
+    for _ in range(3):
+        so, sg = o.step(scenes.DT), g.step(scenes.DT)
+        assert (so.pressure_iterations, so.converged) == (sg.pressure_iterations, sg.converged)
+    assert not compare_fields(g, o)
