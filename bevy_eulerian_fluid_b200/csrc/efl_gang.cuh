@@ -7,9 +7,9 @@
 // becomes idle, the largest simulation that fits the idle CTAs starts (a list in global memory behind a lock).  The
 // streamed form (efl_batch.cuh) runs every simulation in lockstep, each round reading every active tile from L2 behind
 // a barrier of the whole device: about 10 us per red-black iteration whatever the number of simulations left, against
-// 0.9 us here.  64 x 32 tiles because of the throughput per SM, 2190 cells per us (32 x 32: 1380; 64 x 56: 2108, but
-// 1.7 us per iteration and coarser tiles).  A step of 32 pools of 128^2 to 768^2: 91 ms; with an exchange every 8
-// iterations instead of 4, by 4 x 4 blocks that spill, 134 ms.
+// 0.9 us here.  64 x 32 tiles because of the throughput per SM, 2270 cells per us (32 x 32: 1480; 64 x 56: 2200, but
+// 1.6 us per iteration and coarser tiles).  A step of 32 pools of 128^2 to 768^2: 78 ms (91 before the checks shared an
+// exchange; then 134 with an exchange every 8 iterations instead of 4, by 4 x 4 blocks that spill).
 //
 // Each simulation's iterates and iteration count are those of its own solve.  Every wait is bounded.
 #pragma once

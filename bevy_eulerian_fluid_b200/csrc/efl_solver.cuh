@@ -318,7 +318,7 @@ EFL_DEV constexpr int oct_lane(int q) { return (q & 3) >> 1; }
 // Exchanges between the CTAs of a solve: words of 32 bits of data under a 32-bit tag, written and polled as 64-bit
 // relaxed accesses, which are indivisible.  The receiver waits for the tag of the exchange on the data itself, so an
 // exchange costs a store and a load of L2 and no fence, no flag and no barrier (a grid barrier and the loads behind it
-// took 3 us of every 8 iterations: 0.94 us per iteration on a 512^2 pool).  Tags only grow within a solve and the
+// took 3 us of every 8 iterations: 0.94 us per iteration on a 512^2 pool; 0.69 now, 0.38 of them half-sweeps).  Tags only grow within a solve and the
 // words are cleared before its first barrier; two buffers alternate, which suffices because every CTA waits in each
 // exchange for all the CTAs that read its words.
 EFL_DEV void xch_store(ulonglong2* p, uint32_t a, uint32_t b, uint32_t tag) {
@@ -362,33 +362,41 @@ EFL_DEV void xch_store(ulonglong2* p, double v, uint32_t tag) {
 constexpr int OCT_MAX_TILES = 1024;
 constexpr size_t OCT_XCH_SUMS = 2 * 2 * OCT_MAX_TILES;  // the residual sums of every CTA, then its cells
 // Bytes of the exchanges of `ctas` CTAs that own `cells` cells each.
-inline size_t oct_xch_bytes(int ctas, int cells) { return (OCT_XCH_SUMS + 2 * (size_t)ctas * cells) * sizeof(ulonglong2); }
-// ps_total_relative of the sums of check `tag`, in the first warp (every lane); false: a wait ran out.
-EFL_DEV bool oct_total_relative(const ulonglong2* sums, uint32_t tag, int nblocks, GridBarrier* gb, long long limit,
-                                double* rel) {
-    double r = 0.0, b = 0.0;
+inline size_t oct_xch_bytes(int ctas, int cells) { return (OCT_XCH_SUMS + (size_t)ctas * cells) * sizeof(ulonglong2); }
+constexpr int OCT_MAX_CTAS = 512;  // of one solve
+// The sums of check `tag`: fetched by the CTA's first threads, ...
+template <int NT>
+EFL_DEV bool oct_fetch_sums(const ulonglong2* sums, uint32_t tag, int nblocks, GridBarrier* gb, long long limit,
+                            double2* s_sums) {
     bool got = true;
-    for (int i = threadIdx.x; i < nblocks && got; i += 32) {
+    for (int i = threadIdx.x; i < nblocks; i += NT) {
         ulonglong2 w[2];
-        got = xch_poll(sums + ((tag & 1) * OCT_MAX_TILES + i) * 2, 1, tag, w, gb, limit);
-        r += xch_double(w[0]);
-        b += xch_double(w[1]);
+        got = xch_poll(sums + ((tag & 1) * OCT_MAX_TILES + i) * 2, 1, tag, w, gb, limit) && got;
+        s_sums[i] = make_double2(xch_double(w[0]), xch_double(w[1]));
+    }
+    return got;
+}
+// ... and after a barrier added by every warp, in ps_total_relative's order.
+EFL_DEV double oct_total_relative(const double2* s_sums, int nblocks) {
+    double r = 0.0, b = 0.0;
+    for (int i = threadIdx.x & 31; i < nblocks; i += 32) {
+        r += s_sums[i].x;
+        b += s_sums[i].y;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         r += __shfl_xor_sync(0xffffffffu, r, o);
         b += __shfl_xor_sync(0xffffffffu, b, o);
     }
-    *rel = b > 0.0 ? sqrt(r) / sqrt(b) : (r > 0.0 ? __longlong_as_double(0x7ff0000000000000ll) : 0.0);
-    return got;
+    return b > 0.0 ? sqrt(r) / sqrt(b) : (r > 0.0 ? __longlong_as_double(0x7ff0000000000000ll) : 0.0);
 }
 // The smallest tiles first: a CTA's sweeps cover its image, 64 x 64 cells here, and tiles without water need no CTA, so
-// 32 x 32 tiles fit the device up to 148 x 1024 cells of water.  0.74 us per red-black iteration on a 512^2 pool; the
-// same tile by 4 x 2 blocks of cells (512 threads) 0.79, exchanged every 6 iterations 0.86, every 4 iterations 0.91
-// (0.80 by 4 x 2 blocks), every 2 iterations 1.20.
+// 32 x 32 tiles fit the device up to 148 x 1024 cells of water.  0.69 us per red-black iteration on a 512^2 pool.
+// Before the checks shared its last exchange, 0.74; then the same tile by 4 x 2 blocks of cells (512 threads) took 0.79,
+// exchanged every 6 iterations 0.86, every 4 iterations 0.91 (0.80 by 4 x 2 blocks), every 2 iterations 1.20.
 #define OCT_SMALL 64, 64, 8, 256, 4
-// Twice the cells per CTA, by 4 x 2 blocks so that a thread's coefficients stay in its registers: 0.93 us on a full
-// 768 x 640 pool; by 4 x 4 blocks 1.00 (256 threads), and exchanged every 8 iterations 1.40 (384 threads, spilled).
+// Twice the cells per CTA, by 4 x 2 blocks so that a thread's coefficients stay in its registers: 0.90 us on a full
+// 768 x 640 pool; by 4 x 4 blocks 1.00 (256 threads) against 0.93 then, exchanged every 8 iterations 1.40 (spilled).
 #define OCT_MEDIUM 80, 48, 4, 480, 2
 template <int TX, int TY, int NT>
 EFL_DEV void oct_tiles(const PersistentParams& P, unsigned short* list, int* n) {
@@ -449,9 +457,9 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, un
     const int base = (gx0 + gy0) & 1;  // colour of the k = 0 cells (1 = red, (x + y) odd)
     const bool owned = active && bx >= H / 4 && bx < (H + TXo) / 4 && by >= H / ROWS && by < (H + TYo) / ROWS;
     const int x0 = 4 * bx, y0 = ROWS * by;
-    // The words of this thread's block in its owner's part of an exchange: pair pi of corrections, or cell q of p, at
-    // [k][block], k = pi or q.  part: this CTA's; null: the block is outside, or its tile takes no part.
-    constexpr int NBLK = (TXo / 4) * (TYo / ROWS), XP = NC * NBLK;
+    // The words of this thread's block in its owner's part of an exchange: pair pi of corrections at [pi][block].
+    // Null: the block is outside the domain, or its tile takes no part.
+    constexpr int NBLK = (TXo / 4) * (TYo / ROWS), XP = NPAIR * NBLK;
     ulonglong2* part_of = nullptr;
     {
         const int gx = gx0 + x0, gy = gy0 + y0;
@@ -596,25 +604,36 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, un
     auto check = [&]() -> double2 {
         double ar = 0.0, ab = 0.0;
         float frc[NC];
+        // A row's cells of p once for its four cells, under the row's branch (all rows at once, they spill).  Cells of
+        // the outermost ring, whose neighbours lie outside the image, are not counted.
+        const int left = x0 > 0 ? -1 : 0, right = x0 + 4 < EX ? 4 : 3;
 #pragma unroll
-        for (int q = 0; q < NC; ++q) {
-            const int i = oct_pair(q), ln = oct_lane(q);
-            float rcv = 0.0f;
-            if ((fl >> (32 + q)) & 1ull) {
-                const int ci = q & 3, cj = q >> 2;
-                double sum = (double)x2_lane(wl[i], ln) * T.p[pix(ci - 1, cj)];
-                sum = sum + (double)x2_lane(wr[i], ln) * T.p[pix(ci + 1, cj)];
-                sum = sum + (double)x2_lane(wu[i], ln) * T.p[pix(ci, cj - 1)];
-                sum = sum + (double)x2_lane(wd[i], ln) * T.p[pix(ci, cj + 1)];
-                const double bb = T.b[pix(ci, cj)];
-                const double r = bb - factor * (T.den[pix(ci, cj)] * T.p[pix(ci, cj)] - sum);
-                if ((fl >> q) & 1ull) rcv = (float)(cdiv * r);
-                if ((fl >> (48 + q)) & 1ull) {
+        for (int j = 0; j < ROWS; ++j) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) frc[4 * j + i] = 0.0f;
+            if (!((fl >> (32 + 4 * j)) & 15ull)) continue;
+            const int above = y0 + j > 0 ? j - 1 : j, below = y0 + j + 1 < EY ? j + 1 : j;
+            double row[6];
+            row[0] = T.p[pix(left, j)];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) row[1 + i] = T.p[pix(i, j)];
+            row[5] = T.p[pix(right, j)];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int q = 4 * j + i, pi = oct_pair(q), ln = oct_lane(q);
+                double sum = (double)x2_lane(wl[pi], ln) * row[i];
+                sum = sum + (double)x2_lane(wr[pi], ln) * row[i + 2];
+                sum = sum + (double)x2_lane(wu[pi], ln) * T.p[pix(i, above)];
+                sum = sum + (double)x2_lane(wd[pi], ln) * T.p[pix(i, below)];
+                const double bb = T.b[pix(i, j)];
+                const double r = bb - factor * (T.den[pix(i, j)] * row[i + 1] - sum);
+                const bool counted = (fl >> (32 + q)) & 1ull;
+                if (counted && ((fl >> q) & 1ull)) frc[q] = (float)(cdiv * r);
+                if (counted && ((fl >> (48 + q)) & 1ull)) {
                     ar += r * r;
                     ab += bb * bb;
                 }
             }
-            frc[q] = rcv;
         }
 #pragma unroll
         for (int j = 0; j < ROWS; ++j)
@@ -653,25 +672,23 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, un
     const std::integral_constant<int, 0> c0{};
     const std::integral_constant<int, 1> c1{};
 
-    __shared__ double s_rel;
+    __shared__ double2 s_sums[OCT_MAX_CTAS];
     unsigned iters = 0, seq = 0, checks = 0;  // exchanges and checks so far: their tags
     double2 part = check();
     if (threadIdx.x == 0) P.partials[rank] = part;
     bool ok = grid_barrier(P.barrier, nblocks, P.spin_limit);
     double r = ok ? ps_total_relative(P.partials, nblocks) : 0.0;
     const double r0v = r;
-    bool pending = false;  // a check's total, read at the next block's first exchange
-    auto total = [&]() {
-        double rel;
-        const bool got = oct_total_relative(P.xch, checks, (int)nblocks, P.barrier, P.spin_limit, &rel);
-        if (threadIdx.x == 0) s_rel = rel;
-        return got;
+    bool pending = false;  // a check's sums, read with the next exchange
+    unsigned checked = 0;  // iterations at the last check
+    auto fetch = [&]() {
+        return oct_fetch_sums<NT>(P.xch, checks, (int)nblocks, P.barrier, P.spin_limit, s_sums);
     };
     while (ok && (pending || (!(r <= P.tol) && iters < P.max_iters))) {
         unsigned todo = min(P.check_interval, P.max_iters - iters);
-        unsigned done = 0;
+        iters += todo;
         bool converged = false;
-        while (ok && todo > 0) {
+        while (todo > 0) {
             const unsigned kk = min((unsigned)KMAX, todo);
             for (unsigned it = 0; it < kk; ++it) {
                 if (bmax >= 1 + 2 * (int)it) {  // a cell of the block lies in the region still needed
@@ -686,92 +703,67 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, un
                 __syncthreads();
             }
             todo -= kk;
-            done += kk;
-            if (todo > 0) {  // exchange the correction's halo
-                ++seq;
-                ulonglong2* const at = part_of + (seq & 1) * XP;
-                bool got = true;
-                if (owned) {
+            // Exchange the correction's halo.
+            ++seq;
+            ulonglong2* const at = part_of + (seq & 1) * XP;
+            bool got = true;
+            if (owned) {
 #pragma unroll
-                    for (int i = 0; i < NPAIR; ++i)
-                        xch_store(at + i * NBLK, __float_as_uint(x2_lane(dv[i], 0)), __float_as_uint(x2_lane(dv[i], 1)),
-                                  seq);
-                }
-                if (pending && threadIdx.x < 32) got = total();
-                if (active && !owned) {
-                    ulonglong2 w[NPAIR];
-                    const bool from = part_of != nullptr;
-                    if (from) got = xch_poll(at, NBLK, seq, w, P.barrier, P.spin_limit) && got;
+                for (int i = 0; i < NPAIR; ++i)
+                    xch_store(at + i * NBLK, __float_as_uint(x2_lane(dv[i], 0)), __float_as_uint(x2_lane(dv[i], 1)), seq);
+            }
+            if (pending) got = fetch();
+            if (active && !owned) {
+                ulonglong2 w[NPAIR];
+                const bool from = part_of != nullptr;
+                if (from) got = xch_poll(at, NBLK, seq, w, P.barrier, P.spin_limit) && got;
 #pragma unroll
-                    for (int j = 0; j < ROWS; ++j)
+                for (int j = 0; j < ROWS; ++j)
 #pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            // an update cell's correction; every other cell's is 0 (its tile may not take part)
-                            const int pi = 2 * j + k, qa = 4 * j + ((k + j) & 1);
-                            const float a = from && ((upd_halo >> qa) & 1u) ? __uint_as_float((uint32_t)w[pi].x) : 0.0f;
-                            const float b =
-                                from && ((upd_halo >> (qa + 2)) & 1u) ? __uint_as_float((uint32_t)w[pi].y) : 0.0f;
-                            dv[pi] = x2_pack(a, b);
-                            *reinterpret_cast<f32x2*>(&T.d[k][y0 + j][2 * bx]) = dv[pi];
-                        }
-                }
-                ok = __syncthreads_and(got);
-                if (!ok) break;
-                if (pending) {
-                    pending = false;
-                    r = s_rel;
-                    if (r <= P.tol) {
-                        converged = true;
-                        break;
+                    for (int k = 0; k < 2; ++k) {
+                        // an update cell's correction; every other cell's is 0 (its tile may not take part)
+                        const int pi = 2 * j + k, qa = 4 * j + ((k + j) & 1);
+                        const float a = from && ((upd_halo >> qa) & 1u) ? __uint_as_float((uint32_t)w[pi].x) : 0.0f;
+                        const float b = from && ((upd_halo >> (qa + 2)) & 1u) ? __uint_as_float((uint32_t)w[pi].y) : 0.0f;
+                        dv[pi] = x2_pack(a, b);
+                        *reinterpret_cast<f32x2*>(&T.d[k][y0 + j][2 * bx]) = dv[pi];
                     }
+            }
+            ok = __syncthreads_and(got);
+            if (!ok) break;
+            if (pending) {
+                pending = false;
+                r = oct_total_relative(s_sums, (int)nblocks);
+                if (r <= P.tol) {
+                    converged = true;
+                    iters = checked;
+                    break;
                 }
             }
         }
         if (!ok || converged) break;
-        iters += done;
-        // p += d on the owned cells (0 where the reference zeroes p), then exchange p.
-        ++seq;
-        ulonglong2* const at = part_of + (seq & 1) * XP;
-        bool got = true;
-        if (owned) {
+        // p += d on every cell of the image (0 where the reference zeroes p): the halo's corrections are its owners'.
+        if (active) {
 #pragma unroll
-            for (int q = 0; q < NC; ++q) {
-                double pv = 0.0;
-                if ((fl >> q) & (fl >> (48 + q)) & 1ull)
-                    pv = T.p[pix(q & 3, q >> 2)] + (double)x2_lane(dv[oct_pair(q)], oct_lane(q));
-                T.p[pix(q & 3, q >> 2)] = pv;
-                xch_store(at + q * NBLK, pv, seq);
-            }
-        } else if (active) {
-            constexpr int PART = NC / 2;  // cells polled together
-#pragma unroll
-            for (int q0 = 0; q0 < NC; q0 += PART) {
-                ulonglong2 w[PART];
-                const bool from = part_of != nullptr;
-                if (from) got = xch_poll(at + q0 * NBLK, NBLK, seq, w, P.barrier, P.spin_limit) && got;
-#pragma unroll
-                for (int k = 0; k < PART; ++k) {
-                    const int q = q0 + k;
-                    T.p[pix(q & 3, q >> 2)] = from && ((upd_halo >> q) & 1u) ? xch_double(w[k]) : 0.0;
-                }
-            }
+            for (int q = 0; q < NC; ++q)
+                T.p[pix(q & 3, q >> 2)] =
+                    (upd_halo >> q) & 1u ? T.p[pix(q & 3, q >> 2)] + (double)x2_lane(dv[oct_pair(q)], oct_lane(q)) : 0.0;
         }
-        ok = __syncthreads_and(got);
-        if (!ok) break;
+        __syncthreads();
         part = check();
         ++checks;
+        checked = iters;
         if (threadIdx.x == 0) {
             ulonglong2* const sum = P.xch + ((checks & 1) * OCT_MAX_TILES + rank) * 2;
             xch_store(sum, part.x, checks);
             xch_store(sum + 1, part.y, checks);
         }
-        if (min(P.check_interval, P.max_iters - iters) > (unsigned)KMAX) {
+        if (iters < P.max_iters) {
             pending = true;
         } else {
-            ok = __syncthreads_and(threadIdx.x < 32 ? total() : true);
+            ok = __syncthreads_and(fetch());
             if (!ok) break;
-            r = s_rel;
-            __syncthreads();  // before the next total
+            r = oct_total_relative(s_sums, (int)nblocks);
         }
     }
     if (ok && iters > 0 && owned)
@@ -1407,7 +1399,7 @@ inline bool try_plan_oct(const SolverWorkspace& ws, int nx, int ny, PersistentPl
     p->kernel = (const void*)k_gsmix_oct<EX, EY, KMAX, NT, ROWS>;
     p->threads = NT;
     if (p->smem + 4096 > ws.max_smem) return false;
-    if ((int64_t)p->tiles_x * p->tiles_y > OCT_MAX_TILES) return false;
+    if ((int64_t)p->tiles_x * p->tiles_y > OCT_MAX_TILES || ws.num_sms > OCT_MAX_CTAS) return false;
     return p->ok = plan_resident<oct_kernel<EX, EY, KMAX, NT, ROWS>>(NT, p->smem);
 }
 inline std::vector<PersistentPlan> plan_oct(const SolverWorkspace& ws, int nx, int ny) {
@@ -1420,7 +1412,7 @@ inline std::vector<PersistentPlan> plan_oct(const SolverWorkspace& ws, int nx, i
     };
     if (add(try_plan_oct<OCT_SMALL>) ||             // 32 x 32 owned, 8 iterations between exchanges
         add(try_plan_oct<OCT_MEDIUM>) ||            // 64 x 32, 4
-        add(try_plan_oct<80, 72, 4, 384, 4>)) {}    // 64 x 56, 4 (1.70 us per iteration)
+        add(try_plan_oct<80, 72, 4, 384, 4>)) {}    // 64 x 56, 4 (1.63 us per iteration)
     return v;
 }
 
