@@ -19,7 +19,7 @@
 namespace efl {
 
 #define GANG_TILE OCT_MEDIUM
-constexpr int GANG_THREADS = 480, GANG_TX = 64, GANG_TY = 32;
+constexpr int GANG_THREADS = 480, GANG_TX = 64, GANG_TY = 32, GANG_K = 4;
 constexpr int GANG_MAX_SIMS = 512, GANG_MAX_CTAS = 512;
 
 struct GangSim {

@@ -2708,7 +2708,7 @@ efl_status efl_batch_tiles(const efl_batch* b, int32_t* tx, int32_t* ty, int32_t
     if (!c && b->ganged) {  // the gang solve's tiles
         if (tx) *tx = GANG_TX;
         if (ty) *ty = GANG_TY;
-        if (k) *k = 8;
+        if (k) *k = GANG_K;
     }
     if (ns_per_cell_iteration)
         for (int i = 0; i < kBatchConfigs; ++i)

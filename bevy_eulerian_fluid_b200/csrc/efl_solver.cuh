@@ -318,9 +318,9 @@ EFL_DEV constexpr int oct_lane(int q) { return (q & 3) >> 1; }
 // Exchanges between the CTAs of a solve: words of 32 bits of data under a 32-bit tag, written and polled as 64-bit
 // relaxed accesses, which are indivisible.  The receiver waits for the tag of the exchange on the data itself, so an
 // exchange costs a store and a load of L2 and no fence, no flag and no barrier (a grid barrier and the loads behind it
-// took 3 us of every 8 iterations: 0.94 us per iteration on a 512^2 pool; 0.69 now, 0.38 of them half-sweeps).  Tags only grow within a solve and the
-// words are cleared before its first barrier; two buffers alternate, which suffices because every CTA waits in each
-// exchange for all the CTAs that read its words.
+// took 3 us of every 8 iterations: 0.94 us per iteration on a 512^2 pool; 0.69 now, 0.38 of them half-sweeps).  Tags only
+// grow within a solve and the words are cleared before its first barrier; two buffers alternate, which suffices because
+// every CTA waits in each exchange for all the CTAs that read its words.
 EFL_DEV void xch_store(ulonglong2* p, uint32_t a, uint32_t b, uint32_t tag) {
     const unsigned long long t = (unsigned long long)tag << 32;
     asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | a), "l"(t | b) : "memory");

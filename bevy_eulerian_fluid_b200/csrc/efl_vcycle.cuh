@@ -18,9 +18,9 @@
 // and the diagonal is 4) skips the loads of its coefficients; 1 * x and x / 4 = x * 0.25 are exact.
 //
 // Latency bounds it: a half-sweep of a small level is one chain of dependent loads, sums and a division (250 cycles
-// in f64, 500 in f32) and a barrier (the cluster's: 500 cycles).  So the coefficients sit in registers for a level's
-// half-sweeps and the code of each step stands once.  Measured per call: 256^2 levels and below 80 us (f32) and 84
-// (f64), 62 and 66 with the geometry kept; the one-CTA form took 120 us from 128^2 down, after 25 to 97 us for the
+// in f64, 275 in f32) and a barrier (the cluster's: 500 cycles).  So the coefficients sit in registers for a level's
+// half-sweeps and the code of each step stands once.  Measured per call: 256^2 levels and below 74 us (f32) and 84
+// (f64), 58 and 66 with the geometry kept; the one-CTA form took 120 us from 128^2 down, after 25 to 97 us for the
 // 256^2 level's launches.
 #pragma once
 
