@@ -585,6 +585,141 @@ __global__ void k_gs_color(LevelT<T> L, float dx_scaled, float rho, float dt, fl
     L.x.at(x, y) = gs_update(L, gs_cdiv<T>(dx_scaled, rho, dt), (T)weight, x, y);
 }
 
+// n (1 or 2) red-black iterations of a V-cycle's smoother (weight 1) in one pass from L.x to `out`: gs_update on
+// 32 x 32 tiles with a halo of 4 cells, a thread per 2 x 2 block, its coefficients in registers and the image of x in
+// shared memory by colour.  Cells of the image's outermost ring update from clamped neighbours: what is wrong moves
+// inwards a ring per half-sweep and stays in the halo.  A launch per half-sweep read every plane and divided in every
+// cell each time: 149 us of a V-cycle on the levels 2048^2 to 512^2 in f64 (half of them water), 127 here (latency of
+// the first loads, two CTAs per SM); 46 and 27 us in f32 on 768 x 512 and 384 x 256.  wet (or null): tiles without water are skipped, zero in both planes already.
+constexpr int GT_E = 40, GT_H = 4, GT_O = GT_E - 2 * GT_H, GT_B = GT_E / 2, GT_NT = 416, GT_WP = 26;
+template <class T>
+__global__ void __launch_bounds__(GT_NT, 2) k_gs_tile(LevelT<T> L, Plane<T> out, float dx_scaled, float rho, float dt,
+                                                       int first, int n, const unsigned char* wet) {
+    static_assert(GT_B * GT_B <= GT_NT && GT_O == 32, "a thread per block; four 32 x 8 blocks of wet per tile");
+    __shared__ T xs[2][GT_E][GT_WP];  // [k][y][x / 2], k = (x + y) & 1 (1: red)
+    if (wet) {
+        const int w = (L.nx + 31) / 32, h = (L.ny + 7) / 8;
+        unsigned any = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int by = 4 * (int)blockIdx.y + j;
+            any |= by < h ? wet[by * w + blockIdx.x] : 0u;
+        }
+        if (!any) return;
+    }
+    const bool active = threadIdx.x < GT_B * GT_B;
+    const int bx = active ? (int)threadIdx.x % GT_B : 0, by = active ? (int)threadIdx.x / GT_B : 0;
+    const int gx0 = (int)blockIdx.x * GT_O - GT_H + 2 * bx, gy0 = (int)blockIdx.y * GT_O - GT_H + 2 * by;
+    // every load of the block first, at clamped places
+    float lv[4][4], fu[2][3], fv[3][2];
+    T pv[4], cb[4], inv[4];  // inv: 1 / denom in f64, denom in f32 (gs_update)
+    {
+        int xc[4], yc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            xc[i] = min(max(gx0 - 1 + i, 0), L.nx - 1);
+            yc[i] = min(max(gy0 - 1 + i, 0), L.ny - 1);
+        }
+        const int fx[3] = {xc[1], min(max(gx0 + 1, 0), L.nx), min(max(gx0 + 2, 0), L.nx)};
+        const int fy[3] = {yc[1], min(max(gy0 + 1, 0), L.ny), min(max(gy0 + 2, 0), L.ny)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i == 1 || i == 2 || j == 1 || j == 2) lv[j][i] = L.ls.at(xc[i], yc[j]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                pv[2 * j + i] = L.x.at(xc[1 + i], yc[1 + j]);
+                cb[2 * j + i] = L.b.at(xc[1 + i], yc[1 + j]);
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                fu[j][i] = L.fu.at(fx[i], yc[1 + j]);
+                fv[i][j] = L.fv.at(xc[1 + j], fy[i]);
+            }
+        }
+    }
+    const T c_div = gs_cdiv<T>(dx_scaled, rho, dt);
+    float w[4][4];
+    unsigned upd = 0, in = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int qx = q & 1, qy = q >> 1, gx = gx0 + qx, gy = gy0 + qy;
+        const float f[4] = {fu[qy][qx], fu[qy][qx + 1], fv[qy][qx], fv[qy + 1][qx]};
+        const float ln[4] = {lv[1 + qy][qx], lv[1 + qy][qx + 2], lv[qy][1 + qx], lv[qy + 2][1 + qx]};
+        const bool nb[4] = {gx > 0, gx + 1 < L.nx, gy > 0, gy + 1 < L.ny};
+        const float lij = lv[1 + qy][1 + qx];
+        T denom = T(0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[q][k] = 0.0f;
+        if (active && (unsigned)gx < (unsigned)L.nx && (unsigned)gy < (unsigned)L.ny) {
+            in |= 1u << q;
+            if (!(lij >= 0.0f) && !(f[0] == 0.0f && f[1] == 0.0f && f[2] == 0.0f && f[3] == 0.0f)) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (!nb[k]) continue;
+                    if (ln[k] < 0.0f) {
+                        denom += (T)f[k];
+                        w[q][k] = f[k];
+                    } else {
+                        denom += (T)f[k] * (T(1) - (T)ln[k] / (T)lij);
+                    }
+                }
+                if (!(fabs(denom) < (T)1.0e-6f)) upd |= 1u << q;
+            }
+        } else {
+            pv[q] = T(0);
+        }
+        const bool u = (upd >> q) & 1u;
+        cb[q] = u ? c_div * cb[q] : T(0);
+        inv[q] = u ? denom : T(1);
+        if constexpr (sizeof(T) == 8) inv[q] = T(1) / inv[q];
+        if (active) xs[(qx + qy) & 1][2 * by + qy][bx] = pv[q];
+    }
+    __syncthreads();
+    const int r0 = 2 * by, r1 = r0 + 1, up = max(r0 - 1, 0), dn = min(r1 + 1, GT_E - 1);
+    const int lf = max(bx - 1, 0), rt = min(bx + 1, GT_B - 1);
+    auto cell = [&](int q, T l, T r, T u, T d) {
+        T nume = cb[q];
+        nume = nume + (T)w[q][0] * l;
+        nume = nume + (T)w[q][1] * r;
+        nume = nume + (T)w[q][2] * u;
+        nume = nume + (T)w[q][3] * d;
+        const bool up_ = (upd >> q) & 1u;
+        T pn;
+        if constexpr (sizeof(T) == 8) pn = nume * inv[q];
+        else pn = div_zero(up_ ? nume : 1.0f, inv[q]);
+        pv[q] = up_ ? T(1) * pn + T(0) * pv[q] : T(0);
+    };
+    for (int h = 0; h < 2 * n; ++h) {
+        if ((first ^ h) & 1) {  // red: cells 1 and 2
+            const T r = xs[0][r0][rt], u = xs[0][up][bx], l = xs[0][r1][lf], d = xs[0][dn][bx];
+            cell(1, pv[0], r, u, pv[3]);
+            cell(2, l, pv[3], pv[0], d);
+            if (active) {
+                xs[1][r0][bx] = pv[1];
+                xs[1][r1][bx] = pv[2];
+            }
+        } else {  // black: cells 0 and 3
+            const T l = xs[1][r0][lf], u = xs[1][up][bx], r = xs[1][r1][rt], d = xs[1][dn][bx];
+            cell(0, l, pv[1], u, pv[2]);
+            cell(3, pv[2], r, pv[1], d);
+            if (active) {
+                xs[0][r0][bx] = pv[0];
+                xs[0][r1][bx] = pv[3];
+            }
+        }
+        __syncthreads();
+    }
+    constexpr int B0 = GT_H / 2, B1 = B0 + GT_O / 2;
+    if (!active || bx < B0 || bx >= B1 || by < B0 || by >= B1) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if ((in >> q) & 1u) out.at(gx0 + (q & 1), gy0 + (q >> 1)) = pv[q];
+}
+
 // projection/shaders/residual.wgsl:12-57
 template <class T>
 EFL_DEV T residual_factor(float dt, float rho, float dx_scaled) {

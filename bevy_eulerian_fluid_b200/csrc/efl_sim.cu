@@ -738,15 +738,31 @@ efl_status v_cycle(efl_sim* s, std::vector<LevelT<T>>& mg, size_t i, bool symmet
     const bool skip = geom == VC_GEOM_LOAD;
     const unsigned char *wet = skip ? wet_map(s, i) : nullptr, *wetc = skip ? wet_map(s, i + 1) : nullptr;
     if (i == mg.size() - 1) return gs_iterations(s, L, 1.0f, scale, P.mg_coarsest, false, wet);
-    TRY(gs_iterations(s, L, 1.0f, scale, P.mg_pre, false, wet));
+    // One or two iterations (the default) on each side: a pass from the iterate to the level's spare plane, the coarse
+    // correction there, and a pass back.
+    const bool tiles = P.mg_pre >= 1 && P.mg_pre <= 2 && P.mg_post >= 1 && P.mg_post <= 2;
+    auto pass = [&](const LevelT<T>& from, const Plane<T>& to, uint32_t n, bool black_first) -> efl_status {
+        const dim3 g((L.nx + GT_O - 1) / GT_O, (L.ny + GT_O - 1) / GT_O);
+        k_gs_tile<T><<<g, GT_NT, count_launch(), s->stream>>>(from, to, scale * s->U.dx, s->U.rho, s->U.dt,
+                                                              black_first ? 0 : 1, (int)n, wet);
+        LAUNCH_CHECK();
+        return EFL_OK;
+    };
+    LevelT<T> M = L;  // the level between the smoothings
+    if (tiles) {
+        std::swap(M.x, M.r);
+        TRY(pass(L, M.x, P.mg_pre, false));
+    } else {
+        TRY(gs_iterations(s, L, 1.0f, scale, P.mg_pre, false, wet));
+    }
     const LevelT<T>& C = mg[i + 1];
-    k_residual_restrict<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(L, C, s->U.dt, s->U.rho,
+    k_residual_restrict<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(M, C, s->U.dt, s->U.rho,
                                                                                           scale * s->U.dx, wetc);
     LAUNCH_CHECK();
     TRY(v_cycle(s, mg, i + 1, symmetric, geom));
-    k_prolongation<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(L, C, wetc);
+    k_prolongation<T><<<grid2d(C.nx, C.ny, kBlock), kBlock, count_launch(), s->stream>>>(M, C, wetc);
     LAUNCH_CHECK();
-    return gs_iterations(s, L, 1.0f, scale, P.mg_post, symmetric, wet);
+    return tiles ? pass(M, L.x, P.mg_post, symmetric) : gs_iterations(s, L, 1.0f, scale, P.mg_post, symmetric, wet);
 }
 
 // n reference (f32) red-black iterations on the pressure field: the TMA

@@ -183,3 +183,21 @@ def test_exchanges_of_the_larger_tiles(oracle_api, gpu_api):
         so, sg = o.step(scenes.DT), g.step(scenes.DT)
         assert (so.pressure_iterations, so.converged) == (sg.pressure_iterations, sg.converged)
     assert not compare_fields(g, o)
+
+
+@pytest.mark.parametrize("nx,ny,pre,post", [(328, 264, 2, 2), (264, 328, 1, 2), (1024, 72, 2, 1), (520, 136, 1, 1),
+                                            (328, 264, 3, 2), (328, 264, 2, 0), (768, 512, 2, 2)])
+@pytest.mark.parametrize("method,tolerance", [(capi.PROJECTION_MULTIGRID, 0.0), (capi.PROJECTION_MULTIGRID, 1e-3)])
+def test_smoothing_passes_bit_exact(oracle_api, gpu_api, nx, ny, pre, post, method, tolerance):
+    """A level's one or two smoothing iterations in one pass over 32 x 32 tiles with a halo of 4, in f32 and f64, and
+    the launches per half-sweep for other counts."""
+    sc = _splash(nx, ny)
+    sc.cfg.projection.method = method
+    sc.cfg.projection.tolerance = tolerance
+    sc.cfg.projection.mg_pre, sc.cfg.projection.mg_post = pre, post
+    sc.cfg.projection.max_iterations = 5
+    o, g = make_pair(sc, oracle_api, gpu_api)
+    for _ in range(3):
+        so, sg = o.step(scenes.DT), g.step(scenes.DT)
+        assert so.pressure_iterations == sg.pressure_iterations
+    assert not compare_fields(g, o)
