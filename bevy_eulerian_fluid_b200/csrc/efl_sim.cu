@@ -141,6 +141,7 @@ struct efl_sim {
     const float* tma_pre1_x = nullptr;  // level 1's iterate plane the maps were built over
     SweepTma tma_pre;    // TMA maps of the preconditioner's level 0 (error flag shared with tma)
     std::vector<unsigned char*> wet_lv;  // wet blocks of the levels above the cluster's (level 0: solver.wet)
+    size_t wet_levels = 0;               // the levels whose map is of the present solve (wet_update)
     int* wet_list[2] = {nullptr, nullptr};  // tiles of levels 0 and 1 for the TMA sweep, wet ones first
     int* wet_count = nullptr;               // their counts, 2 per level
     DevBuf vc_image[2];           // the coarse levels' geometry in a solve's V-cycles (f32, f64 levels); owned by bufs
@@ -605,9 +606,10 @@ efl_status relative_residual(efl_sim* s, const LevelT<T>& L0, double* rel) {
 }
 
 // What the solves skip: wet blocks (32 x 8 cells) of level 0 and of the first `levels` - 1 coarse ones, and the tile
-// lists of the TMA sweep on levels 0 and 1.  The buffers are made on first use, outside any stream capture.
+// lists of the TMA sweep on levels 0 and 1.  The buffers are made on first use, outside any stream capture.  A level
+// that the present solve has no map of (its buffer may hold another solve's) is not skipped: null.
 const unsigned char* wet_map(const efl_sim* s, size_t level) {
-    return level == 0 ? s->solver.wet : level <= s->wet_lv.size() ? s->wet_lv[level - 1] : nullptr;
+    return level >= s->wet_levels ? nullptr : level == 0 ? s->solver.wet : s->wet_lv[level - 1];
 }
 WetList wet_tiles_of(const efl_sim* s, int level, bool zero) {
     return s->wet_list[level] ? WetList{s->wet_list[level], s->wet_count + 2 * level, zero ? 1 : 0} : WetList{};
@@ -629,6 +631,7 @@ efl_status wet_alloc(efl_sim* s, size_t levels, bool lists) {
     return EFL_OK;
 }
 efl_status wet_update(efl_sim* s, size_t levels, bool lists) {
+    s->wet_levels = levels;
     k_wet_blocks<<<grid2d(s->nx, s->ny, kBlock), kBlock, count_launch(), s->stream>>>(s->ls0, s->solver.wet);
     auto w = [&](size_t l) { return ((s->nx >> l) + 31) / 32; };
     auto h = [&](size_t l) { return ((s->ny >> l) + 7) / 8; };

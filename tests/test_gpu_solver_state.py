@@ -1,0 +1,35 @@
+"""What one solve leaves on a simulation must not reach the next: maps of the water, exchange words, scheduler state."""
+import numpy as np
+import pytest
+
+from bevy_eulerian_fluid_b200 import _capi as capi
+from bevy_eulerian_fluid_b200 import scenes
+
+from .helpers import compare_fields, make_pair
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx,ny,pre", [(768, 80, 2), (768, 80, 3), (520, 120, 2), (2048, 32, 2), (768, 512, 2)])
+def test_water_moves_between_solves_of_two_methods(oracle_api, gpu_api, nx, ny, pre):
+    """MGPCG, then the water on the other side and iterated V-cycles on the same simulation.  The first three grids are
+    at most 256^2 cells and too wide for the V-cycle's cluster, so that their levels run as launches, which skip the
+    blocks without water; the V-cycles make a map of level 0 only there."""
+    cfg = scenes.base_config(nx, ny)
+    sc = scenes.Scene(f"left_{nx}x{ny}", cfg, oneshot=[scenes.aabb_source((-0.4 * nx, -0.2 * ny), (0.1 * nx, 0.3 * ny))])
+    P = cfg.projection
+    P.method, P.tolerance, P.max_iterations, P.mg_pre = capi.PROJECTION_MGPCG, 1e-5, 12, pre
+    o, g = make_pair(sc, oracle_api, gpu_api)
+    for _ in range(3):
+        so, sg = o.step(scenes.DT), g.step(scenes.DT)
+    assert not compare_fields(g, o)
+    for f in (capi.FIELD_LEVELSET_AIR, capi.FIELD_LEVELSET_AIR1):
+        mirrored = np.ascontiguousarray(o.get(f)[:, ::-1])
+        for s in (o, g):
+            s.set(f, mirrored)
+    P.method, P.tolerance = capi.PROJECTION_MULTIGRID, 1e-6
+    for s in (o, g):
+        s.set_projection(P)
+    so, sg = o.step(scenes.DT), g.step(scenes.DT)
+    assert (so.pressure_iterations, so.residual_initial) == (sg.pressure_iterations, sg.residual_initial)
+    assert not compare_fields(g, o)
