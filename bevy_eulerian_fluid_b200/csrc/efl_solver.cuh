@@ -32,25 +32,32 @@ namespace efl {
 struct GridBarrier {
     unsigned int count;
     unsigned int gen;  // unused (layout kept)
-    int error;
+    int error;  // the first wait that ran out: 1 a barrier, 2 an exchange (xch_poll)
     int pad;
 };
 
 struct SolveResult {
     unsigned int iterations;
     int converged;
-    int error;  // 1: a grid barrier timed out
+    int error;  // 1: a wait of the first CTA ran out, 2: more tiles with water than CTAs
     int pad;
     double r0, r1;  // relative residual before / after
+};
+// Read back together: any CTA's wait may run out, after the last exchange too, when the first CTA, which writes the
+// result, has what it waited for; only the barrier's flag says so then.
+struct SolveState {
+    SolveResult result;
+    GridBarrier barrier;
 };
 
 struct SolverWorkspace {
     int nx = 0, ny = 0, device = 0;
     int num_sms = 0;
     size_t max_smem = 0;
-    GridBarrier* barrier = nullptr;
-    SolveResult* result = nullptr;    // device
-    SolveResult* h_result = nullptr;  // pinned host
+    SolveState* state = nullptr;    // device
+    GridBarrier* barrier = nullptr;  // state's
+    SolveResult* result = nullptr;   // state's
+    SolveState* h_state = nullptr;  // pinned host
     double2* partials = nullptr;
     int max_blocks = 0;
     long long spin_limit = 0;  // grid-barrier polls before giving up (0: kBarrierSpinLimit)
@@ -178,23 +185,23 @@ inline efl_status solver_init(SolverWorkspace& ws, int nx, int ny, int device, s
     ws.num_sms = prop.multiProcessorCount;
     ws.max_smem = prop.sharedMemPerBlockOptin;
     ws.max_blocks = 4 * ws.num_sms;
-    if (cudaMalloc(&ws.barrier, sizeof(GridBarrier)) != cudaSuccess ||
-        cudaMalloc(&ws.result, sizeof(SolveResult)) != cudaSuccess ||
+    if (cudaMalloc(&ws.state, sizeof(SolveState)) != cudaSuccess ||
         cudaMalloc(&ws.partials, ws.max_blocks * sizeof(double2)) != cudaSuccess ||
         cudaMalloc(&ws.wet, (size_t)((nx + 31) / 32) * ((ny + 7) / 8)) != cudaSuccess ||
-        cudaMallocHost(&ws.h_result, sizeof(SolveResult)) != cudaSuccess) {
+        cudaMallocHost(&ws.h_state, sizeof(SolveState)) != cudaSuccess) {
         *err = "solver workspace allocation failed";
         return EFL_ERR_OUT_OF_MEMORY;
     }
+    ws.barrier = &ws.state->barrier;
+    ws.result = &ws.state->result;
     return EFL_OK;
 }
 inline void solver_free(SolverWorkspace& ws) {
-    if (ws.barrier) cudaFree(ws.barrier);
-    if (ws.result) cudaFree(ws.result);
+    if (ws.state) cudaFree(ws.state);
     if (ws.partials) cudaFree(ws.partials);
     if (ws.xch) cudaFree(ws.xch);
     if (ws.wet) cudaFree(ws.wet);
-    if (ws.h_result) cudaFreeHost(ws.h_result);
+    if (ws.h_state) cudaFreeHost(ws.h_state);
     ws = SolverWorkspace{};
 }
 
@@ -344,7 +351,7 @@ EFL_DEV bool xch_poll(const ulonglong2* p, int stride, uint32_t tag, ulonglong2 
             int e;
             asm volatile("ld.acquire.gpu.s32 %0, [%1];" : "=r"(e) : "l"(&gb->error) : "memory");
             if (e || spins >= limit) {
-                atomicExch(&gb->error, 1);
+                atomicCAS(&gb->error, 0, 2);
                 return false;
             }
         }
@@ -1479,15 +1486,16 @@ inline efl_status solve_gsmix_persistent(SolverWorkspace& ws, const Level64& L, 
             return EFL_ERR_CUDA;
         }
     }
-    if (cudaMemcpyAsync(ws.h_result, ws.result, sizeof(SolveResult), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+    if (cudaMemcpyAsync(ws.h_state, ws.state, sizeof(SolveState), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
         cudaStreamSynchronize(stream) != cudaSuccess) {
         *err = std::string("mixed solver failed: ") + cudaGetErrorString(cudaGetLastError());
         return EFL_ERR_CUDA;
     }
-    *out = *ws.h_result;
+    *out = ws.h_state->result;
+    const int waits = ws.h_state->barrier.error;
     if (out->error == 2) return EFL_ERR_STATE;  // more tiles with water than the device holds
-    if (out->error) {
-        *err = "mixed solver: a grid barrier timed out";
+    if (out->error || waits) {
+        *err = waits == 2 ? "mixed solver: a halo exchange timed out" : "mixed solver: a grid barrier timed out";
         return EFL_ERR_CUDA;
     }
     return EFL_OK;

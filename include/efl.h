@@ -339,9 +339,10 @@ EFL_API efl_status efl_residual(efl_sim* sim, double* relative, double* norm_r, 
  * counterpart (the reference records wgpu command buffers per frame). */
 EFL_API efl_status efl_set_graph_capture(efl_sim* sim, int32_t enable);
 /* Bounds of the device-side waits (extension, no reference counterpart).
- * barrier_polls: polls of the grid barrier inside the cooperative pressure
- * solves before a CTA gives up; every CTA then leaves the launch and the
- * step returns EFL_ERR_CUDA ("... a grid barrier timed out").
+ * barrier_polls: polls of a grid barrier, or of the words of a halo exchange,
+ * inside the cooperative pressure solves before a CTA gives up; every CTA
+ * then leaves the launch and the step returns EFL_ERR_CUDA ("... a grid
+ * barrier timed out" or "... a halo exchange timed out").
  * mbarrier_polls: polls of the TMA sweep's wait for a tile's copies; a CTA
  * that gives up waits (default bound) for its own copies still in flight and
  * leaves, and the next efl_synchronize / efl_read_solid_forces returns

@@ -33,3 +33,33 @@ def test_water_moves_between_solves_of_two_methods(oracle_api, gpu_api, nx, ny, 
     so, sg = o.step(scenes.DT), g.step(scenes.DT)
     assert (so.pressure_iterations, so.residual_initial) == (sg.pressure_iterations, sg.residual_initial)
     assert not compare_fields(g, o)
+
+
+def test_every_wait_that_runs_out_is_reported(gpu_api):
+    """The tolerance-driven solve with limits of a few polls: whichever CTA's wait runs out, in the first barrier, in an
+    exchange or in the last one, when the first CTA may be done already, the solve is an error that names the wait;
+    otherwise it is the whole solve.  Aborted solves leave nothing behind: the pressure of before, and exchange words
+    that the next solve clears."""
+    sc = scenes.coupled(256, tolerance=1e-5, n_per_shape=2)
+    sc.cfg.projection.max_iterations, sc.cfg.projection.check_interval = 24, 8
+    g = sc.make(gpu_api)
+    g.step(sc.dt)
+    for stage in range(capi.STAGE_UPDATE_SOLID, capi.STAGE_PROJECTION):
+        g.run_stage(stage, sc.dt)
+    before = g.get(capi.FIELD_PRESSURE)
+    st = g.run_stage(capi.STAGE_PROJECTION, sc.dt)
+    want = g.get(capi.FIELD_PRESSURE)
+    assert st.pressure_iterations == 24 and not np.array_equal(before, want)
+    for limit in [*range(1, 17), 0]:
+        for _ in range(6):
+            g.set(capi.FIELD_PRESSURE, before)
+            g.set_wait_limits(barrier_polls=limit)
+            try:
+                g.run_stage(capi.STAGE_PROJECTION, sc.dt)
+            except capi.EflError as e:
+                assert limit and e.status == capi.ERR_CUDA
+                assert str(e).endswith(("a grid barrier timed out", "a halo exchange timed out")), str(e)
+                assert np.array_equal(g.get(capi.FIELD_PRESSURE), before)
+            else:
+                assert np.array_equal(g.get(capi.FIELD_PRESSURE), want), limit
+    g.close()
