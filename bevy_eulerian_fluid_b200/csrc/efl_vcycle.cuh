@@ -345,21 +345,20 @@ __global__ void __launch_bounds__(VC_THREADS, 1) k_vcycle_cluster(const __grid_c
         const int fy0 = rows_from(F), fr = rows_of(F), cy0 = C.gathered && !F.gathered ? 0 : rows_from(C);
         const int Y0 = fy0 / 2, Y1 = min((fy0 + fr) / 2, C.ny);
         unsigned char* to = C.gathered && !F.gathered ? head : sm;
-        // Two lanes per coarse cell, one per row of its children; the first adds them up.
+        // Two lanes per coarse cell, one per row of its children; the first adds them up.  The two have the same q and j,
+        // so both come to each shuffle, which waits for them (the residuals branch per cell, and the other lanes of the
+        // warp may have fewer rows).
         const int sub = tid & 1, j0 = (tid >> 1) & ((1 << F.lc) - 1), step = max((NT / 2) >> F.lc, 1);
         const int rows = Y1 - Y0, q0 = (tid >> 1) >> F.lc, jstep = min(1 << F.lc, NT / 2);
+        const unsigned pair = 3u << (tid & 30);
 #pragma unroll 1
         for (int q = q0; q < rows; q += step)
 #pragma unroll 1
-            for (int j = j0 & (jstep - 1); j < (C.nx + 15) / 16 * 16; j += jstep) {  // whole warps
-                const bool in = j < C.nx;
-                T ra = T(0), rb = T(0);
-                if (in) {
-                    ra = residual(F, factor, fy0, 2 * q + sub, 2 * j);
-                    rb = residual(F, factor, fy0, 2 * q + sub, 2 * j + 1);
-                }
-                const T ra1 = __shfl_xor_sync(__activemask(), ra, 1), rb1 = __shfl_xor_sync(__activemask(), rb, 1);
-                if (in && sub == 0)
+            for (int j = j0 & (jstep - 1); j < C.nx; j += jstep) {
+                const T ra = residual(F, factor, fy0, 2 * q + sub, 2 * j);
+                const T rb = residual(F, factor, fy0, 2 * q + sub, 2 * j + 1);
+                const T ra1 = __shfl_xor_sync(pair, ra, 1), rb1 = __shfl_xor_sync(pair, rb, 1);
+                if (sub == 0)
                     B(to, C, (j + Y0 + q) & 1)[(Y0 + q - cy0) * C.HW + (j >> 1) + 1] = T(0.25) * (ra + ra1 + rb + rb1);
             }
     };
