@@ -11,7 +11,10 @@
 // 1.6 us per iteration and coarser tiles).  A step of 32 pools of 128^2 to 768^2: 78 ms (91 before the checks shared an
 // exchange; then 134 with an exchange every 8 iterations instead of 4, by 4 x 4 blocks that spill).
 //
-// Each simulation's iterates and iteration count are those of its own solve.  Every wait is bounded.
+// Each simulation's iterates and iteration count are those of its own solve.  Every wait is bounded: those of a gang
+// by polls, an idle CTA's (for its next gang, which may take other simulations' whole solves, or for the lock) by polls
+// in which no gang comes to its next residual check; gang_idle_limit gives a gang's own waits up to there time to run out
+// first.  (A report per exchange instead cost 0.6 % of a step.)
 #pragma once
 
 #include "efl_solver.cuh"
@@ -32,6 +35,7 @@ struct GangState {  // zeroed before each launch
     int started;    // simulations started or not schedulable
     int smallest;   // no simulation left has fewer tiles
     int error;      // a wait ran out
+    unsigned beat;  // grows with all progress: CTAs that become idle, simulations started, residual checks
     unsigned taken[GANG_MAX_SIMS / 32];
     int idle[GANG_MAX_CTAS];
     int2 mail[GANG_MAX_CTAS];  // (simulation + 1, rank) for a CTA; x = 0: none yet, -1: leave
@@ -43,6 +47,35 @@ EFL_DEV int gang_load(const int* p) {
     asm volatile("ld.acquire.gpu.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+
+// Polls between two checks `interval` iterations apart: the exchanges' and a check's at most `limit` each.
+inline long long gang_idle_limit(long long limit, unsigned interval) {
+    const long long waits = (long long)interval / GANG_K + 3;
+    return limit > (1ll << 62) / waits ? 1ll << 62 : limit * waits;
+}
+// A wait for other CTAs' progress: true while it may go on.
+struct GangWait {
+    volatile GangState* V;
+    long long limit, spins = 0;
+    unsigned seen;
+    EFL_DEV GangWait(GangState* G, long long lim) : V(G), limit(lim), seen(V->beat) {}
+    EFL_DEV bool poll() {
+        if ((++spins & 1023) != 0 && spins < limit) return true;
+        if (V->error) return false;
+        const unsigned now = V->beat;
+        if (now == seen) return spins < limit;
+        seen = now;
+        spins = 0;
+        return true;
+    }
+};
+// oct_solve's report of a residual check.
+struct GangBeat {
+    GangState* G;
+    EFL_DEV void operator()(unsigned rank) const {
+        if (rank == 0) atomicAdd(&G->beat, 1u);
+    }
+};
 
 // Starts simulations while one fits the idle CTAs; lets the idle CTAs go when none is left.  Under the lock.
 EFL_DEV void gang_schedule(GangState* G, int ns) {
@@ -65,6 +98,7 @@ EFL_DEV void gang_schedule(GangState* G, int ns) {
         V->taken[best >> 5] = V->taken[best >> 5] | (1u << (best & 31));
         __threadfence();
         ++started;
+        atomicAdd(&G->beat, 1u);
         for (int r = 0; r < bn; ++r) {
             const int c = V->idle[--nidle];
             V->mail[c].y = r;
@@ -82,35 +116,25 @@ EFL_DEV void gang_schedule(GangState* G, int ns) {
 // The calling CTA (its first thread) joins the idle ones and waits for its next gang: (simulation, rank), or x < 0.
 EFL_DEV int2 gang_next(GangState* G, int ns, bool first, long long limit) {
     volatile GangState* V = G;
-    long long spins = 0;
-    while (atomicCAS(&G->lock, 0u, 1u) != 0u)
-        if (++spins >= limit || ((spins & 1023) == 0 && V->error)) {
+    for (GangWait w(G, limit); atomicCAS(&G->lock, 0u, 1u) != 0u;)
+        if (!w.poll()) {
             atomicExch(&G->error, 1);
             return make_int2(-1, 0);
         }
     __threadfence();
+    atomicAdd(&G->beat, 1u);
     V->idle[V->nidle] = (int)blockIdx.x;
     V->nidle = V->nidle + 1;
     if (first) V->arrived = V->arrived + 1;
     if (V->arrived == (int)gridDim.x) gang_schedule(G, ns);  // every simulation's tile count is known from here on
     __threadfence();
     atomicExch(&G->lock, 0u);
-    int seen = V->started, sim = 0;
-    spins = 0;
-    while ((sim = gang_load(&G->mail[blockIdx.x].x)) == 0) {
-        ++spins;
-        if ((spins & 1023) == 0 || spins >= limit) {
-            const int now = V->started;  // progress elsewhere: not stalled
-            if (now != seen && spins < limit) {
-                seen = now;
-                spins = 0;
-            } else if (V->error || spins >= limit) {
-                atomicExch(&G->error, 1);
-                return make_int2(-1, 0);
-            }
+    int sim = 0;
+    for (GangWait w(G, limit); (sim = gang_load(&G->mail[blockIdx.x].x)) == 0; __nanosleep(100))
+        if (!w.poll()) {
+            atomicExch(&G->error, 1);
+            return make_int2(-1, 0);
         }
-        __nanosleep(100);
-    }
     const int rank = V->mail[blockIdx.x].y;
     V->mail[blockIdx.x].x = 0;
     return make_int2(sim > 0 ? sim - 1 : -1, rank);
@@ -154,7 +178,7 @@ __global__ void __launch_bounds__(GANG_THREADS, 1) k_batch_gang(const GangSim* s
         const int2 j = job;
         if (j.x < 0) return;
         load(j.x);
-        if (!oct_solve<GANG_TILE>(S.P, list, (unsigned)j.y, (unsigned)n)) {
+        if (!oct_solve<GANG_TILE>(S.P, list, (unsigned)j.y, (unsigned)n, GangBeat{G})) {
             if (threadIdx.x == 0) atomicExch(&G->error, 1);
             return;
         }

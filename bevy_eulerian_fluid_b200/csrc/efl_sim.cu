@@ -2422,6 +2422,7 @@ efl_status gang_solve(efl_batch* b, const std::vector<int>& which, efl_step_stat
     for (size_t at = 0; at < which.size();) {
         std::vector<GangSim> hs;
         std::vector<int> ids;
+        unsigned interval = 1;  // the longest between two residual checks
         for (; at < which.size() && ids.size() < GANG_MAX_SIMS; ++at) {
             efl_sim* s = b->sims[which[at]];
             GangSim S{};
@@ -2449,6 +2450,7 @@ efl_status gang_solve(efl_batch* b, const std::vector<int>& which, efl_step_stat
             P.one = 1.0f;
             P.wet = s->solver.wet;
             P.wet_w = (s->nx + 31) / 32;
+            interval = std::max(interval, std::min(P.check_interval, P.max_iters));
             hs.push_back(S);
             ids.push_back(which[at]);
         }
@@ -2458,7 +2460,7 @@ efl_status gang_solve(efl_batch* b, const std::vector<int>& which, efl_step_stat
             cudaMemsetAsync(b->d_gang_barrier, 0, ns * sizeof(GridBarrier), st) != cudaSuccess ||
             cudaMemsetAsync(b->d_gang_state, 0, sizeof(GangState), st) != cudaSuccess)
             return batch_err(b, EFL_ERR_CUDA, "batch upload failed");
-        long long limit = b->spin_limit > 0 ? b->spin_limit : kBarrierSpinLimit;
+        long long limit = gang_idle_limit(b->spin_limit > 0 ? b->spin_limit : kBarrierSpinLimit, interval);
         const GangSim* dg = b->d_gang;
         GangState* gs = b->d_gang_state;
         void* args[] = {&dg, &ns, &gs, &limit};

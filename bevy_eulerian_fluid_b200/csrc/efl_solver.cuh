@@ -443,9 +443,13 @@ EFL_DEV void oct_tiles(const PersistentParams& P, unsigned short* list, int* n) 
 
 // One simulation's solve by `nblocks` CTAs, this one being number `rank` of them and owning tile list[rank] (the
 // simulation's active tiles: a tile without a cell of level set < 0 takes no part, as its correction is 0 and no
-// weight points at its cells).  False: a grid barrier timed out.
-template <int EX, int EY, int KMAX, int NT, int ROWS>
-EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, unsigned rank, unsigned nblocks) {
+// weight points at its cells).  beat(rank) at each check, from the CTA's first thread.  False: a wait ran out.
+struct OctNoBeat {
+    EFL_DEV void operator()(unsigned) const {}
+};
+template <int EX, int EY, int KMAX, int NT, int ROWS, class Beat = OctNoBeat>
+EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, unsigned rank, unsigned nblocks,
+                       Beat beat = Beat()) {
     using Tile = OctTile<EX, EY, ROWS>;
     constexpr int NC = 4 * ROWS, NPAIR = 2 * ROWS;
     static_assert(KMAX >= 1 && EX % 4 == 0 && EY % ROWS == 0 && ROWS % 2 == 0, "4 x ROWS blocks");
@@ -764,6 +768,7 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, un
             ulonglong2* const sum = P.xch + ((checks & 1) * OCT_MAX_TILES + rank) * 2;
             xch_store(sum, part.x, checks);
             xch_store(sum + 1, part.y, checks);
+            beat(rank);
         }
         if (iters < P.max_iters) {
             pending = true;

@@ -468,10 +468,12 @@ EFL_API efl_status efl_batch_set_tiles(efl_batch* batch, int32_t config);
  * alone; 0, 0, 0 while tuning) and the measured cost of each (ns_per_cell_iteration: 4 entries or NULL; 0 = not tried). */
 EFL_API efl_status efl_batch_tiles(const efl_batch* batch, int32_t* tx, int32_t* ty, int32_t* k,
                                    double* ns_per_cell_iteration);
-/* Grid-barrier poll limit of the batched solve (efl_set_wait_limits'
- * barrier_polls; 0 = the default).  A barrier that runs out makes
- * efl_batch_step return EFL_ERR_CUDA ("batched solver: a grid barrier timed
- * out"). */
+/* Poll limit of the batched solve's waits (efl_set_wait_limits'
+ * barrier_polls; 0 = the default): of each barrier and halo exchange.  A CTA
+ * without a simulation gives up after as many polls as those of one check
+ * interval add up to in which no simulation comes to a residual check.  A
+ * wait that runs out makes efl_batch_step return EFL_ERR_CUDA ("batched
+ * solver: a grid barrier timed out"). */
 EFL_API efl_status efl_batch_set_wait_limits(efl_batch* batch, uint64_t barrier_polls);
 /* Device time of the last batched pressure solve (the cooperative launch), in
  * milliseconds; waits for it to finish. */

@@ -63,3 +63,25 @@ def test_every_wait_that_runs_out_is_reported(gpu_api):
             else:
                 assert np.array_equal(g.get(capi.FIELD_PRESSURE), want), limit
     g.close()
+
+
+def test_batch_waits_as_long_as_a_gang_makes_progress(gpu_api):
+    """Two pools of which the device holds one at a time: the CTAs left over wait for the second through the first
+    one's whole solve (20000 iterations, 18 ms or more), with a limit of 2000 polls (about 2 ms) that is ample for a
+    barrier or an exchange."""
+    scs = []
+    for i in range(2):
+        sc = scenes.batch(1, seed=3 + i, shapes=[(640, 320)]).scenes[0]
+        sc.oneshot = [scenes.aabb_source((0.0, 0.0), (320.0, 150.0))]
+        sc.cfg.projection.max_iterations, sc.cfg.projection.tolerance = 20000, 1e-14
+        scs.append(sc)
+    alone = [sc.make(gpu_api) for sc in scs]
+    with capi.Batch(gpu_api, [sc.cfg for sc in scs]) as batch:
+        scenes.BatchScene("two pools", scs, 0).setup(batch.sims)
+        batch.set_wait_limits(2000)
+        for _ in range(3):  # the first is the initialisation
+            sb = batch.step(scenes.DT)
+            sa = [s.step(scenes.DT) for s in alone]
+        assert [s.pressure_iterations for s in sb] == [s.pressure_iterations for s in sa] == [20000, 20000]
+        for b, a in zip(batch.sims, alone):
+            assert not compare_fields(b, a)
