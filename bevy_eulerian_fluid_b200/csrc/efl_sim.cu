@@ -2726,7 +2726,7 @@ efl_status efl_batch_tiles(const efl_batch* b, int32_t* tx, int32_t* ty, int32_t
     if (tx) *tx = c ? c->tx : 0;
     if (ty) *ty = c ? c->ty : 0;
     if (k) *k = c ? c->k : 0;
-    if (!c && b->ganged) {  // the gang solve's tiles
+    if (b->tile_fixed < 0 && b->ganged) {  // the gang solve's tiles, whatever the tuned streamed ones are
         if (tx) *tx = GANG_TX;
         if (ty) *ty = GANG_TY;
         if (k) *k = GANG_K;

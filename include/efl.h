@@ -464,8 +464,10 @@ EFL_API efl_status efl_batch_step(efl_batch* batch, float dt, efl_step_stats* st
  * cell-iteration, and the fastest stays; every form and configuration gives
  * the same iterates and iteration counts.  No reference counterpart. */
 EFL_API efl_status efl_batch_set_tiles(efl_batch* batch, int32_t config);
-/* The configuration in use (64, 32, 4 where the last solve ran by gangs
- * alone; 0, 0, 0 while tuning) and the measured cost of each (ns_per_cell_iteration: 4 entries or NULL; 0 = not tried). */
+/* The configuration in use (the fixed one; else 64, 32, 4 where the last
+ * solve ran by gangs alone, and the streamed one otherwise: 0, 0, 0 while
+ * tuning) and the measured cost of each (ns_per_cell_iteration: 4 entries or
+ * NULL; 0 = not tried). */
 EFL_API efl_status efl_batch_tiles(const efl_batch* batch, int32_t* tx, int32_t* ty, int32_t* k,
                                    double* ns_per_cell_iteration);
 /* Poll limit of the batched solve's waits (efl_set_wait_limits'

@@ -85,3 +85,25 @@ def test_batch_waits_as_long_as_a_gang_makes_progress(gpu_api):
         assert [s.pressure_iterations for s in sb] == [s.pressure_iterations for s in sa] == [20000, 20000]
         for b, a in zip(batch.sims, alone):
             assert not compare_fields(b, a)
+
+
+def test_batch_reports_the_tiles_of_its_last_solve(gpu_api):
+    """A simulation with more water than the device holds streams until the tuner has chosen; without its water the
+    solves run by gangs again, and their tiles are reported.  A residual test after every iteration makes the tuner
+    choose few iterations per round, other tiles than the gangs'."""
+    scs = [scenes.batch(1, seed=100 + i, shapes=[s]).scenes[0] for i, s in enumerate([(1024, 640), (64, 64)])]
+    scs[0].oneshot = [scenes.aabb_source((0.0, 0.0), (512.0, 314.0))]
+    for sc in scs:
+        sc.cfg.projection.max_iterations, sc.cfg.projection.check_interval = 20, 1
+    with capi.Batch(gpu_api, [sc.cfg for sc in scs]) as batch:
+        scenes.BatchScene("one large", scs, 0).setup(batch.sims)
+        for _ in range(8):  # the initialisation, a step that converges at once and four that tune
+            batch.step(scenes.DT)
+        tuned, cost = batch.tiles()
+        assert tuned in [(64, 32, 2), (64, 32, 4), (32, 32, 2), (64, 32, 8)] and all(cost)
+        for f in (capi.FIELD_LEVELSET_AIR, capi.FIELD_LEVELSET_AIR1):
+            batch.sims[0].set(f, np.full_like(batch.sims[0].get(f), 50.0))
+        batch.step(scenes.DT)
+        assert batch.tiles()[0] == (64, 32, 4)
+        batch.set_tiles(2)
+        assert batch.tiles()[0] == (32, 32, 2)
