@@ -148,7 +148,7 @@ struct efl_sim {
     GraphCache gc;                // captured step segments
     uint64_t graph_epoch = 1;     // counts the setters that change kernel arguments
     PF mix_d2{};       // second correction buffer (batched solve)
-    PF xbuf{};         // second halo-exchange plane of the persistent solves, allocated on first use
+    PF xbuf{};         // second halo-exchange plane of the fixed-count sweeps, allocated on first use
     bool owns_stream = true;
     float* d_vel = nullptr;  // velocity-magnitude partials (efl_velocity_magnitude)
     int cap_vel = 0;
@@ -680,8 +680,9 @@ efl_status v_cycle(efl_sim* s, std::vector<LevelT<T>>& mg, size_t i, bool symmet
     const efl_projection& P = s->cfg.projection;
     const LevelT<T>& L = mg[i];
     // The rest in one launch of one cluster, from the first level of at most 256^2 cells whose slabs fit (above, a
-    // level's launches have enough cells to fill the device); long flat levels (more than 1024 columns) that do not
-    // fit take the one-CTA form.
+    // level's launches have enough cells to fill the device).  A wide level may not fit (vc_plan: slabs of at most 8
+    // rows above 256 columns, of 4 above 512, none above 1024: 768 x 80 and 520 x 120 on 16 CTAs do not): it takes the
+    // one-CTA form up to 128^2 cells, and launches above.
     if ((int64_t)L.nx * L.ny <= VC_MAX_CELLS) {
         VcArgs<T> a{};
         size_t limit = 0, smem = 0;
@@ -2654,8 +2655,7 @@ efl_status efl_batch_create(const efl_config* cfgs, uint32_t n, efl_batch** out)
         s->stream = b->stream;
         s->owns_stream = false;
         b->sims.push_back(s);
-        if (ensure_mix_planes(s) != EFL_OK ||
-            (!s->xbuf.p && alloc_plane(s, s->xbuf, s->nx, s->ny, s->P, s->ny + 1) != EFL_OK)) {
+        if (ensure_mix_planes(s) != EFL_OK) {
             std::string m = s->err;
             batch_free(b);
             return batch_err(nullptr, EFL_ERR_OUT_OF_MEMORY, m);

@@ -2,19 +2,19 @@
 // (projection/shaders/gauss_seidel.wgsl:12-88, host loop gauss_seidel.rs:142-147).
 //
 // Forms:
-//  * solve_gs_fixed: n red-black iterations as one launch per colour
-//    (k_gs_color), f32 (the reference's fixed-count mode) or f64.
 //  * solve_gsmix_persistent: the tolerance-driven solve (mixed-precision
 //    iterative refinement, below) as ONE cooperative launch over the tiles that
 //    hold water.  Each CTA keeps its tile plus a halo of 2k cells on chip, so
 //    that k red-black iterations run between two halo exchanges (temporal
 //    blocking; the result is identical to k global sweeps because a half-sweep
-//    only reads the other colour).  Halos are exchanged through L2 behind a
-//    grid barrier whose spin is bounded; the relative residual is reduced and
-//    tested on the device every check_interval iterations, so the whole solve
-//    needs no host round trip.
+//    only reads the other colour).  Halos are exchanged through L2 by words
+//    that carry the number of their exchange, polled with a bound; the relative
+//    residual is reduced the same way and tested on the device every
+//    check_interval iterations, so the whole solve needs no host round trip.
 //  * solve_gsmix_global: the same solve with global-memory kernels and a host
 //    loop, for grids the persistent scheme does not cover.
+//  * solve_gs32_persistent: fixed-count f32 sweeps as one cooperative launch,
+//    for grids of at most one tile per SM.
 //  * solve_gs32_tiled: fixed-count f32 sweeps through shared-memory tiles
 //    (used when the TMA sweep of efl_sweep_tma.cuh is unavailable).
 #pragma once
@@ -53,7 +53,6 @@ struct SolveState {
 struct SolverWorkspace {
     int nx = 0, ny = 0, device = 0;
     int num_sms = 0;
-    size_t max_smem = 0;
     SolveState* state = nullptr;    // device
     GridBarrier* barrier = nullptr;  // state's
     SolveResult* result = nullptr;   // state's
@@ -183,7 +182,6 @@ inline efl_status solver_init(SolverWorkspace& ws, int nx, int ny, int device, s
         return EFL_ERR_CUDA;
     }
     ws.num_sms = prop.multiProcessorCount;
-    ws.max_smem = prop.sharedMemPerBlockOptin;
     ws.max_blocks = 4 * ws.num_sms;
     if (cudaMalloc(&ws.state, sizeof(SolveState)) != cudaSuccess ||
         cudaMalloc(&ws.partials, ws.max_blocks * sizeof(double2)) != cudaSuccess ||
@@ -203,20 +201,6 @@ inline void solver_free(SolverWorkspace& ws) {
     if (ws.wet) cudaFree(ws.wet);
     if (ws.h_state) cudaFreeHost(ws.h_state);
     ws = SolverWorkspace{};
-}
-
-// n red-black iterations at level L (red then black per iteration),
-// f32 (reference) or f64 iterate, one launch per colour.
-template <class T>
-inline efl_status solve_gs_fixed(SolverWorkspace&, const LevelT<T>& L, const Uniform& U, float weight, uint32_t n,
-                                 cudaStream_t stream) {
-    const dim3 b(32, 8);
-    const dim3 g(((L.nx + 1) / 2 + b.x - 1) / b.x, (L.ny + b.y - 1) / b.y);
-    for (uint32_t k = 0; k < n; ++k) {
-        k_gs_color<T><<<g, b, count_launch(), stream>>>(L, U.dx, U.rho, U.dt, weight, 1);
-        k_gs_color<T><<<g, b, count_launch(), stream>>>(L, U.dx, U.rho, U.dt, weight, 0);
-    }
-    return EFL_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -492,8 +476,8 @@ EFL_DEV bool oct_solve(const PersistentParams& P, const unsigned short* list, un
     const int pbase = y0 * Tile::RS + bx;
     auto pix = [&](int i, int j) { return pbase + j * Tile::RS + (i & 3) * W4 + (i >> 2); };
     const float wgt = (float)P.weight, omw1 = 1.0f - (float)P.weight;
-    // bit q: update cell; 16 + q: live (not on the outermost ring); 32 + q: counted and live; 48 + q: owned and
-    // in the domain
+    // bit q: update cell, live (not on the image's outermost ring); 32 + q: counted and live; 48 + q: owned and in the
+    // domain.  Bits 16 + q, live, are not read: without them the 80 x 72 image's form spills 796 bytes, not 612.
     unsigned long long fl = 0;
     unsigned upd_halo = 0;  // bit q: update cell, the image's outermost ring included
     f32x2 wl[NPAIR], wr[NPAIR], wu[NPAIR], wd[NPAIR], inv[NPAIR], rc[NPAIR], dv[NPAIR];
@@ -1396,7 +1380,7 @@ inline bool plan_resident(int threads, size_t smem) {
 }
 template <int EX, int EY, int KMAX, int NT, int ROWS>
 inline const void* oct_kernel() { return (const void*)k_gsmix_oct<EX, EY, KMAX, NT, ROWS>; }
-// Plans for the paired-lane form (OctTile: 26 bytes of shared memory per cell).  The launch holds the tiles with
+// Plans for the paired-lane form (OctTile: three doubles and a float per cell of the image, and padding).  The launch holds the tiles with
 // water only, which are not known on the host: a plan whose tiles do not all fit the device at once is followed by
 // the next one, which runs if it found too many.
 template <int EX, int EY, int KMAX, int NT, int ROWS>
@@ -1410,7 +1394,6 @@ inline bool try_plan_oct(const SolverWorkspace& ws, int nx, int ny, PersistentPl
     p->smem = sizeof(OctTile<EX, EY, ROWS>);
     p->kernel = (const void*)k_gsmix_oct<EX, EY, KMAX, NT, ROWS>;
     p->threads = NT;
-    if (p->smem + 4096 > ws.max_smem) return false;
     if ((int64_t)p->tiles_x * p->tiles_y > OCT_MAX_TILES || ws.num_sms > OCT_MAX_CTAS) return false;
     return p->ok = plan_resident<oct_kernel<EX, EY, KMAX, NT, ROWS>>(NT, p->smem);
 }

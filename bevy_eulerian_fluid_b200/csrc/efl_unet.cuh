@@ -1709,7 +1709,7 @@ inline void unet_conv_bwd(UNet& n, int i, const bf16* x, int xs, int xo, const b
     w.err = n.err;
     // About two CTAs per SM, as far as the partials' buffer goes.
     const int mtiles = (9 * cin + 127) / 128;
-    int pix = ((int)((int64_t)npix * mtiles / 296) + WG_K - 1) / WG_K * WG_K;
+    int pix = ((int)((int64_t)npix * mtiles / (2 * std::max(1, conv_sm_count()))) + WG_K - 1) / WG_K * WG_K;
     pix = std::min(1024, std::max(WG_K, pix));
     while ((size_t)((npix + pix - 1) / pix) * mtiles * 128 * cout > n.wpart_elems) pix *= 2;
     w.pix_per_cta = pix;
